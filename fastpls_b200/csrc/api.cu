@@ -105,10 +105,9 @@ void host_gemm(const T* left, const T* right, int rows, int inner, int columns,
   g.K = inner;
   g.A = a.get();
   g.lda = rows;
-  g.a_f32 = std::is_same<T, float>::value;
   g.B = b.get();
   g.ldb = inner;
-  g.b_f32 = g.a_f32;
+  g.f32 = std::is_same<T, float>::value;
   g.C = c.get();
   g.ldc = rows;
   gemm_f64(g, s);

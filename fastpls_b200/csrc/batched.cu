@@ -1103,7 +1103,7 @@ void BatchedCv<T>::form_gram(const double* kscale, cudaStream_t s) {
   g.trans_b = true;
   g.C = ws->gram.get();
   g.ldc = n;
-  g.lower = gemm_mma_supported(g);
+  g.lower = true;
   gemm_f64(g, s);
 }
 

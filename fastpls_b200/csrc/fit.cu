@@ -596,10 +596,10 @@ void fit_simpls(const T* X, int n, int p, long ld, const double* Yc,
     g.A = X;
     g.lda = ld;
     g.trans_a = true;
-    g.a_f32 = std::is_same<T, float>::value;
     g.B = X;
     g.ldb = ld;
-    g.b_f32 = std::is_same<T, float>::value;
+    g.f32 = std::is_same<T, float>::value;
+    g.lower = true;
     g.C = Gs.get();
     g.ldc = p;
     gemm_f64(g, stream);

@@ -1,21 +1,32 @@
-// FP64 GEMM on the FP64 tensor-core path (DMMA, mma.sync m8n8k4 f64).
+// FP64 GEMM on the FP64 tensor-core path (DMMA, mma.sync m16n8k8 f64).
 //
-//   C[M x N] = alpha * A[M x K] * op(B) (+ beta C), all FP64, column-major;
-//   op(B) = B (K x N, ld >= K) or B^T (B stored N x K, ld >= N).
+//   C[M x N] = alpha * op(A)[M x K] * op(B)[K x N] (+ beta C), column-major;
+//   op(X) = X or X^T, A and B both FP64 or both FP32 (widened exactly as the
+//   fragments are loaded), every product and sum FP64.
 //
 // B200 has no tcgen05 kind for FP64; its FP64 tensor path is the warp-level
-// DMMA instruction (same peak as DFMA, ~37 TFLOP/s, but one instruction does
-// 256 FMAs from register fragments, so shared-memory and issue bandwidth stop
-// being the limit of a SIMT register-tiled kernel).
+// DMMA instruction (36.8 to 37.0 TFLOP/s measured for every shape from m8n8k4
+// to m16n8k16, the rate of DFMA, but one instruction does 1024 FMAs from
+// register fragments, so shared-memory and issue bandwidth stop being the
+// limit of a SIMT register-tiled kernel).
 //
-// Block tile 128 x 128 x 16, 8 warps (2 x 4) each owning a 64 x 32 tile
-// (8 x 4 DMMA tiles, 64 FP64 accumulators per thread). Operand slabs stream
-// through a 3-stage cp.async ring (16-byte copies, zero-filled outside the
-// matrix). Shared layouts are padded so the fragment loads are conflict-free:
-// k-major [16][136] for operands contiguous along M/N, n-major [128][20] for
-// B contiguous along K. `lower` restricts the grid to the lower triangle of
-// block tiles (symmetric products such as the Gram X X^T); the caller mirrors.
+// Block tile TM x TN x 16, 8 warps. Operand slabs stream through a 4-stage
+// cp.async ring: 16-byte copies when the operand's base and column stride
+// are 16-byte multiples, one element per copy otherwise (odd row counts,
+// which a SIMT kernel took before), zero-filled outside the matrix either
+// way. Shared layouts are padded so that fragment loads are conflict-free:
+// k-major [16][T + pad] for operands contiguous along M or N (row stride
+// 4 mod 16 doubles or 8 mod 32 floats), row-major [T][20] for operands
+// contiguous along K. `lower` restricts the grid to the lower triangle of
+// square block tiles (symmetric products such as the Gram X X^T).
+//
+// The tile and the K splits come from gemm_plan (gemm.cu): most products of
+// this library are far from square -- a sketch of 41 columns, a 41 x 41 Gram
+// over 3000 rows, a 500 x 500 Gram over 40000 -- so narrow tiles and slices
+// over K are what fill the SMs. 128 x 128 alone and whole K left a 41 x 41
+// Gram over 3001 rows on one SM.
 #include "common.cuh"
+#include "gemm_mma.cuh"
 #include "kernels.cuh"
 
 #include <algorithm>
@@ -24,36 +35,110 @@ namespace fpls {
 
 namespace {
 
-constexpr int TM = 128, TN = 128, TK = 16, STAGES = 3, NT = 256;
-constexpr int LDA_S = TM + 8;   // k-major stride (doubles)
-constexpr int LDBN_S = TK + 4;  // n-major stride (doubles)
+constexpr int TK = 16, STAGES = 4, NT = 256;
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
+// Elements per row of a k-major slab [TK][row] / of a row-major slab [T][TK + 4].
+template <class T>
+constexpr int row_pad(int t) {
+  return t + (sizeof(T) == 8 ? 4 : 8);
+}
+constexpr int LDK = TK + 4;
+
+template <class T>
+constexpr int slab_elems(bool kcontig, int t) {
+  return kcontig ? t * LDK : TK * row_pad<T>(t);
+}
+
+// Copies of 16 bytes (or one element) with the bytes past `bytes` zero-filled.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int bytes) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  const int bytes = valid ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes));
+}
+__device__ __forceinline__ void cp_async1(double* smem, const double* gmem, bool ok) {
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(ok ? 8 : 0));
+}
+__device__ __forceinline__ void cp_async1(float* smem, const float* gmem, bool ok) {
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gmem), "r"(ok ? 4 : 0));
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
+// D += A B: A 16 x 8 (a[i]: row g + 8 (i & 1), k tg + 4 (i >> 1)), B 8 x 8
+// (b[i]: k tg + 4 i, column g), C rows g, g + 8 and columns 2 tg, 2 tg + 1.
+__device__ __forceinline__ void dmma(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};\n"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-// B_T: op(B) = B^T (B stored N x K, contiguous along N)
-template <bool B_T>
-__global__ void __launch_bounds__(NT, 1)
-    dgemm_mma(int M, int N, int K, const double* __restrict__ A, long lda,
-              const double* __restrict__ B, long ldb, double alpha, double beta,
-              double* __restrict__ C, long ldc, long split_stride,
-              int k_per_split, int lower) {
-  extern __shared__ __align__(16) double smem[];
-  double* As = smem;                                  // STAGES x TK x LDA_S
-  double* Bs = smem + STAGES * TK * LDA_S;            // STAGES x (TK x LDA_S | TN x LDBN_S)
-  constexpr int B_STAGE = B_T ? TK * LDA_S : TN * LDBN_S;
+// One slab (TR rows of op(X) by TK of k) into shared memory. Element (r, k)
+// is X[k + r ld] when KCONTIG, X[r + k ld] otherwise.
+template <class T, bool KCONTIG, int TR>
+__device__ __forceinline__ void load_slab(T* s, const T* __restrict__ X, long ld, int rows, int kend,
+                                          int r0, int k0, bool vec) {
+  constexpr int V = 16 / (int)sizeof(T);
+  const int tid = threadIdx.x;
+  if (vec) {
+    constexpr int CH = TR * TK / V;
+#pragma unroll
+    for (int it = 0; it < (CH + NT - 1) / NT; ++it) {
+      const int c = tid + it * NT;
+      if (CH % NT != 0 && c >= CH) break;
+      if (KCONTIG) {
+        const int r = c / (TK / V), k = (c % (TK / V)) * V;
+        const int left = r0 + r < rows ? min(V, max(0, kend - (k0 + k))) : 0;
+        cp_async16(s + r * LDK + k, left ? X + (k0 + k) + (long)(r0 + r) * ld : X, left * (int)sizeof(T));
+      } else {
+        const int k = c / (TR / V), r = (c % (TR / V)) * V;
+        const int left = k0 + k < kend ? min(V, max(0, rows - (r0 + r))) : 0;
+        cp_async16(s + k * row_pad<T>(TR) + r, left ? X + (r0 + r) + (long)(k0 + k) * ld : X,
+                   left * (int)sizeof(T));
+      }
+    }
+  } else {
+    constexpr int CH = TR * TK;
+#pragma unroll
+    for (int it = 0; it < CH / NT; ++it) {
+      const int c = tid + it * NT;
+      if (KCONTIG) {
+        const int r = c / TK, k = c % TK;
+        const bool ok = r0 + r < rows && k0 + k < kend;
+        cp_async1(s + r * LDK + k, ok ? X + (k0 + k) + (long)(r0 + r) * ld : X, ok);
+      } else {
+        const int k = c / TR, r = c % TR;
+        const bool ok = r0 + r < rows && k0 + k < kend;
+        cp_async1(s + k * row_pad<T>(TR) + r, ok ? X + (r0 + r) + (long)(k0 + k) * ld : X, ok);
+      }
+    }
+  }
+}
+
+template <class T, bool KCONTIG, int TR>
+__device__ __forceinline__ double slab_at(const T* s, int r, int k) {
+  return as_f64(KCONTIG ? s[r * LDK + k] : s[k * row_pad<T>(TR) + r]);
+}
+
+// A_T: A stored K x M (contiguous along K); B_T: B stored N x K (contiguous
+// along N).
+template <class T, bool A_T, bool B_T, int TM, int TN>
+__global__ void __launch_bounds__(NT, TM * TN >= 128 * 128 ? 1 : 2)
+    dgemm_mma(int M, int N, int K, const T* __restrict__ A, long lda, const T* __restrict__ B,
+              long ldb, double alpha, double beta, double* __restrict__ C, long ldc,
+              long split_stride, int k_per_split, int lower, int vec) {
+  constexpr int WARPS_N = TN == 128 ? 4 : TN == 64 ? 2 : 1;
+  constexpr int WARPS_M = 8 / WARPS_N;
+  constexpr int WM = TM / WARPS_M, WN = TN / WARPS_N;
+  constexpr int MT = WM / 16, NTL = WN / 8;
+  static_assert(WM % 16 == 0 && WN % 8 == 0, "whole DMMA tiles per warp");
+  constexpr int SA = slab_elems<T>(A_T, TM), SB = slab_elems<T>(!B_T, TN);
+  extern __shared__ __align__(16) unsigned char gemm_smem[];
+  T* As = reinterpret_cast<T*>(gemm_smem);  // STAGES slabs of A, then of B
+  T* Bs = As + STAGES * SA;
 
   int bm, bn;
   if (lower) {
@@ -68,55 +153,26 @@ __global__ void __launch_bounds__(NT, 1)
     bm = blockIdx.y;
   }
   const int m0 = bm * TM, n0 = bn * TN;
-  const int kbeg = blockIdx.z * k_per_split;
+  const int kbeg = min(K, (int)blockIdx.z * k_per_split);
   const int kend = min(K, kbeg + k_per_split);
-  const int ktiles = kend > kbeg ? (kend - kbeg + TK - 1) / TK : 0;
+  const int ktiles = (kend - kbeg + TK - 1) / TK;
   double* Cz = C + (long)blockIdx.z * split_stride;
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp >> 2, wn = warp & 3;  // 2 x 4 warps
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wm = (warp / WARPS_N) * WM, wn = (warp % WARPS_N) * WN;
 
   auto load_stage = [&](int stage, int kt) {
-    const int k0 = kbeg + kt * TK;
-    double* as = As + stage * TK * LDA_S;
-    double* bs = Bs + stage * B_STAGE;
-    // A: TK rows (k) of 128 contiguous m -> 16 x 64 chunks of 2 doubles
-#pragma unroll
-    for (int it = 0; it < (TK * TM / 2) / NT; ++it) {
-      const int c = tid + it * NT;
-      const int kk = c / (TM / 2), mm = (c % (TM / 2)) * 2;
-      const int gm = m0 + mm, gk = k0 + kk;
-      const bool ok = gm < M && gk < kend;
-      cp_async16(as + kk * LDA_S + mm, ok ? A + gm + (long)gk * lda : A, ok);
-    }
-    if (B_T) {
-      // op(B)(k, n) = B[n + k*ldb]: contiguous along n, stored k-major
-#pragma unroll
-      for (int it = 0; it < (TK * TN / 2) / NT; ++it) {
-        const int c = tid + it * NT;
-        const int kk = c / (TN / 2), nn = (c % (TN / 2)) * 2;
-        const int gn = n0 + nn, gk = k0 + kk;
-        const bool ok = gn < N && gk < kend;
-        cp_async16(bs + kk * LDA_S + nn, ok ? B + gn + (long)gk * ldb : B, ok);
-      }
-    } else {
-      // op(B)(k, n) = B[k + n*ldb]: contiguous along k, stored n-major
-#pragma unroll
-      for (int it = 0; it < (TK * TN / 2) / NT; ++it) {
-        const int c = tid + it * NT;
-        const int nn = c / (TK / 2), kk = (c % (TK / 2)) * 2;
-        const int gn = n0 + nn, gk = k0 + kk;
-        const bool ok = gn < N && gk < kend;
-        cp_async16(bs + nn * LDBN_S + kk, ok ? B + gk + (long)gn * ldb : B, ok);
-      }
-    }
+    load_slab<T, A_T, TM>(As + stage * SA, A, lda, M, kend, m0, kbeg + kt * TK, vec & 1);
+    load_slab<T, !B_T, TN>(Bs + stage * SB, B, ldb, N, kend, n0, kbeg + kt * TK, vec & 2);
   };
 
-  double acc[8][4][2];
+  double acc[MT][NTL][4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < MT; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < NTL; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
 
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
@@ -130,108 +186,97 @@ __global__ void __launch_bounds__(NT, 1)
     const int pre = kt + STAGES - 1;
     if (pre < ktiles) load_stage(pre % STAGES, pre);
     cp_commit();
-    const double* as = As + (kt % STAGES) * TK * LDA_S;
-    const double* bs = Bs + (kt % STAGES) * B_STAGE;
+    const T* as = As + (kt % STAGES) * SA;
+    const T* bs = Bs + (kt % STAGES) * SB;
 #pragma unroll
-    for (int kk = 0; kk < TK; kk += 4) {
-      double af[8], bf[4];
+    for (int kk = 0; kk < TK; kk += 8) {
+      double af[MT][4], bf[NTL][2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) af[i] = as[(kk + tg) * LDA_S + wm * 64 + i * 8 + g];
+      for (int i = 0; i < MT; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int nn = wn * 32 + j * 8 + g;
-        bf[j] = B_T ? bs[(kk + tg) * LDA_S + nn] : bs[nn * LDBN_S + kk + tg];
-      }
+        for (int e = 0; e < 4; ++e)
+          af[i][e] = slab_at<T, A_T, TM>(as, wm + i * 16 + g + 8 * (e & 1), kk + tg + 4 * (e >> 1));
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int j = 0; j < NTL; ++j)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+        for (int e = 0; e < 2; ++e) bf[j][e] = slab_at<T, !B_T, TN>(bs, wn + j * 8 + g, kk + tg + 4 * e);
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NTL; ++j) dmma(acc[i][j], af[i], bf[j]);
     }
   }
   cp_wait<0>();
 
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int row = m0 + wm * 64 + i * 8 + g;
-    if (row >= M) continue;
+  for (int i = 0; i < MT; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < NTL; ++j)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int col = n0 + wn * 32 + j * 8 + tg * 2 + h;
-        if (col >= N) continue;
-        double* dst = Cz + row + (long)col * ldc;
-        const double v = alpha * acc[i][j][h];
-        *dst = beta != 0.0 ? fma(beta, *dst, v) : v;
+      for (int e = 0; e < 4; ++e) {
+        const int row = m0 + wm + i * 16 + g + 8 * (e >> 1);
+        const int col = n0 + wn + j * 8 + tg * 2 + (e & 1);
+        if (row < M && col < N) {
+          double* dst = Cz + row + (long)col * ldc;
+          const double v = alpha * acc[i][j][e];
+          *dst = beta != 0.0 ? fma(beta, *dst, v) : v;
+        }
       }
-    }
-  }
 }
 
-__global__ void mirror_lower(double* C, int n, long ldc) {
-  const long total = (long)n * n;
-  for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long)gridDim.x * blockDim.x) {
-    const int r = (int)(idx % n), c = (int)(idx / n);
-    if (r < c) C[r + (long)c * ldc] = C[c + (long)r * ldc];
-  }
+bool aligned16(const void* p, long ld, size_t es) {
+  return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && (ld * (long)es) % 16 == 0;
 }
 
-size_t smem_bytes(bool b_t) {
-  const size_t a = (size_t)STAGES * TK * LDA_S;
-  const size_t b = (size_t)STAGES * (b_t ? TK * LDA_S : TN * LDBN_S);
-  return (a + b) * sizeof(double);
-}
-
-bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
-
-}  // namespace
-
-bool gemm_mma_supported(const GemmArgs& g) {
-  if (g.a_f32 || g.b_f32 || g.trans_a || g.kscale) return false;
-  if (!aligned16(g.A) || !aligned16(g.B)) return false;
-  if ((g.lda & 1) || (g.ldb & 1)) return false;
-  if (g.M & 1) return false;
-  if (!g.trans_b && (g.K & 1)) return false;
-  if (g.trans_b && (g.N & 1)) return false;
-  return true;
-}
-
-void gemm_mma_launch(const GemmArgs& g, bool lower, cudaStream_t stream) {
-  const size_t smem = smem_bytes(g.trans_b);
-  static bool configured[2] = {false, false};
-  if (!configured[g.trans_b]) {
-    if (g.trans_b)
-      FPLS_CHECK(cudaFuncSetAttribute(dgemm_mma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    else
-      FPLS_CHECK(cudaFuncSetAttribute(dgemm_mma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured[g.trans_b] = true;
-  }
-  const int kps = ((g.K + g.splits - 1) / g.splits + TK - 1) / TK * TK;
-  dim3 grid;
-  if (lower) {
-    const unsigned tiles = ceil_div(g.M, TM);
-    grid = dim3(tiles * (tiles + 1) / 2, 1, g.splits);
-  } else {
-    grid = dim3(ceil_div(g.N, TN), ceil_div(g.M, TM), g.splits);
-  }
-  if (g.trans_b)
-    dgemm_mma<true><<<grid, NT, smem, stream>>>(g.M, g.N, g.K, static_cast<const double*>(g.A), g.lda,
-                                                static_cast<const double*>(g.B), g.ldb, g.alpha, g.beta,
-                                                g.C, g.ldc, g.split_stride, kps, lower ? 1 : 0);
-  else
-    dgemm_mma<false><<<grid, NT, smem, stream>>>(g.M, g.N, g.K, static_cast<const double*>(g.A), g.lda,
-                                                 static_cast<const double*>(g.B), g.ldb, g.alpha, g.beta,
-                                                 g.C, g.ldc, g.split_stride, kps, lower ? 1 : 0);
+template <class T, bool A_T, bool B_T, int TM, int TN>
+void launch(const GemmArgs& g, const GemmPlan& plan, double* C, long ldc, long stride, double alpha,
+            double beta, cudaStream_t stream) {
+  constexpr size_t smem =
+      (size_t)STAGES * (slab_elems<T>(A_T, TM) + slab_elems<T>(!B_T, TN)) * sizeof(T);
+  static const bool configured = [] {
+    FPLS_CHECK(cudaFuncSetAttribute(dgemm_mma<T, A_T, B_T, TM, TN>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    return true;
+  }();
+  (void)configured;
+  const int kps = ((g.K + plan.splits - 1) / plan.splits + TK - 1) / TK * TK;
+  const unsigned tm = ceil_div(g.M, TM), tn = ceil_div(g.N, TN);
+  const dim3 grid = g.lower ? dim3(tm * (tm + 1) / 2, 1, plan.splits) : dim3(tn, tm, plan.splits);
+  const int vec = (aligned16(g.A, g.lda, sizeof(T)) ? 1 : 0) | (aligned16(g.B, g.ldb, sizeof(T)) ? 2 : 0);
+  dgemm_mma<T, A_T, B_T, TM, TN><<<grid, NT, smem, stream>>>(
+      g.M, g.N, g.K, static_cast<const T*>(g.A), g.lda, static_cast<const T*>(g.B), g.ldb, alpha, beta,
+      C, ldc, stride, kps, g.lower ? 1 : 0, vec);
   count_launch();
   FPLS_LAUNCH("dgemm_mma");
 }
 
-void mirror_lower_triangle(double* C, int n, long ldc, cudaStream_t stream) {
-  const long total = (long)n * n;
-  mirror_lower<<<(unsigned)std::min<long>((total + 255) / 256, 16L * num_sms()), 256, 0, stream>>>(C, n, ldc);
-  count_launch();
-  FPLS_LAUNCH("mirror_lower");
+template <class T, bool A_T, bool B_T>
+void by_tile(const GemmArgs& g, const GemmPlan& pl, double* C, long ldc, long stride, double alpha,
+             double beta, cudaStream_t s) {
+  if (pl.tm == 64) launch<T, A_T, B_T, 64, 64>(g, pl, C, ldc, stride, alpha, beta, s);
+  else if (pl.tn == 128) launch<T, A_T, B_T, 128, 128>(g, pl, C, ldc, stride, alpha, beta, s);
+  else if (pl.tn == 64) launch<T, A_T, B_T, 128, 64>(g, pl, C, ldc, stride, alpha, beta, s);
+  else launch<T, A_T, B_T, 128, 32>(g, pl, C, ldc, stride, alpha, beta, s);
+}
+
+template <class T>
+void by_layout(const GemmArgs& g, const GemmPlan& pl, double* C, long ldc, long stride, double alpha,
+               double beta, cudaStream_t s) {
+  if (g.trans_a) {
+    if (g.trans_b) by_tile<T, true, true>(g, pl, C, ldc, stride, alpha, beta, s);
+    else by_tile<T, true, false>(g, pl, C, ldc, stride, alpha, beta, s);
+  } else {
+    if (g.trans_b) by_tile<T, false, true>(g, pl, C, ldc, stride, alpha, beta, s);
+    else by_tile<T, false, false>(g, pl, C, ldc, stride, alpha, beta, s);
+  }
+}
+
+}  // namespace
+
+void gemm_mma_launch(const GemmArgs& g, const GemmPlan& plan, double* C, long ldc, long split_stride,
+                     double alpha, double beta, cudaStream_t stream) {
+  if (g.f32) by_layout<float>(g, plan, C, ldc, split_stride, alpha, beta, stream);
+  else by_layout<double>(g, plan, C, ldc, split_stride, alpha, beta, stream);
 }
 
 }  // namespace fpls

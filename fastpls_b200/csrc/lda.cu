@@ -128,36 +128,15 @@ void LdaState::train(const double* scores, int n_, long lds, int a_,
   g.ldb = lds;
   g.C = gram.get();
   g.ldc = a;
-  g.splits = gemm_pick_splits(a, a, n);
-  DeviceArray<double> split_buf;
-  if (g.splits > 1) {
-    split_buf.allocate((size_t)g.splits * a * a, stream);
-    g.C = split_buf.get();
-    g.split_stride = (long)a * a;
-  }
   gemm_f64(g, stream);
-  if (g.splits > 1)
-    FPLS_CHECK(cudaMemcpyAsync(gram.get(), split_buf.get(), sizeof(double) * a * a,
-                               cudaMemcpyDeviceToDevice, stream));
   GemmArgs h = g;
   h.M = c;
   h.N = a;
   h.A = oh.get();
   h.lda = n;
-  h.splits = gemm_pick_splits(c, a, n);
   h.C = sums.get();
   h.ldc = c;
-  DeviceArray<double> split_buf2;
-  if (h.splits > 1) {
-    split_buf2.allocate((size_t)h.splits * c * a, stream);
-    h.C = split_buf2.get();
-    h.split_stride = (long)c * a;
-  }
-  h.split_stride = h.splits > 1 ? (long)c * a : 0;
   gemm_f64(h, stream);
-  if (h.splits > 1)
-    FPLS_CHECK(cudaMemcpyAsync(sums.get(), split_buf2.get(), sizeof(double) * c * a,
-                               cudaMemcpyDeviceToDevice, stream));
   prefixes.clear();
 }
 

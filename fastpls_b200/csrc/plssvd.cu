@@ -170,14 +170,9 @@ void fit_plssvd(const T* X, int n, int p, long ld, const double* Yc,
   h.trans_a = true;
   h.B = model.T.get();
   h.ldb = n;
-  h.splits = gemm_pick_splits(k, k, n);
-  DeviceArray<double> parts((size_t)h.splits * k * k, stream);
-  h.C = parts.get();
+  h.C = gram.get();
   h.ldc = k;
-  h.split_stride = (long)k * k;
   gemm_f64(h, stream);
-  FPLS_CHECK(cudaMemcpyAsync(gram.get(), parts.get(), sizeof(double) * k * k,
-                             cudaMemcpyDeviceToDevice, stream));
   model.W.allocate((size_t)k * k * m, stream);
   DeviceArray<double> lwork((size_t)k * k, stream);
   plssvd_weights_kernel<<<1, 128, 0, stream>>>(gram.get(), k, model.sigma.get(),

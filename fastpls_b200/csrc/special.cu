@@ -317,7 +317,7 @@ void fit_kernelpls(const T* X, int n, int p, long ld, const double* Yc,
   g.trans_b = true;
   g.C = design.get();
   g.ldc = n;
-  g.lower = gemm_mma_supported(g);
+  g.lower = true;
   gemm_f64(g, s);
   kernel_transform<<<grid_for((long)n * n), TB, 0, s>>>(design.get(), n, n, n, kind, gamma, degree, coef0,
                                                          model.ref_norms.get(), model.ref_norms.get());

@@ -129,7 +129,7 @@ void fastcor_impl(const T* a, const T* b, int rows_a, int cols_a, int rows_b,
     g.trans_b = true;
     g.C = C.get();
     g.ldc = units_a;
-    g.lower = !b && gemm_mma_supported(g);
+    g.lower = !b;
     gemm_f64(g, s);
   }
   FPLS_CHECK(cudaMemcpyAsync(out, C.get(), sizeof(double) * count, cudaMemcpyDeviceToHost, s));

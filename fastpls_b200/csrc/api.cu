@@ -107,7 +107,7 @@ void host_gemm(const T* left, const T* right, int rows, int inner, int columns,
   g.lda = rows;
   g.B = b.get();
   g.ldb = inner;
-  g.f32 = std::is_same<T, float>::value;
+  g.a_type = g.b_type = gemm_type<T>::value;
   g.C = c.get();
   g.ldc = rows;
   gemm_f64(g, s);

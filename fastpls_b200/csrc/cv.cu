@@ -22,12 +22,15 @@ namespace fpls {
 
 namespace {
 
+// Block (response, prefix): squared errors and squares about the training mean.
 __global__ void fold_sums_kernel(const double* __restrict__ pred,
                                  const double* __restrict__ y,
                                  const double* __restrict__ ymean, int n,
                                  int q, double* out) {
   __shared__ double scratch[32];
   const int c = blockIdx.x;
+  pred += (long)blockIdx.y * n * q;
+  out += (long)blockIdx.y * 2 * q;
   double sse = 0.0, st = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double v = y[i + (long)c * n];
@@ -140,7 +143,8 @@ void cv_regression(int method, const T* predictors, const T* responses,
     DeviceArray<int> idx_tr(fp.max_train, s), idx_te(fp.max_test, s);
     DeviceArray<double> Yc((size_t)fp.max_train * q, s), ycsum(q, s);
     DeviceArray<double> scores((size_t)fp.max_test * maximum_prefix, s);
-    DeviceArray<double> pred((size_t)fp.max_test * q, s);
+    const int step = prefixes_at_once((size_t)fp.max_test * q * sizeof(double), prefix_count);
+    DeviceArray<double> pred((size_t)fp.max_test * q * step, s);
     DeviceArray<double> sums((size_t)2 * q * prefix_count, s);
     Workspace ws;
     ws.ensure(fp.max_train, p, q, maximum_prefix, s);
@@ -177,13 +181,14 @@ void cv_regression(int method, const T* predictors, const T* responses,
       fit_method<T>(method, Xtr.get(), ntr, p, Yc.get(), ycsum.get(), q, maximum_prefix, scaling, model, ws, s);
       project_rows<T>(model, Xte.get(), nte, nte, maximum_prefix, scores.get(), nte, ws, s);
       if (store_predictions) host_pred.resize((size_t)nte * q * prefix_count);
-      for (int j = 0; j < prefix_count; ++j) {
-        predict_from_scores(model, scores.get(), nte, nte, prefixes[j], pred.get(), nte, s);
+      for (int j = 0; j < prefix_count; j += step) {
+        const int w = std::min(step, prefix_count - j);
+        predict_prefixes<double>(model, scores.get(), nte, nte, prefixes + j, w, pred.get(), s);
         if (store_predictions)
           FPLS_CHECK(cudaMemcpyAsync(host_pred.data() + (size_t)j * nte * q, pred.get(),
-                                     sizeof(double) * nte * q, cudaMemcpyDeviceToHost, s));
-        fold_sums_kernel<<<q, 256, 0, s>>>(pred.get(), Yte.get(), model.ymean.get(), nte, q,
-                                           sums.get() + (size_t)2 * q * j);
+                                     sizeof(double) * nte * q * w, cudaMemcpyDeviceToHost, s));
+        fold_sums_kernel<<<dim3(q, w), 256, 0, s>>>(pred.get(), Yte.get(), model.ymean.get(), nte, q,
+                                                    sums.get() + (size_t)2 * q * j);
         count_launch();
         FPLS_LAUNCH("fold_sums");
       }
@@ -269,10 +274,11 @@ void cv_classification(int method, const T* predictors, const int* labels,
     upload_h2d(X.get(), predictors, sizeof(T) * n * p, s);
     DeviceArray<T> Xtr((size_t)fp.max_train * p, s), Xte((size_t)fp.max_test * p, s);
     DeviceArray<int> idx_tr(fp.max_train, s), idx_te(fp.max_test, s);
-    DeviceArray<int> lab_tr(fp.max_train, s), top(fp.max_test, s);
+    const int step = prefixes_at_once((size_t)fp.max_test * classes * sizeof(double), prefix_count);
+    DeviceArray<int> lab_tr(fp.max_train, s), top((size_t)fp.max_test * step, s);
     DeviceArray<double> Yc((size_t)fp.max_train * classes, s), ycsum(classes, s);
     DeviceArray<double> scores((size_t)fp.max_test * maximum_prefix, s);
-    DeviceArray<double> pred((size_t)fp.max_test * classes, s), disc((size_t)fp.max_test * classes, s);
+    DeviceArray<double> pred((size_t)fp.max_test * classes * step, s);
     Workspace ws;
     ws.ensure(fp.max_train, p, classes, maximum_prefix, s);
     std::fill(metrics, metrics + prefix_count, 0.0);
@@ -342,19 +348,17 @@ void cv_classification(int method, const T* predictors, const int* labels,
       }
       host_labels.resize((size_t)nte * prefix_count);
       if (store_scores) host_scores.resize((size_t)nte * c * prefix_count);
-      for (int j = 0; j < prefix_count; ++j) {
-        predict_from_scores(model, scores.get(), nte, nte, prefixes[j], pred.get(), nte, s);
+      for (int j = 0; j < prefix_count; j += step) {
+        const int w = std::min(step, prefix_count - j);
+        if (store_scores || !use_lda)
+          predict_prefixes<double>(model, scores.get(), nte, nte, prefixes + j, w, pred.get(), s);
         if (store_scores)
           FPLS_CHECK(cudaMemcpyAsync(host_scores.data() + (size_t)j * nte * c, pred.get(),
-                                     sizeof(double) * nte * c, cudaMemcpyDeviceToHost, s));
-        const double* decoded = pred.get();
-        if (use_lda) {
-          lda->discriminants(scores.get(), nte, nte, prefixes[j], disc.get(), nte, s);
-          decoded = disc.get();
-        }
-        topk_rows(decoded, nte, c, 1, top.get(), nte, s);
+                                     sizeof(double) * nte * c * w, cudaMemcpyDeviceToHost, s));
+        if (use_lda) lda->discriminants(scores.get(), nte, nte, prefixes + j, w, pred.get(), s);
+        topk_rows(pred.get(), nte, c, 1, w, top.get(), nte, s);
         FPLS_CHECK(cudaMemcpyAsync(host_labels.data() + (size_t)j * nte, top.get(),
-                                   sizeof(int) * nte, cudaMemcpyDeviceToHost, s));
+                                   sizeof(int) * nte * w, cudaMemcpyDeviceToHost, s));
       }
       raise_on_flag(ws, s, method == kPlssvd
           ? "resident PLS-SVD failed: invalid labels, decomposition or score Gram"

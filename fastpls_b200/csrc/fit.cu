@@ -381,33 +381,6 @@ __global__ void finish_component(double* Tcol, int n, const double* scal,
     for (int c = threadIdx.x; c < m; c += blockDim.x) Qcol[c] = hq[a_cur + c];
 }
 
-// Rs = R / scale (p x k), roff[c] = mean . Rs[:,c]
-__global__ void scaled_weights(const double* __restrict__ R, int p, int k,
-                               const double* __restrict__ mean,
-                               const double* __restrict__ scale, double* Rs,
-                               double* roff) {
-  __shared__ double scratch[32];
-  const int c = blockIdx.x;
-  double acc = 0.0;
-  for (int j = threadIdx.x; j < p; j += blockDim.x) {
-    const double w = R[j + (long)c * p] / scale[j];
-    Rs[j + (long)c * p] = w;
-    acc = fma(mean[j], w, acc);
-  }
-  acc = block_sum(acc, scratch);
-  if (threadIdx.x == 0) roff[c] = acc;
-}
-
-__global__ void fill_rows_mean(double* out, int rows, int m, long ldo,
-                               const double* ymean) {
-  const long total = (long)rows * m;
-  for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(idx % rows), c = (int)(idx / rows);
-    out[i + (long)c * ldo] = ymean[c];
-  }
-}
-
 // Gs[j, k] = (G[j, k] - n mean_j mean_k) / (scale_j scale_k): the Gram of
 // the standardised predictors from the raw X^T X.
 __global__ void standardize_gram(double* G, int p, int n, const double* __restrict__ mean,
@@ -598,7 +571,7 @@ void fit_simpls(const T* X, int n, int p, long ld, const double* Yc,
     g.trans_a = true;
     g.B = X;
     g.ldb = ld;
-    g.f32 = std::is_same<T, float>::value;
+    g.a_type = g.b_type = gemm_type<T>::value;
     g.lower = true;
     g.C = Gs.get();
     g.ldc = p;
@@ -664,7 +637,7 @@ void fit_simpls(const T* X, int n, int p, long ld, const double* Yc,
       count_launch();
       FPLS_LAUNCH("gram_tstats");
     } else {
-      xr_product<T>(X, n, p, ld, rt, p, 1, scal, tcol, n, ws.stream_partial, stream);
+      xr_product<T>(X, n, p, ld, rt, p, 1, scal, 1, tcol, n, ws.stream_partial, stream);
       tstats_kernel<<<std::min<unsigned>(ceil_div(n, TB), 2 * num_sms()), TB, 0, stream>>>(
           tcol, n, part, ctr + 1, scal);
       count_launch();
@@ -697,53 +670,6 @@ void fit_simpls(const T* X, int n, int p, long ld, const double* Yc,
   }
 }
 
-template <class T>
-void project_rows(const DeviceModel& model, const T* X, int rows, long ld,
-                  int k, double* out, long ldo, Workspace& ws,
-                  cudaStream_t stream) {
-  require(k >= 1 && k <= model.a, "invalid projection prefix");
-  const int p = model.p;
-  DeviceArray<double> Rs((size_t)p * k + k, stream);
-  double* roff = Rs.get() + (size_t)p * k;
-  scaled_weights<<<k, TB, 0, stream>>>(model.R.get(), p, k, model.mean.get(),
-                                       model.scale.get(), Rs.get(), roff);
-  count_launch();
-  FPLS_LAUNCH("scaled_weights");
-  xr_product<T>(X, rows, p, ld, Rs.get(), p, k, roff, out, ldo,
-                ws.stream_partial, stream, ws.flag.get());
-}
-
-void predict_from_scores(const DeviceModel& model, const double* scores,
-                         int rows, long lds, int k, double* out, long ldo,
-                         cudaStream_t stream) {
-  require(k >= 1 && k <= model.a, "invalid prediction prefix");
-  const int m = model.m;
-  const long total = (long)rows * m;
-  fill_rows_mean<<<(unsigned)std::min<long>((total + 255) / 256, 8L * num_sms()), 256, 0, stream>>>(
-      out, rows, m, ldo, model.ymean.get());
-  count_launch();
-  FPLS_LAUNCH("fill_rows_mean");
-  GemmArgs g;
-  g.M = rows;
-  g.N = m;
-  g.K = k;
-  g.A = scores;
-  g.lda = lds;
-  if (model.method == kPlssvd) {
-    // W block for prefix k: k x m at offset (k-1) * a * m in model.W
-    g.B = model.W.get() + (size_t)(k - 1) * model.a * m;
-    g.ldb = k;
-  } else {
-    g.B = model.Q.get();
-    g.ldb = m;
-    g.trans_b = true;
-  }
-  g.C = out;
-  g.ldc = ldo;
-  g.beta = 1.0;
-  gemm_f64(g, stream);
-}
-
 template void prepare_responses<float>(const float*, const int*, int, int, double*,
                                        double*, double*, int*, cudaStream_t);
 template void prepare_responses<double>(const double*, const int*, int, int, double*,
@@ -752,8 +678,6 @@ template void prepare_responses<double>(const double*, const int*, int, int, dou
   template void fit_simpls<T>(const T*, int, int, long, const double*,        \
                               const double*, int, int, int, DeviceModel&,     \
                               Workspace&, cudaStream_t, int, bool);           \
-  template void project_rows<T>(const DeviceModel&, const T*, int, long, int, \
-                                double*, long, Workspace&, cudaStream_t);   \
   template void compute_crossprod<T>(const T*, int, int, long, const double*, \
                                      const double*, int, int, DeviceModel&,   \
                                      double*, Workspace&, cudaStream_t);

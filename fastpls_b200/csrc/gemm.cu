@@ -33,15 +33,49 @@ __device__ __forceinline__ double slice_sum(const double* __restrict__ slices, i
   return v;
 }
 
-// C = alpha * (sum of `splits` contiguous M x N slices) (+ beta C)
+// C = alpha * (sum of `splits` contiguous M x N slices) - coff (+ beta C)
 __global__ void sum_slices(const double* __restrict__ slices, int splits, int M, int N, double alpha,
-                           double beta, double* C, long ldc) {
+                           double beta, double* C, long ldc, const double* __restrict__ coff,
+                           int coff_parts) {
   const long total = (long)M * N;
   for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
        idx += (long)gridDim.x * blockDim.x) {
-    const double v = alpha * slice_sum(slices, splits, idx, total);
+    double v = alpha * slice_sum(slices, splits, idx, total);
+    if (coff) v -= column_offset(coff, coff_parts, (int)(idx / M));
     double* dst = C + (idx % M) + (idx / M) * ldc;
     *dst = beta != 0.0 ? fma(beta, *dst, v) : v;
+  }
+}
+
+// The same for many slices of a small result: 8 threads an element, thread q
+// summing slices q, q + 8, ... and the 8 sums added in order, so that 144
+// slices of a 9 x 9 Gram are 18 loads deep instead of 144 (61 us, 5 us so).
+// Which of the two runs depends on the number of slices alone.
+constexpr int kManySlices = 16;
+__global__ void __launch_bounds__(256)
+    sum_many_slices(const double* __restrict__ slices, int splits, int M, int N, double alpha,
+                    double beta, double* C, long ldc, const double* __restrict__ coff, int coff_parts) {
+  __shared__ double part[8][32];
+  const long total = (long)M * N;
+  const int x = threadIdx.x & 31, q = threadIdx.x >> 5;
+  for (long base = blockIdx.x * 32L; base < total; base += gridDim.x * 32L) {
+    const long idx = base + x;
+    double v = 0.0;
+    if (idx < total) {
+#pragma unroll 6
+      for (int z = q; z < splits; z += 8) v += slices[idx + z * total];
+    }
+    part[q][x] = v;
+    __syncthreads();
+    if (q == 0 && idx < total) {
+#pragma unroll
+      for (int u = 1; u < 8; ++u) v += part[u][x];
+      v *= alpha;
+      if (coff) v -= column_offset(coff, coff_parts, (int)(idx / M));
+      double* dst = C + (idx % M) + (idx / M) * ldc;
+      *dst = beta != 0.0 ? fma(beta, *dst, v) : v;
+    }
+    __syncthreads();
   }
 }
 
@@ -104,8 +138,8 @@ GemmTiming& timing() {
 // practice), a slab takes no less than about 500 clocks of load latency
 // through the 4-stage ring, a block about 4000 clocks to start, fill and
 // store, and K slices cost a second kernel that reads them.
-GemmPlan gemm_plan(int M, int N, int K, bool lower) {
-  static const int tiles[4][2] = {{128, 128}, {128, 64}, {128, 32}, {64, 64}};
+GemmPlan gemm_plan(int M, int N, int K, bool lower, int k_slice) {
+  static const int tiles[5][2] = {{128, 128}, {128, 64}, {128, 32}, {128, 16}, {64, 64}};
   const double sms = num_sms();
   GemmPlan best;
   double best_cost = -1.0;
@@ -116,10 +150,11 @@ GemmPlan gemm_plan(int M, int N, int K, bool lower) {
     const double count = lower ? (double)tm * (tm + 1) / 2 : (double)tm * tn;
     const int occ = t[0] * t[1] >= 128 * 128 ? 1 : 2;
     const double slab_clk = t[0] * t[1] / 4.0 * 1.25;
-    const int most = std::max(1, std::min(256, K / 64));
-    for (int s = 1; s <= most; s = s < 8 ? s + 1 : s + s / 8) {
-      // slices are kept to what a small product needs
-      if (s > 1 && (double)s * M * N * 8.0 > 256.0 * 1024 * 1024) break;
+    // slices are kept to 256 MB
+    const double room = 256.0 * 1024 * 1024 / ((double)M * N * 8.0);
+    const int most = (int)std::max(1.0, std::min(room, k_slice > 0 ? (double)ceil_div(std::max(K, 1), k_slice)
+                                                                   : std::min(256.0, K / 64.0)));
+    for (int s = k_slice > 0 ? most : 1; s <= most; s = s < 8 ? s + 1 : s + s / 8) {
       const double slabs = ceil_div(ceil_div(K, s), 16);
       const double per_sm = std::ceil(count * s / sms);
       const double waves = std::ceil(per_sm / occ);
@@ -160,28 +195,32 @@ void gemm_profile_read(double* ms, double* flops, unsigned long long* launches) 
 void gemm_f64(const GemmArgs& g, cudaStream_t stream) {
   require(g.M >= 0 && g.N >= 0 && g.K >= 0, "invalid GEMM dimensions");
   if (g.M == 0 || g.N == 0) return;
-  require(!g.lower || (g.M == g.N && g.beta == 0.0), "symmetric GEMM takes a square product");
+  require(!g.lower || (g.M == g.N && g.beta == 0.0 && !g.coff), "symmetric GEMM takes a square product");
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   if (timing().enabled) {
     FPLS_CHECK(cudaEventCreate(&ev0));
     FPLS_CHECK(cudaEventCreate(&ev1));
     FPLS_CHECK(cudaEventRecord(ev0, stream));
   }
-  const GemmPlan plan = gemm_plan(g.M, g.N, g.K, g.lower);
+  const GemmPlan plan = gemm_plan(g.M, g.N, g.K, g.lower, g.k_slice);
   if (plan.splits > 1) {
     const long total = (long)g.M * g.N;
     DeviceArray<double> slices((size_t)plan.splits * total, stream);
-    gemm_mma_launch(g, plan, slices.get(), g.M, total, 1.0, 0.0, stream);
+    gemm_mma_launch(g, plan, slices.get(), g.M, total, 1.0, 0.0, nullptr, stream);
     if (g.lower) {
       launch_mirror(slices.get(), plan.splits, g.alpha, g.C, g.M, g.ldc, stream);
     } else {
-      sum_slices<<<(unsigned)std::min<long>((total + 127) / 128, 16L * num_sms()), 128, 0, stream>>>(
-          slices.get(), plan.splits, g.M, g.N, g.alpha, g.beta, g.C, g.ldc);
+      if (plan.splits >= kManySlices)
+        sum_many_slices<<<(unsigned)std::min<long>((total + 31) / 32, 32L * num_sms()), 256, 0, stream>>>(
+            slices.get(), plan.splits, g.M, g.N, g.alpha, g.beta, g.C, g.ldc, g.coff, g.coff_parts);
+      else
+        sum_slices<<<(unsigned)std::min<long>((total + 127) / 128, 16L * num_sms()), 128, 0, stream>>>(
+            slices.get(), plan.splits, g.M, g.N, g.alpha, g.beta, g.C, g.ldc, g.coff, g.coff_parts);
       count_launch();
       FPLS_LAUNCH("sum_slices");
     }
   } else {
-    gemm_mma_launch(g, plan, g.C, g.ldc, 0, g.alpha, g.beta, stream);
+    gemm_mma_launch(g, plan, g.C, g.ldc, 0, g.alpha, g.beta, g.coff, stream);
     if (g.lower) mirror_lower_triangle(g.C, g.M, g.ldc, stream);
   }
   if (ev0) {

@@ -1,8 +1,9 @@
 // FP64 GEMM on the FP64 tensor-core path (DMMA, mma.sync m16n8k8 f64).
 //
 //   C[M x N] = alpha * op(A)[M x K] * op(B)[K x N] (+ beta C), column-major;
-//   op(X) = X or X^T, A and B both FP64 or both FP32 (widened exactly as the
-//   fragments are loaded), every product and sum FP64.
+//   op(X) = X or X^T, A and B both FP64 or both FP32, or (A X-like predictors,
+//   not transposed) A FP32 or BF16 and B FP64; narrow types are widened
+//   exactly as the fragments are loaded, every product and sum is FP64.
 //
 // B200 has no tcgen05 kind for FP64; its FP64 tensor path is the warp-level
 // DMMA instruction (36.8 to 37.0 TFLOP/s measured for every shape from m8n8k4
@@ -62,6 +63,11 @@ __device__ __forceinline__ void cp_async1(float* smem, const float* gmem, bool o
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gmem), "r"(ok ? 4 : 0));
 }
+__device__ __forceinline__ void cp_async1(bf16* smem, const bf16* gmem, bool ok) {
+  // cp.async copies no less than 4 bytes: a plain store, ordered by the
+  // barrier that ends the stage's wait
+  *smem = ok ? *gmem : __ushort_as_bfloat16((unsigned short)0);
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
@@ -102,6 +108,7 @@ __device__ __forceinline__ void load_slab(T* s, const T* __restrict__ X, long ld
     }
   } else {
     constexpr int CH = TR * TK;
+    static_assert(CH % NT == 0, "whole passes of element copies");
 #pragma unroll
     for (int it = 0; it < CH / NT; ++it) {
       const int c = tid + it * NT;
@@ -125,20 +132,22 @@ __device__ __forceinline__ double slab_at(const T* s, int r, int k) {
 
 // A_T: A stored K x M (contiguous along K); B_T: B stored N x K (contiguous
 // along N).
-template <class T, bool A_T, bool B_T, int TM, int TN>
+template <class TA, class TB, bool A_T, bool B_T, int TM, int TN>
 __global__ void __launch_bounds__(NT, TM * TN >= 128 * 128 ? 1 : 2)
-    dgemm_mma(int M, int N, int K, const T* __restrict__ A, long lda, const T* __restrict__ B,
+    dgemm_mma(int M, int N, int K, const TA* __restrict__ A, long lda, const TB* __restrict__ B,
               long ldb, double alpha, double beta, double* __restrict__ C, long ldc,
-              long split_stride, int k_per_split, int lower, int vec) {
+              long split_stride, int k_per_split, int lower, int vec,
+              const double* __restrict__ coff, int coff_parts) {
   constexpr int WARPS_N = TN == 128 ? 4 : TN == 64 ? 2 : 1;
   constexpr int WARPS_M = 8 / WARPS_N;
   constexpr int WM = TM / WARPS_M, WN = TN / WARPS_N;
   constexpr int MT = WM / 16, NTL = WN / 8;
   static_assert(WM % 16 == 0 && WN % 8 == 0, "whole DMMA tiles per warp");
-  constexpr int SA = slab_elems<T>(A_T, TM), SB = slab_elems<T>(!B_T, TN);
+  constexpr int SA = slab_elems<TA>(A_T, TM), SB = slab_elems<TB>(!B_T, TN);
+  static_assert(STAGES * SA * sizeof(TA) % 16 == 0, "B slabs stay 16-byte aligned");
   extern __shared__ __align__(16) unsigned char gemm_smem[];
-  T* As = reinterpret_cast<T*>(gemm_smem);  // STAGES slabs of A, then of B
-  T* Bs = As + STAGES * SA;
+  TA* As = reinterpret_cast<TA*>(gemm_smem);  // STAGES slabs of A, then of B
+  TB* Bs = reinterpret_cast<TB*>(As + STAGES * SA);
 
   int bm, bn;
   if (lower) {
@@ -162,8 +171,8 @@ __global__ void __launch_bounds__(NT, TM * TN >= 128 * 128 ? 1 : 2)
   const int wm = (warp / WARPS_N) * WM, wn = (warp % WARPS_N) * WN;
 
   auto load_stage = [&](int stage, int kt) {
-    load_slab<T, A_T, TM>(As + stage * SA, A, lda, M, kend, m0, kbeg + kt * TK, vec & 1);
-    load_slab<T, !B_T, TN>(Bs + stage * SB, B, ldb, N, kend, n0, kbeg + kt * TK, vec & 2);
+    load_slab<TA, A_T, TM>(As + stage * SA, A, lda, M, kend, m0, kbeg + kt * TK, vec & 1);
+    load_slab<TB, !B_T, TN>(Bs + stage * SB, B, ldb, N, kend, n0, kbeg + kt * TK, vec & 2);
   };
 
   double acc[MT][NTL][4];
@@ -186,8 +195,8 @@ __global__ void __launch_bounds__(NT, TM * TN >= 128 * 128 ? 1 : 2)
     const int pre = kt + STAGES - 1;
     if (pre < ktiles) load_stage(pre % STAGES, pre);
     cp_commit();
-    const T* as = As + (kt % STAGES) * SA;
-    const T* bs = Bs + (kt % STAGES) * SB;
+    const TA* as = As + (kt % STAGES) * SA;
+    const TB* bs = Bs + (kt % STAGES) * SB;
 #pragma unroll
     for (int kk = 0; kk < TK; kk += 8) {
       double af[MT][4], bf[NTL][2];
@@ -195,11 +204,11 @@ __global__ void __launch_bounds__(NT, TM * TN >= 128 * 128 ? 1 : 2)
       for (int i = 0; i < MT; ++i)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          af[i][e] = slab_at<T, A_T, TM>(as, wm + i * 16 + g + 8 * (e & 1), kk + tg + 4 * (e >> 1));
+          af[i][e] = slab_at<TA, A_T, TM>(as, wm + i * 16 + g + 8 * (e & 1), kk + tg + 4 * (e >> 1));
 #pragma unroll
       for (int j = 0; j < NTL; ++j)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) bf[j][e] = slab_at<T, !B_T, TN>(bs, wn + j * 8 + g, kk + tg + 4 * e);
+        for (int e = 0; e < 2; ++e) bf[j][e] = slab_at<TB, !B_T, TN>(bs, wn + j * 8 + g, kk + tg + 4 * e);
 #pragma unroll
       for (int i = 0; i < MT; ++i)
 #pragma unroll
@@ -209,32 +218,44 @@ __global__ void __launch_bounds__(NT, TM * TN >= 128 * 128 ? 1 : 2)
   cp_wait<0>();
 
 #pragma unroll
-  for (int i = 0; i < MT; ++i)
+  for (int j = 0; j < NTL; ++j)
 #pragma unroll
-    for (int j = 0; j < NTL; ++j)
+    for (int h = 0; h < 2; ++h) {
+      const int col = n0 + wn + j * 8 + tg * 2 + h;
+      if (col >= N) continue;
+      const double off = coff ? column_offset(coff, coff_parts, col) : 0.0;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int row = m0 + wm + i * 16 + g + 8 * (e >> 1);
-        const int col = n0 + wn + j * 8 + tg * 2 + (e & 1);
-        if (row < M && col < N) {
-          double* dst = Cz + row + (long)col * ldc;
-          const double v = alpha * acc[i][j][e];
-          *dst = beta != 0.0 ? fma(beta, *dst, v) : v;
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int row = m0 + wm + i * 16 + g + 8 * e;
+          if (row < M) {
+            double* dst = Cz + row + (long)col * ldc;
+            const double v = alpha * acc[i][j][2 * e + h] - off;
+            *dst = beta != 0.0 ? fma(beta, *dst, v) : v;
+          }
         }
-      }
+    }
 }
 
 bool aligned16(const void* p, long ld, size_t es) {
   return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && (ld * (long)es) % 16 == 0;
 }
 
-template <class T, bool A_T, bool B_T, int TM, int TN>
-void launch(const GemmArgs& g, const GemmPlan& plan, double* C, long ldc, long stride, double alpha,
-            double beta, cudaStream_t stream) {
-  constexpr size_t smem =
-      (size_t)STAGES * (slab_elems<T>(A_T, TM) + slab_elems<T>(!B_T, TN)) * sizeof(T);
+// Where the result goes: C, or the slices over K.
+struct Target {
+  double* C;
+  long ldc, stride;
+  double alpha, beta;
+  const double* coff;
+};
+
+template <class TA, class TB, bool A_T, bool B_T, int TM, int TN>
+void launch(const GemmArgs& g, const GemmPlan& plan, const Target& t, cudaStream_t stream) {
+  constexpr size_t smem = (size_t)STAGES * (slab_elems<TA>(A_T, TM) * sizeof(TA) +
+                                            slab_elems<TB>(!B_T, TN) * sizeof(TB));
   static const bool configured = [] {
-    FPLS_CHECK(cudaFuncSetAttribute(dgemm_mma<T, A_T, B_T, TM, TN>,
+    FPLS_CHECK(cudaFuncSetAttribute(dgemm_mma<TA, TB, A_T, B_T, TM, TN>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return true;
   }();
@@ -242,41 +263,48 @@ void launch(const GemmArgs& g, const GemmPlan& plan, double* C, long ldc, long s
   const int kps = ((g.K + plan.splits - 1) / plan.splits + TK - 1) / TK * TK;
   const unsigned tm = ceil_div(g.M, TM), tn = ceil_div(g.N, TN);
   const dim3 grid = g.lower ? dim3(tm * (tm + 1) / 2, 1, plan.splits) : dim3(tn, tm, plan.splits);
-  const int vec = (aligned16(g.A, g.lda, sizeof(T)) ? 1 : 0) | (aligned16(g.B, g.ldb, sizeof(T)) ? 2 : 0);
-  dgemm_mma<T, A_T, B_T, TM, TN><<<grid, NT, smem, stream>>>(
-      g.M, g.N, g.K, static_cast<const T*>(g.A), g.lda, static_cast<const T*>(g.B), g.ldb, alpha, beta,
-      C, ldc, stride, kps, g.lower ? 1 : 0, vec);
+  const int vec = (aligned16(g.A, g.lda, sizeof(TA)) ? 1 : 0) | (aligned16(g.B, g.ldb, sizeof(TB)) ? 2 : 0);
+  dgemm_mma<TA, TB, A_T, B_T, TM, TN><<<grid, NT, smem, stream>>>(
+      g.M, g.N, g.K, static_cast<const TA*>(g.A), g.lda, static_cast<const TB*>(g.B), g.ldb, t.alpha,
+      t.beta, t.C, t.ldc, t.stride, kps, g.lower ? 1 : 0, vec, t.coff, g.coff_parts);
   count_launch();
   FPLS_LAUNCH("dgemm_mma");
 }
 
-template <class T, bool A_T, bool B_T>
-void by_tile(const GemmArgs& g, const GemmPlan& pl, double* C, long ldc, long stride, double alpha,
-             double beta, cudaStream_t s) {
-  if (pl.tm == 64) launch<T, A_T, B_T, 64, 64>(g, pl, C, ldc, stride, alpha, beta, s);
-  else if (pl.tn == 128) launch<T, A_T, B_T, 128, 128>(g, pl, C, ldc, stride, alpha, beta, s);
-  else if (pl.tn == 64) launch<T, A_T, B_T, 128, 64>(g, pl, C, ldc, stride, alpha, beta, s);
-  else launch<T, A_T, B_T, 128, 32>(g, pl, C, ldc, stride, alpha, beta, s);
+template <class TA, class TB, bool A_T, bool B_T>
+void by_tile(const GemmArgs& g, const GemmPlan& pl, const Target& t, cudaStream_t s) {
+  if (pl.tm == 64) launch<TA, TB, A_T, B_T, 64, 64>(g, pl, t, s);
+  else if (pl.tn == 128) launch<TA, TB, A_T, B_T, 128, 128>(g, pl, t, s);
+  else if (pl.tn == 64) launch<TA, TB, A_T, B_T, 128, 64>(g, pl, t, s);
+  else if (pl.tn == 32) launch<TA, TB, A_T, B_T, 128, 32>(g, pl, t, s);
+  else launch<TA, TB, A_T, B_T, 128, 16>(g, pl, t, s);
 }
 
 template <class T>
-void by_layout(const GemmArgs& g, const GemmPlan& pl, double* C, long ldc, long stride, double alpha,
-               double beta, cudaStream_t s) {
+void by_layout(const GemmArgs& g, const GemmPlan& pl, const Target& t, cudaStream_t s) {
   if (g.trans_a) {
-    if (g.trans_b) by_tile<T, true, true>(g, pl, C, ldc, stride, alpha, beta, s);
-    else by_tile<T, true, false>(g, pl, C, ldc, stride, alpha, beta, s);
+    if (g.trans_b) by_tile<T, T, true, true>(g, pl, t, s);
+    else by_tile<T, T, true, false>(g, pl, t, s);
   } else {
-    if (g.trans_b) by_tile<T, false, true>(g, pl, C, ldc, stride, alpha, beta, s);
-    else by_tile<T, false, false>(g, pl, C, ldc, stride, alpha, beta, s);
+    if (g.trans_b) by_tile<T, T, false, true>(g, pl, t, s);
+    else by_tile<T, T, false, false>(g, pl, t, s);
   }
 }
 
 }  // namespace
 
 void gemm_mma_launch(const GemmArgs& g, const GemmPlan& plan, double* C, long ldc, long split_stride,
-                     double alpha, double beta, cudaStream_t stream) {
-  if (g.f32) by_layout<float>(g, plan, C, ldc, split_stride, alpha, beta, stream);
-  else by_layout<double>(g, plan, C, ldc, split_stride, alpha, beta, stream);
+                     double alpha, double beta, const double* coff, cudaStream_t stream) {
+  const Target t{C, ldc, split_stride, alpha, beta, coff};
+  if (g.a_type == g.b_type) {
+    require(g.a_type != GemmType::kBf16, "FP64 GEMM: unsupported operand types");
+    if (g.a_type == GemmType::kF32) by_layout<float>(g, plan, t, stream);
+    else by_layout<double>(g, plan, t, stream);
+    return;
+  }
+  require(g.b_type == GemmType::kF64 && !g.trans_a && !g.trans_b, "FP64 GEMM: unsupported operand types");
+  if (g.a_type == GemmType::kF32) by_tile<float, double, false, false>(g, plan, t, stream);
+  else by_tile<bf16, double, false, false>(g, plan, t, stream);
 }
 
 }  // namespace fpls

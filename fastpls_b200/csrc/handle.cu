@@ -297,14 +297,16 @@ class TypedHandle final : public ResidentHandle {
     upload_rows(x, rows);
     score_rows(rows, kmax);
     const int q = model_.m;
-    pred_.reserve((size_t)rows * q, stream_);
-    conv_.reserve((size_t)rows * q, stream_);
+    const size_t block = (size_t)rows * q;
+    const int step = prefixes_at_once(block * sizeof(TO), count);
+    conv_.reserve(block * step, stream_);
     TO* dst = static_cast<TO*>(out);
-    for (int j = 0; j < count; ++j) {
-      const int k = prefixes[j];
-      if (lda) lda_state().discriminants(scores_.get(), rows, rows, k, pred_.get(), rows, stream_);
-      else predict_from_scores(model_, scores_.get(), rows, rows, k, pred_.get(), rows, stream_);
-      download(pred_.get(), (long)rows * q, dst + (size_t)j * rows * q);
+    for (int j = 0; j < count; j += step) {
+      const int w = std::min(step, count - j);
+      if (lda) lda_state().discriminants(scores_.get(), rows, rows, prefixes + j, w, conv_.get(), stream_);
+      else predict_prefixes<TO>(model_, scores_.get(), rows, rows, prefixes + j, w, conv_.get(), stream_);
+      FPLS_CHECK(cudaMemcpyAsync(dst + j * block, conv_.get(), sizeof(TO) * block * w,
+                                 cudaMemcpyDeviceToHost, stream_));
     }
     FPLS_CHECK(cudaStreamSynchronize(stream_));
   }
@@ -320,26 +322,25 @@ class TypedHandle final : public ResidentHandle {
     const int kmax = prefixes[count - 1];
     upload_rows(x, rows);
     score_rows(rows, kmax);
-    pred_.reserve((size_t)rows * q, stream_);
-    disc_.reserve((size_t)rows * q, stream_);
-    conv_.reserve((size_t)rows * q, stream_);
-    top_.reserve((size_t)rows * top, stream_);
+    const size_t block = (size_t)rows * q;
+    const int step = prefixes_at_once(block * sizeof(double), count);
+    pred_.reserve(block * step, stream_);
+    top_.reserve((size_t)rows * top * step, stream_);
     TO* resp = static_cast<TO*>(response_out);
-    for (int j = 0; j < count; ++j) {
-      const int k = prefixes[j];
-      const double* decoded = pred_.get();
-      if (!lda || resp) {
-        predict_from_scores(model_, scores_.get(), rows, rows, k, pred_.get(), rows, stream_);
-        if (resp) download(pred_.get(), (long)rows * q, resp + (size_t)j * rows * q);
-      }
-      if (lda) {
-        lda_state().discriminants(scores_.get(), rows, rows, k, disc_.get(), rows, stream_);
-        decoded = disc_.get();
-      }
-      topk_rows(decoded, rows, q, top, top_.get(), rows, stream_);
-      FPLS_CHECK(cudaMemcpyAsync(out + (size_t)j * rows * top, top_.get(),
-                                 sizeof(int) * rows * top,
+    for (int j = 0; j < count; j += step) {
+      const int w = std::min(step, count - j);
+      // the decoded values stay FP64; the responses go out in the result type
+      if (lda) lda_state().discriminants(scores_.get(), rows, rows, prefixes + j, w, pred_.get(), stream_);
+      else predict_prefixes<double>(model_, scores_.get(), rows, rows, prefixes + j, w, pred_.get(), stream_);
+      topk_rows(pred_.get(), rows, q, top, w, top_.get(), rows, stream_);
+      FPLS_CHECK(cudaMemcpyAsync(out + (size_t)j * rows * top, top_.get(), sizeof(int) * rows * top * w,
                                  cudaMemcpyDeviceToHost, stream_));
+      if (resp) {
+        conv_.reserve(block * step, stream_);
+        predict_prefixes<TO>(model_, scores_.get(), rows, rows, prefixes + j, w, conv_.get(), stream_);
+        FPLS_CHECK(cudaMemcpyAsync(resp + j * block, conv_.get(), sizeof(TO) * block * w,
+                                   cudaMemcpyDeviceToHost, stream_));
+      }
     }
     FPLS_CHECK(cudaStreamSynchronize(stream_));
   }
@@ -365,7 +366,7 @@ class TypedHandle final : public ResidentHandle {
     upload_rows(x, rows);
     score_rows(rows, prefix);
     pred_.reserve((size_t)rows * q, stream_);
-    predict_from_scores(model_, scores_.get(), rows, rows, prefix, pred_.get(), rows, stream_);
+    predict_prefixes<double>(model_, scores_.get(), rows, rows, &prefix, 1, pred_.get(), stream_);
     DeviceArray<TO> yd;
     DeviceArray<int> ld;
     if (labels) {
@@ -606,7 +607,6 @@ class TypedHandle final : public ResidentHandle {
       from = conv_.get();
     }
     FPLS_CHECK(cudaMemcpyAsync(dst, from, sizeof(TO) * count, cudaMemcpyDeviceToHost, stream_));
-    if (!std::is_same<TO, double>::value) FPLS_CHECK(cudaStreamSynchronize(stream_));
   }
 
   LdaState& lda_state() {
@@ -688,7 +688,6 @@ class TypedHandle final : public ResidentHandle {
     xbuf_.release();
     scores_.release();
     pred_.release();
-    disc_.release();
     conv_.release();
     top_.release();
     loadings_.release();
@@ -706,7 +705,7 @@ class TypedHandle final : public ResidentHandle {
   Workspace ws_;
   DeviceArray<T> xtrain_, xbuf_;
   DeviceArray<TO> conv_;
-  DeviceArray<double> scores_, pred_, disc_, loadings_, var_ss_, design_;
+  DeviceArray<double> scores_, pred_, loadings_, var_ss_, design_;
   DeviceArray<int> top_;
   std::unique_ptr<LdaState> lda_;
   std::unique_ptr<PersistentPlan> pending_;

@@ -28,18 +28,26 @@ __global__ void one_hot_kernel(const int* __restrict__ labels, int n, int c,
   }
 }
 
-// One block: pooled covariance for the first k components, ridge retries,
-// linear (c x k, row-major per class) and constants (c).
-__global__ void lda_finalize(const double* __restrict__ gram, int a,
-                             const double* __restrict__ sums, int c,
-                             const double* __restrict__ counts, int n, int k,
-                             double* linear, double* constants, double* ridge,
-                             int* flag) {
+// One block per prefix: pooled covariance for its first k components, ridge
+// retries, linear (c x k) and constants (c). Latency-bound; the factor by the
+// whole block and one class per thread in the solves, every prefix of a call
+// in one launch (a serial thread per launch took 43 us a prefix at k <= 9, 10
+// classes; 14 us for four prefixes so).
+constexpr int kLdaBatch = 32;
+struct LdaJobs {
+  int k[kLdaBatch];
+  double* linear[kLdaBatch];
+  double* constants[kLdaBatch];
+};
+__global__ void lda_finalize(const double* __restrict__ gram, int a, const double* __restrict__ sums,
+                             int c, const double* __restrict__ counts, int n, LdaJobs jobs, int* flag) {
   extern __shared__ double sm[];
+  const int k = jobs.k[blockIdx.x];
+  double* linear = jobs.linear[blockIdx.x];
+  double* constants = jobs.constants[blockIdx.x];
   double* cov = sm;                 // k x k
   double* L = cov + k * k;          // k x k
   double* means = L + k * k;        // c x k (class-major)
-  double* rhs = means + c * k;      // k
   const int t = threadIdx.x;
   for (int idx = t; idx < c * k; idx += blockDim.x) {
     const int cls = idx / k, j = idx % k;
@@ -54,43 +62,30 @@ __global__ void lda_finalize(const double* __restrict__ gram, int a,
     cov[i + j * k] = v / denom;
   }
   __syncthreads();
-  if (t == 0) {
-    double scale = 0.0;
-    for (int i = 0; i < k; ++i) scale += cov[i + i * k];
-    scale /= k;
-    if (!isfinite(scale) || scale <= 0.0) scale = 1.0;
-    const double grid[6] = {1e-8, 1e-6, 1e-5, 1e-4, 1e-3, 1e-2};
-    bool solved = false;
-    for (int g = 0; g < 6 && !solved; ++g) {
-      for (int idx = 0; idx < k * k; ++idx) L[idx] = cov[idx];
-      if (!cholesky_serial(L, k, grid[g] * scale)) continue;
-      bool ok = true;
-      for (int cls = 0; cls < c && ok; ++cls) {
-        for (int j = 0; j < k; ++j) rhs[j] = means[cls * k + j];
-        ok = cholesky_solve_serial(L, k, rhs);
-        for (int j = 0; j < k; ++j) linear[cls + (long)j * c] = rhs[j];
-      }
-      if (!ok) continue;
-      solved = true;
-      *ridge = grid[g] * scale;
+  double scale = 0.0;
+  for (int i = 0; i < k; ++i) scale += cov[i + i * k];
+  scale /= k;
+  if (!isfinite(scale) || scale <= 0.0) scale = 1.0;
+  const double grid[6] = {1e-8, 1e-6, 1e-5, 1e-4, 1e-3, 1e-2};
+  bool solved = false;
+  for (int g = 0; g < 6 && !solved; ++g) {
+    __syncthreads();
+    for (int idx = t; idx < k * k; idx += blockDim.x) L[idx] = cov[idx];
+    if (!cholesky_block(L, k, grid[g] * scale)) continue;
+    int ok = 1;
+    for (int cls = t; cls < c; cls += blockDim.x) {
+      for (int j = 0; j < k; ++j) linear[cls + (long)j * c] = means[cls * k + j];
+      if (!cholesky_solve_strided(L, k, linear + cls, c)) ok = 0;
     }
-    if (!solved) flag_error(flag, 5);
-    for (int cls = 0; cls < c; ++cls) {
-      double prod = 0.0;
-      for (int j = 0; j < k; ++j) prod += means[cls * k + j] * linear[cls + (long)j * c];
-      const double prior = counts[cls] / n;
-      constants[cls] = -0.5 * prod + log(fmax(prior, DBL_MIN));
-    }
+    solved = __syncthreads_and(ok) != 0;
+    if (solved && t == 0) constants[c] = grid[g] * scale;
   }
-}
-
-__global__ void fill_constants(double* out, int rows, int c, long ldo,
-                               const double* constants) {
-  const long total = (long)rows * c;
-  for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(idx % rows), k = (int)(idx / rows);
-    out[i + (long)k * ldo] = constants[k];
+  if (!solved && t == 0) flag_error(flag, 5);
+  for (int cls = t; cls < c; cls += blockDim.x) {
+    double prod = 0.0;
+    for (int j = 0; j < k; ++j) prod += means[cls * k + j] * linear[cls + (long)j * c];
+    const double prior = counts[cls] / n;
+    constants[cls] = -0.5 * prod + log(fmax(prior, DBL_MIN));
   }
 }
 
@@ -140,48 +135,62 @@ void LdaState::train(const double* scores, int n_, long lds, int a_,
   prefixes.clear();
 }
 
-const LdaState::Prefix& LdaState::prefix(int k, cudaStream_t stream) {
-  require(k >= 1 && k <= a, "invalid LDA prefix");
-  for (auto& pr : prefixes)
-    if (pr.k == k) return pr;
-  prefixes.emplace_back();
-  Prefix& pr = prefixes.back();
-  pr.k = k;
-  pr.linear.allocate((size_t)c * k, stream);
-  pr.constants.allocate(c + 1, stream);
-  const size_t smem = (2 * (size_t)k * k + (size_t)c * k + k) * sizeof(double);
-  if (smem > 48 * 1024)
-    FPLS_CHECK(cudaFuncSetAttribute(lda_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  lda_finalize<<<1, 256, smem, stream>>>(gram.get(), a, sums.get(), c,
-                                         counts_dev.get(), n, k,
-                                         pr.linear.get(), pr.constants.get(),
-                                         pr.constants.get() + c, flag);
-  count_launch();
-  FPLS_LAUNCH("lda_finalize");
-  return pr;
+void LdaState::finalize(const int* ks, int count, cudaStream_t stream) {
+  LdaJobs jobs;
+  int pending = 0, kmax = 0;
+  auto flush = [&] {
+    if (pending == 0) return;
+    const size_t smem = (2 * (size_t)kmax * kmax + (size_t)c * kmax) * sizeof(double);
+    if (smem > 48 * 1024)
+      FPLS_CHECK(cudaFuncSetAttribute(lda_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    lda_finalize<<<pending, 256, smem, stream>>>(gram.get(), a, sums.get(), c, counts_dev.get(), n, jobs, flag);
+    count_launch();
+    FPLS_LAUNCH("lda_finalize");
+    pending = kmax = 0;
+  };
+  for (int j = 0; j < count; ++j) {
+    const int k = ks[j];
+    require(k >= 1 && k <= a, "invalid LDA prefix");
+    if (find(k)) continue;
+    prefixes.emplace_back();
+    Prefix& pr = prefixes.back();
+    pr.k = k;
+    pr.linear.allocate((size_t)c * k, stream);
+    pr.constants.allocate(c + 1, stream);
+    jobs.k[pending] = k;
+    jobs.linear[pending] = pr.linear.get();
+    jobs.constants[pending] = pr.constants.get();
+    kmax = std::max(kmax, k);
+    if (++pending == kLdaBatch) flush();
+  }
+  flush();
 }
 
-void LdaState::discriminants(const double* scores, int rows, long lds, int k,
-                             double* out, long ldo, cudaStream_t stream) {
-  const Prefix& pr = prefix(k, stream);
-  const long total = (long)rows * c;
-  fill_constants<<<(unsigned)std::min<long>((total + 255) / 256, 8L * num_sms()), 256, 0, stream>>>(
-      out, rows, c, ldo, pr.constants.get());
-  count_launch();
-  FPLS_LAUNCH("fill_constants");
-  GemmArgs g;
-  g.M = rows;
-  g.N = c;
-  g.K = k;
-  g.A = scores;
-  g.lda = lds;
-  g.B = pr.linear.get();  // c x k: op(B) = linear^T (k x c)
-  g.ldb = c;
-  g.trans_b = true;
-  g.C = out;
-  g.ldc = ldo;
-  g.beta = 1.0;
-  gemm_f64(g, stream);
+const LdaState::Prefix* LdaState::find(int k) const {
+  for (const auto& pr : prefixes)
+    if (pr.k == k) return &pr;
+  return nullptr;
+}
+
+void LdaState::discriminants(const double* scores, int rows, long lds, const int* ks, int count,
+                             double* out, cudaStream_t stream) {
+  finalize(ks, count, stream);
+  apply_prefix_maps<double>(scores, rows, lds, c, maps(ks, count).data(), count, out, stream);
+}
+
+void LdaState::discriminants(const double* scores, int rows, long lds, const int* ks, int count,
+                             float* out, cudaStream_t stream) {
+  finalize(ks, count, stream);
+  apply_prefix_maps<float>(scores, rows, lds, c, maps(ks, count).data(), count, out, stream);
+}
+
+std::vector<PrefixMap> LdaState::maps(const int* ks, int count) const {
+  std::vector<PrefixMap> out(count);
+  for (int j = 0; j < count; ++j) {
+    const Prefix* pr = find(ks[j]);
+    out[j] = {pr->k, pr->linear.get(), pr->constants.get(), c, 1};
+  }
+  return out;
 }
 
 }  // namespace fpls

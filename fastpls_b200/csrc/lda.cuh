@@ -2,6 +2,7 @@
 #pragma once
 
 #include "kernels.cuh"
+#include "model.cuh"
 
 #include <deque>
 #include <vector>
@@ -25,10 +26,17 @@ struct LdaState {
   void train(const double* scores, int n, long lds, int a, const int* labels,
              int c, const std::vector<int>& counts, int* flag,
              cudaStream_t stream);
-  const Prefix& prefix(int k, cudaStream_t stream);
-  // out (rows x c) = constants + scores_k linear^T
-  void discriminants(const double* scores, int rows, long lds, int k,
-                     double* out, long ldo, cudaStream_t stream);
+  // per prefix k of ks a column-major rows x c block: constants + scores_k linear^T
+  void discriminants(const double* scores, int rows, long lds, const int* ks, int count, double* out,
+                     cudaStream_t stream);
+  void discriminants(const double* scores, int rows, long lds, const int* ks, int count, float* out,
+                     cudaStream_t stream);
+
+ private:
+  // the terms of every prefix of ks not there yet
+  void finalize(const int* ks, int count, cudaStream_t stream);
+  const Prefix* find(int k) const;
+  std::vector<PrefixMap> maps(const int* ks, int count) const;
 };
 
 }  // namespace fpls

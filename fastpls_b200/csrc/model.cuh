@@ -148,10 +148,31 @@ void project_rows(const DeviceModel& model, const T* X, int rows, long ld,
                   int k, double* out, long ldo, Workspace& ws,
                   cudaStream_t stream);
 
-// Responses for prefix k from scores (rows x >= k): out = ymean + T_k B_k.
-void predict_from_scores(const DeviceModel& model, const double* scores,
-                         int rows, long lds, int k, double* out, long ldo,
-                         cudaStream_t stream);
+// Responses from scores (rows x max prefix, column stride lds): for each of
+// the `count` increasing prefixes k a column-major rows x m block ymean + T_k
+// B_k at out + j rows m, in the result type.
+template <class TO>
+void predict_prefixes(const DeviceModel& model, const double* scores, int rows, long lds,
+                      const int* prefixes, int count, TO* out, cudaStream_t stream);
+
+// Affine maps of the leading scores, one per prefix: out block j, entry (row,
+// r) = base[r] + sum_{c < k} T[row, c] w[c * stride_c + r * stride_r].
+struct PrefixMap {
+  int k;
+  const double* w;
+  const double* base;
+  int stride_c, stride_r;
+};
+template <class TO>
+void apply_prefix_maps(const double* scores, int rows, long lds, int m, const PrefixMap* maps,
+                       int count, TO* out, cudaStream_t stream);
+
+// Prefixes to evaluate at a time so that `bytes` per prefix stay within a
+// workspace of 256 MB (at least one).
+inline int prefixes_at_once(size_t bytes, int count) {
+  const size_t cap = size_t(256) << 20;
+  return (int)std::max<size_t>(1, std::min<size_t>((size_t)count, cap / std::max<size_t>(bytes, 1)));
+}
 
 // Throws when the device error flag was raised (synchronises the stream).
 void raise_on_flag(Workspace& ws, cudaStream_t stream, const char* message);

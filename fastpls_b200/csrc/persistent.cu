@@ -1219,16 +1219,16 @@ void launch_persistent(const std::vector<PersistentPlan*>& plans, cudaStream_t s
 namespace {
 
 // out[i + b ldo] = sum over the column ranges k (in order) of
-// part[(k nb + b) n + i] - offset[b].
+// part[(k nb + b) n + i] - offset of column b.
 __global__ void ring_finish(const double* __restrict__ part, int ranges, int n, int nb,
-                            const double* offset, double* out, long ldo) {
+                            const double* offset, int offset_parts, double* out, long ldo) {
   const long total = (long)n * nb;
   for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
        idx += (long)gridDim.x * blockDim.x) {
     const int i = (int)(idx % n), b = (int)(idx / n);
     double v = 0.0;
     for (int k = 0; k < ranges; ++k) v += part[((long)k * nb + b) * n + i];
-    if (offset) v -= offset[b];
+    if (offset) v -= column_offset(offset, offset_parts, b);
     out[i + (long)b * ldo] = v;
   }
 }
@@ -1250,7 +1250,7 @@ void launch_xr_ring(const Fit& f, const double* Rt, int nb, double* part, cudaSt
 
 template <class T>
 bool xr_ring(const T* X, int n, int p, long ld, const double* R, long ldr, int nb,
-             const double* offset, double* out, long ldo, int* flag, cudaStream_t s) {
+             const double* offset, int offset_parts, double* out, long ldo, int* flag, cudaStream_t s) {
   if (nb < 3 || nb > 16 || n < 1 || p < 1) return false;
   const int NB = nb <= 4 ? 4 : nb <= 8 ? 8 : nb <= 10 ? 10 : nb <= 12 ? 12 : 16;
   // row blocks of at most kBlockRows rows, about one wave of two CTAs per SM
@@ -1285,18 +1285,18 @@ bool xr_ring(const T* X, int n, int p, long ld, const double* R, long ldr, int n
   }
   const long total = (long)n * nb;
   ring_finish<<<(unsigned)std::min<long>((total + 255) / 256, 8L * num_sms()), 256, 0, s>>>(
-      part.get(), Cc, n, nb, offset, out, ldo);
+      part.get(), Cc, n, nb, offset, offset_parts, out, ldo);
   count_launch();
   FPLS_LAUNCH("ring_finish");
   return true;
 }
 
-template bool xr_ring<float>(const float*, int, int, long, const double*, long, int, const double*,
+template bool xr_ring<float>(const float*, int, int, long, const double*, long, int, const double*, int,
                              double*, long, int*, cudaStream_t);
-template bool xr_ring<double>(const double*, int, int, long, const double*, long, int, const double*,
-                              double*, long, int*, cudaStream_t);
-template bool xr_ring<bf16>(const bf16*, int, int, long, const double*, long, int, const double*,
-                            double*, long, int*, cudaStream_t);
+template bool xr_ring<double>(const double*, int, int, long, const double*, long, int, const double*, int,
+                             double*, long, int*, cudaStream_t);
+template bool xr_ring<bf16>(const bf16*, int, int, long, const double*, long, int, const double*, int,
+                             double*, long, int*, cudaStream_t);
 
 template bool plan_simpls_persistent<float>(const float*, int, int, long, int, int, DeviceModel&,
                                             DeviceArray<double>&, double*, Workspace&, cudaStream_t,

@@ -66,46 +66,25 @@ __global__ void small_svd_kernel(const double* __restrict__ gpk, int m, int k,
   }
 }
 
-// Cholesky of the score Gram once; thread j forms the prefix (j+1) weights
-// W_{j+1} = G_{j+1}^-1 diag(sigma_1..j+1) V_{j+1}^T into its own block.
-__global__ void plssvd_weights_kernel(const double* __restrict__ gram, int a,
-                                      const double* __restrict__ sigma,
-                                      const double* __restrict__ Vk, int m,
-                                      double* W, double* lwork, int* flag) {
-  __shared__ bool ok;
-  if (threadIdx.x == 0) {
-    for (int idx = 0; idx < a * a; ++idx) lwork[idx] = gram[idx];
-    ok = cholesky_serial(lwork, a, 0.0);
-    if (!ok) flag_error(flag, 6);
+// Block k - 1: the prefix-k weights W_k = G_k^-1 diag(sigma_1..k) V_k^T (k x m)
+// from the Cholesky factor of the leading k x k block of the score Gram, one
+// response column per thread. Latency-bound; one thread per prefix with a
+// serial factor took 126 us at k = 9, 10 responses, 13 us so.
+constexpr int kWeightThreads = 128;
+__global__ void __launch_bounds__(kWeightThreads)
+    plssvd_weights_kernel(const double* __restrict__ gram, int a, const double* __restrict__ sigma,
+                          const double* __restrict__ Vk, int m, double* W, int* flag) {
+  extern __shared__ double L[];  // k x k
+  const int k = blockIdx.x + 1;
+  for (int e = threadIdx.x; e < k * k; e += blockDim.x) L[e] = gram[e % k + (long)(e / k) * a];
+  if (!cholesky_block(L, k, 0.0)) {
+    if (threadIdx.x == 0) flag_error(flag, 6);
+    return;
   }
-  __syncthreads();
-  if (!ok) return;
-  for (int j = threadIdx.x; j < a; j += blockDim.x) {
-    const int k = j + 1;
-    double* Wk = W + (size_t)j * a * m;  // k x m, ld k
-    double col[128];
-    for (int c = 0; c < k; ++c) {
-      // latent column c: solve L_k L_k^T x = sigma_c e_c (L_k = leading block)
-      for (int i = 0; i < k; ++i) col[i] = (i == c) ? sigma[c] : 0.0;
-      for (int i = 0; i < k; ++i) {
-        double v = col[i];
-        for (int q = 0; q < i; ++q) v -= lwork[i + q * a] * col[q];
-        col[i] = v / lwork[i + i * a];
-      }
-      for (int i = k - 1; i >= 0; --i) {
-        double v = col[i];
-        for (int q = i + 1; q < k; ++q) v -= lwork[q + i * a] * col[q];
-        col[i] = v / lwork[i + i * a];
-      }
-      // W_k[:, r] += latent[:, c] * V[r, c]
-      for (int r = 0; r < m; ++r) {
-        const double vr = Vk[r + c * m];
-        for (int i = 0; i < k; ++i) {
-          const double prev = (c == 0) ? 0.0 : Wk[i + r * k];
-          Wk[i + r * k] = prev + col[i] * vr;
-        }
-      }
-    }
+  double* Wk = W + (size_t)(k - 1) * a * m;
+  for (int r = threadIdx.x; r < m; r += blockDim.x) {
+    for (int c = 0; c < k; ++c) Wk[c + (long)r * k] = sigma[c] * Vk[r + c * m];
+    cholesky_solve_strided(L, k, Wk + (long)r * k, 1);
   }
 }
 
@@ -174,10 +153,11 @@ void fit_plssvd(const T* X, int n, int p, long ld, const double* Yc,
   h.ldc = k;
   gemm_f64(h, stream);
   model.W.allocate((size_t)k * k * m, stream);
-  DeviceArray<double> lwork((size_t)k * k, stream);
-  plssvd_weights_kernel<<<1, 128, 0, stream>>>(gram.get(), k, model.sigma.get(),
-                                               model.Q.get(), m, model.W.get(),
-                                               lwork.get(), ws.flag.get());
+  const size_t smem_w = (size_t)k * k * sizeof(double);
+  if (smem_w > 48 * 1024)
+    FPLS_CHECK(cudaFuncSetAttribute(plssvd_weights_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_w));
+  plssvd_weights_kernel<<<k, kWeightThreads, smem_w, stream>>>(gram.get(), k, model.sigma.get(), model.Q.get(),
+                                                               m, model.W.get(), ws.flag.get());
   count_launch();
   FPLS_LAUNCH("plssvd_weights");
 }

@@ -387,6 +387,49 @@ __device__ inline bool cholesky_serial(double* A, int k, double ridge) {
   return true;
 }
 
+// The same factorisation by the whole block (A in shared memory; every thread
+// calls it and receives the result): right-looking, the trailing columns
+// updated element by element after each pivot.
+__device__ inline bool cholesky_block(double* A, int k, double ridge) {
+  __syncthreads();
+  for (int i = threadIdx.x; i < k; i += blockDim.x) A[i + i * k] += ridge;
+  __syncthreads();
+  for (int j = 0; j < k; ++j) {
+    const double piv = A[j + j * k];
+    if (!(piv > 0.0) || !isfinite(piv)) return false;  // the same value in every thread
+    const double d = sqrt(piv);
+    __syncthreads();
+    for (int i = j + threadIdx.x; i < k; i += blockDim.x) A[i + j * k] = i == j ? d : A[i + j * k] / d;
+    __syncthreads();
+    const int left = k - 1 - j;
+    for (int e = threadIdx.x; e < left * left; e += blockDim.x) {
+      const int i = j + 1 + e % left, c = j + 1 + e / left;
+      if (i >= c) A[i + c * k] = fma(-A[i + j * k], A[c + j * k], A[i + c * k]);
+    }
+    __syncthreads();
+  }
+  return true;
+}
+
+// Solve L L^T x = b in place for b[i * stride] (L lower, k x k,
+// column-major), one thread.
+__device__ inline bool cholesky_solve_strided(const double* L, int k, double* b, long stride) {
+  for (int i = 0; i < k; ++i) {
+    double v = b[i * stride];
+    for (int q = 0; q < i; ++q) v -= L[i + q * k] * b[q * stride];
+    b[i * stride] = v / L[i + i * k];
+  }
+  bool ok = true;
+  for (int i = k - 1; i >= 0; --i) {
+    double v = b[i * stride];
+    for (int q = i + 1; q < k; ++q) v -= L[q + i * k] * b[q * stride];
+    v /= L[i + i * k];
+    b[i * stride] = v;
+    ok = ok && isfinite(v);
+  }
+  return ok;
+}
+
 // Solve L L^T x = b in place (L lower, k x k, column-major), one thread.
 __device__ inline bool cholesky_solve_serial(const double* L, int k, double* b) {
   for (int i = 0; i < k; ++i) {

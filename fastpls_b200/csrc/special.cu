@@ -247,7 +247,7 @@ void fit_opls(const T* X, int n, int p, long ld, const double* Yc,
     gram_of_columns(S.get(), p, m, gpk, ws, s);
     dominant_direction(S.get(), p, m, gpk, zs, w.get(), ws, s);
     // t = Xf w ; p = Xf^T t / t't ; wo = normalise(p - (w'p / w'w) w)
-    xr_product<double>(xf, n, p, n, w.get(), p, 1, nullptr, t.get(), n, ws.stream_partial, s);
+    xr_product<double>(xf, n, p, n, w.get(), p, 1, nullptr, 1, t.get(), n, ws.stream_partial, s);
     xtv_product<double>(xf, n, p, n, t.get(), n, 1, pv.get(), p, ws.stream_partial, s);
     dot_kernel<<<gd, TB, 0, s>>>(t.get(), t.get(), n, part, ctr, sc.get());
     scale_vec<<<gd, TB, 0, s>>>(pv.get(), p, sc.get(), 1, ws.flag.get());
@@ -261,7 +261,7 @@ void fit_opls(const T* X, int n, int p, long ld, const double* Yc,
     FPLS_LAUNCH("opls filter direction");
     // t_o = Xf wo ; p_o = Xf^T t_o / t_o't_o ; Xf -= t_o p_o^T
     double* po = Po.get() + (size_t)c * p;
-    xr_product<double>(xf, n, p, n, wo, p, 1, nullptr, t.get(), n, ws.stream_partial, s);
+    xr_product<double>(xf, n, p, n, wo, p, 1, nullptr, 1, t.get(), n, ws.stream_partial, s);
     xtv_product<double>(xf, n, p, n, t.get(), n, 1, po, p, ws.stream_partial, s);
     dot_kernel<<<gd, TB, 0, s>>>(t.get(), t.get(), n, part, ctr + 4, sc.get() + 4);
     scale_vec<<<gd, TB, 0, s>>>(po, p, sc.get() + 4, 1, ws.flag.get());

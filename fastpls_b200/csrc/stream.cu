@@ -448,27 +448,26 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 __global__ void xr_finish(const double* __restrict__ partial, int chunks, int n,
-                          int nb, const double* offset, double* out, long ldo) {
+                          int nb, const double* offset, int offset_parts, double* out, long ldo) {
   const long total = (long)n * nb;
   for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
        idx += (long)gridDim.x * blockDim.x) {
     const int i = (int)(idx % n), c = (int)(idx / n);
     double v = 0.0;
     for (int k = 0; k < chunks; ++k) v += partial[(long)k * n * nb + idx];
-    if (offset) v -= offset[c];
+    if (offset) v -= column_offset(offset, offset_parts, c);
     out[i + (long)c * ldo] = v;
   }
 }
 
 template <class T, int NB>
 void xr_launch(const T* X, int n, int p, long ld, const double* R, long ldr,
-               int nb, const double* offset, double* out, long ldo,
+               int nb, const double* offset, int offset_parts, double* out, long ldo,
                DeviceArray<double>& scratch, cudaStream_t stream) {
-  // 16-byte row vectors for the one- and two-column products (HBM-bound);
-  // wider products are FP64-issue-bound and keep two rows per thread. The
-  // column chunks depend on n and p only (a nominal 1024-row tile), so every
+  static_assert(NB <= 2, "wider products run on the FP64 tensor path");
+  // 16-byte row vectors where the column stride allows. The column chunks depend on n and p only (a nominal 1024-row tile), so every
   // storage type and both kernels sum each row in the same order.
-  const bool vec = NB <= 2 && ld % 8 == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0;
+  const bool vec = ld % 8 == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0;
   const int nominal_tiles = (int)ceil_div(n, 1024);
   const int want = 16 * num_sms();
   int chunks = std::max(1, std::min((int)ceil_div(want, nominal_tiles), (int)ceil_div(p, 64)));
@@ -477,22 +476,17 @@ void xr_launch(const T* X, int n, int p, long ld, const double* R, long ldr,
   chunks = (int)ceil_div(p, cc);
   scratch.reserve((size_t)chunks * n * nb, stream);
   const size_t smem = (size_t)cc * NB * sizeof(double);
-  bool launched = false;
-  if constexpr (NB <= 2) {
-    if (vec) {
-      xr_vec_kernel<T, NB><<<dim3(ceil_div(n, kThreads * Vec16<T>::V), chunks), kThreads, smem,
-                             stream>>>(X, n, p, ld, R, ldr, nb, cc, scratch.get());
-      launched = true;
-    }
-  }
-  if (!launched)
+  if (vec)
+    xr_vec_kernel<T, NB><<<dim3(ceil_div(n, kThreads * Vec16<T>::V), chunks), kThreads, smem,
+                           stream>>>(X, n, p, ld, R, ldr, nb, cc, scratch.get());
+  else
     xr_kernel<T, NB><<<dim3(ceil_div(n, 2 * kThreads), chunks), kThreads, smem, stream>>>(
         X, n, p, ld, R, ldr, nb, cc, scratch.get());
   count_launch();
   FPLS_LAUNCH("xr_kernel");
   const long total = (long)n * nb;
   const unsigned blocks = (unsigned)std::min<long>((total + 255) / 256, 8L * num_sms());
-  xr_finish<<<blocks, 256, 0, stream>>>(scratch.get(), chunks, n, nb, offset, out, ldo);
+  xr_finish<<<blocks, 256, 0, stream>>>(scratch.get(), chunks, n, nb, offset, offset_parts, out, ldo);
   count_launch();
   FPLS_LAUNCH("xr_finish");
 }
@@ -514,6 +508,8 @@ __global__ void topk_kernel(const double* __restrict__ v, int rows, int classes,
                             int top, int* __restrict__ out, long ldo) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= rows) return;
+  v += (long)blockIdx.y * rows * classes;  // prefix blockIdx.y
+  out += (long)blockIdx.y * ldo * top;
   // repeated strict-'>' scans: the lowest index wins ties, ranks are distinct
   unsigned long long used_lo = 0ull;
   for (int k = 0; k < top; ++k) {
@@ -700,25 +696,11 @@ void xtv_product(const T* X, int n, int p, long ld, const double* V, long ldv,
 
 template <class T>
 void xr_product(const T* X, int n, int p, long ld, const double* R, long ldr,
-                int nb, const double* offset, double* out, long ldo,
-                DeviceArray<double>& scratch, cudaStream_t stream, int* flag) {
-  // 3..16 columns of a large X: one pass over X on bulk-copy stages instead
-  // of a pass per 8 columns
-  if (nb >= 3 && nb <= 16 && (long)n * p >= (1L << 24) &&
-      xr_ring<T>(X, n, p, ld, R, ldr, nb, offset, out, ldo, flag, stream))
-    return;
-  for (int c0 = 0; c0 < nb; c0 += 8) {
-    const int w = std::min(8, nb - c0);
-    const double* off = offset ? offset + c0 : nullptr;
-    if (w == 1)
-      xr_launch<T, 1>(X, n, p, ld, R + (long)c0 * ldr, ldr, w, off, out + (long)c0 * ldo, ldo, scratch, stream);
-    else if (w <= 2)
-      xr_launch<T, 2>(X, n, p, ld, R + (long)c0 * ldr, ldr, w, off, out + (long)c0 * ldo, ldo, scratch, stream);
-    else if (w <= 4)
-      xr_launch<T, 4>(X, n, p, ld, R + (long)c0 * ldr, ldr, w, off, out + (long)c0 * ldo, ldo, scratch, stream);
-    else
-      xr_launch<T, 8>(X, n, p, ld, R + (long)c0 * ldr, ldr, w, off, out + (long)c0 * ldo, ldo, scratch, stream);
-  }
+                int nb, const double* offset, int offset_parts, double* out, long ldo,
+                DeviceArray<double>& scratch, cudaStream_t stream) {
+  require(nb == 1 || nb == 2, "streamed X R takes one or two columns");
+  if (nb == 1) xr_launch<T, 1>(X, n, p, ld, R, ldr, nb, offset, offset_parts, out, ldo, scratch, stream);
+  else xr_launch<T, 2>(X, n, p, ld, R, ldr, nb, offset, offset_parts, out, ldo, scratch, stream);
 }
 
 template <class T>
@@ -732,10 +714,10 @@ void gather_rows(const T* src, long ld_src, int cols, const int* idx, int count,
   FPLS_LAUNCH("gather_rows");
 }
 
-void topk_rows(const double* values, int rows, int classes, int top, int* out,
+void topk_rows(const double* values, int rows, int classes, int top, int count, int* out,
                long ldo, cudaStream_t stream) {
-  if (rows <= 0) return;
-  topk_kernel<<<ceil_div(rows, 128), 128, 0, stream>>>(values, rows, classes, top, out, ldo);
+  if (rows <= 0 || count <= 0) return;
+  topk_kernel<<<dim3(ceil_div(rows, 128), count), 128, 0, stream>>>(values, rows, classes, top, out, ldo);
   count_launch();
   FPLS_LAUNCH("topk_rows");
 }
@@ -751,8 +733,8 @@ void topk_rows(const double* values, int rows, int classes, int top, int* out,
                                int, double*, long, DeviceArray<double>&,      \
                                cudaStream_t);                                 \
   template void xr_product<T>(const T*, int, int, long, const double*, long,  \
-                              int, const double*, double*, long,              \
-                              DeviceArray<double>&, cudaStream_t, int*);      \
+                              int, const double*, int, double*, long,         \
+                              DeviceArray<double>&, cudaStream_t);            \
   template void gather_rows<T>(const T*, long, int, const int*, int, T*,      \
                                long, cudaStream_t);
 FPLS_INSTANTIATE(float)

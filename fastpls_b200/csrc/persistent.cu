@@ -10,20 +10,20 @@
 // grid of CTAs stays resident for the whole fit and walks through the
 // phases of each component, separated by group barriers:
 //
-//   B0  (last CTA) reduce the Gram of the deflated S, Jacobi -> z / sqrt(lambda)
-//   P1  r = S z, rt = r / scale, partial  c = mean . rt             -> B1: c
-//   P2  t partials over column chunks: sum_j X[i, j] rt[j]          -> B2
-//   P3  t = sum of partials - c, partial |t|^2 and sum t            -> B3: |t|, sum t
-//   P4  loading partials over row chunks: sum_i X[i, j] t[i]        -> B4
+//   B0  Gram and u = S^T (mean / scale) of the deflated S summed, dominant
+//       pair -> z / sqrt(lambda), score offset c = z . u
+//   P2  t partials over column ranges: sum_j X[i, j] (S z)_j / scale_j  -> B2
+//   P4  t = sum of partials - c, |t|^2 and sum t; loading partials over row
+//       blocks: sum_i X[i, j] t[i]                                  -> B4
 //   P5  p = (X^T t - mean sum t) / (scale |t|), R[:, a] = r / |t|,
 //       partial V^T p and S0^T R[:, a]                              -> B5: h, q
 //   P6  v = p - V h, partial v.v and S^T v                          -> B6: |v|, S^T v
 //   P7  V[:, a] = v / |v|, S -= V[:, a] (S^T v / |v|)^T, partial Gram
-//       of S, T[:, a] /= |t|
+//       and u of S, T[:, a] /= |t|
 //
-// At each barrier the last CTA to arrive adds the per-CTA partials in CTA
-// order (deterministic) and publishes the result before releasing the
-// others. Chunk sizes depend only on (n, p), so the result does not depend
+// At each barrier every CTA sums the per-CTA partials itself, in one order
+// (deterministic); B2 has nothing to sum and joins only the CTAs of a row
+// block. Chunk sizes depend only on (n, p), so the result does not depend
 // on the storage type of X: BF16 storage gives the same bits as FP32
 // storage of the same values. All arithmetic is FP64.
 //
@@ -46,18 +46,17 @@ namespace {
 
 constexpr int PT = 256;                       // threads per CTA
 constexpr int kGramRows = 64;                 // S rows staged per Gram step
-constexpr int kSmemDoubles = 4096;            // 32 KB of dynamic shared memory
+// dynamic shared memory of the vector phases (the ring is idle then): scratch
+// of the phases, the barriers' per-thread sums, and the sums of the last one
+constexpr int kSmemDoubles = 4096;
+constexpr int kPartOffset = kSmemDoubles;
+constexpr int kSumsOffset = kPartOffset + PT;
+constexpr int kMaxSums = 576;  // Gram and u of 32 responses, or h and q of 256 components
+constexpr int kPhaseDoubles = kSumsOffset + kMaxSums;
+static_assert(kPersistMaxResponses * (kPersistMaxResponses + 3) / 2 <= kMaxSums &&
+                  kPersistMaxComponents + kPersistMaxResponses <= kMaxSums,
+              "every reduction fits the sums");
 constexpr long long kBarrierCycles = 4000000000LL;  // about 2 s
-
-// scalar slots of a fit (global, FP64)
-constexpr int SC_Z = 0;            // z / sqrt(lambda): kPersistMaxResponses
-constexpr int SC_C = 32;           // mean . rt
-constexpr int SC_T2 = 33;          // |t|^2
-constexpr int SC_ST = 34;          // sum t
-constexpr int SC_VV = 35;          // |v|^2
-constexpr int SC_Q = 40;           // q (m)
-constexpr int SC_SV = 72;          // S^T v (m)
-constexpr int SC_H = 104;          // V^T p (a)
 
 using Fit = PersistentFit;
 
@@ -66,125 +65,108 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-// Arrival: releases this CTA's earlier writes (ordered before it by the CTA
-// barrier) and acquires those released by earlier arrivals, in one atomic.
-__device__ __forceinline__ unsigned atom_add_acq_rel(unsigned* p, unsigned v) {
-  unsigned old;
-  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-  return old;
-}
 __device__ __forceinline__ void red_add_release(unsigned* p, unsigned v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ void st_relaxed(unsigned* p, unsigned v) {
-  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 
-// Barrier of the fit's CTAs with a deterministic reduction of their
-// partials (slots 0 .. count-1 of each CTA's row of cpart). Every thread of
-// the CTA calls it after writing its partials; the reducing CTA calls
-// store(k, sum) in the thread of slot k, then (after a CTA barrier) after(),
-// and releases everyone. Returns false when a wait ran out (flag set to 5);
-// the caller returns.
-//
-// Up to kFlatSlots slots: every CTA arrives at one counter and the last one
-// reduces, Q = PT / count threads per slot, thread q of slot k summing CTAs
-// q, q + Q, ... in order, then the Q sums in order. Wider reductions arrive
-// in groups of kBarGroup CTAs: the last CTA of a group sums the group's
-// partials (thread k: slot k, the group's CTAs in order) into its row of
-// gpart and arrives at the top counter; the last group's reducer sums the
-// group rows in order.
-constexpr int kBarGroup = 32;
-constexpr int kFlatSlots = 64;
-template <class S, class A>
-__device__ bool group_sync(const Fit& f, int* flag, unsigned& epoch, int count, S&& store, A&& after) {
-  __shared__ int role_s, ok_s;  // role: 0 waits, 1 reduced its group, 2 reduces all
-  // per-thread sums of the flat reduction: dynamic shared memory past psm and
-  // hs (the ring is idle at barriers; a static array would be duplicated per
-  // instantiation)
-  extern __shared__ __align__(16) double dyn_smem[];
-  double* const part_s = dyn_smem + kSmemDoubles + kPersistMaxComponents;
-  const bool flat = count <= kFlatSlots;
-  const int cta = (int)blockIdx.x - f.cta0;
-  const int g = cta / kBarGroup;
-  const int ngroups = (f.C + kBarGroup - 1) / kBarGroup;
-  const int gsize = min(kBarGroup, f.C - g * kBarGroup);
-  // the generation after this barrier (every CTA passes the same barriers)
-  const unsigned target = epoch + 1u;
+// Full barriers passed by this CTA, those of them that summed partials, and
+// those that needed a second level.
+struct Passed {
+  unsigned full = 0, turn = 0, wide = 0;
+};
+
+// Whole CTA: arrives at a barrier (one counter, never reset) and waits for its
+// count to reach target. The arrival releases this CTA's earlier writes
+// (ordered before it by the CTA barrier); a barrier costs one reduction and
+// one load latency (an arrival counter, its last arriver and a released
+// generation were three; a flag per CTA polled by every other CTA was slower
+// than that at 100 CTAs and more: the polls delay the stores). False when the
+// wait ran out (flag set to 5); the caller returns.
+__device__ __forceinline__ bool arrive_and_wait(const Fit& f, int* flag, unsigned* counter,
+                                                unsigned target, bool arrive = true) {
   __syncthreads();
+  int ok = 1;
   if (threadIdx.x == 0) {
-    ok_s = 1;
-    if (flat) role_s = atom_add_acq_rel(f.bar, 1u) == (unsigned)f.C - 1u ? 2 : 0;
-    else role_s = atom_add_acq_rel(f.bar + 2 + g, 1u) == (unsigned)gsize - 1u ? 1 : 0;
-  }
-  __syncthreads();
-  if (role_s == 1) {
-    for (int k = threadIdx.x; k < count; k += PT) {
-      const double* src = f.cpart + (long)g * kBarGroup * f.cslots + k;
-      double sum = 0.0;
-#pragma unroll 8
-      for (int c = 0; c < gsize; ++c) sum += __ldcg(src + (long)c * f.cslots);
-      f.gpart[(long)g * f.cslots + k] = sum;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      st_relaxed(f.bar + 2 + g, 0u);
-      if (atom_add_acq_rel(f.bar, 1u) == (unsigned)ngroups - 1u) role_s = 2;
-    }
-    __syncthreads();
-  }
-  if (role_s == 2) {
-    if (flat) {
-      if (count > 0) {
-        const int Q = PT / count;
-        const int t = threadIdx.x;
-        if (t < Q * count) {
-          const int k = t % count, q = t / count;
-          double sum = 0.0;
-#pragma unroll 8
-          for (int c = q; c < f.C; c += Q) sum += __ldcg(f.cpart + (long)c * f.cslots + k);
-          part_s[t] = sum;
-        }
-        __syncthreads();
-        for (int k = t; k < count; k += PT) {
-          double sum = 0.0;
-          for (int q = 0; q < Q; ++q) sum += part_s[q * count + k];
-          store(k, sum);
-        }
-      }
-    } else {
-      for (int k = threadIdx.x; k < count; k += PT) {
-        double sum = 0.0;
-        for (int q = 0; q < ngroups; ++q) sum += __ldcg(f.gpart + (long)q * f.cslots + k);
-        store(k, sum);
-      }
-    }
-    __syncthreads();
-    after();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      st_relaxed(f.bar, 0u);
-      red_add_release(f.bar + 1, 1u);
-    }
-  } else if (threadIdx.x == 0) {
+    if (arrive) red_add_release(counter, 1u);
     const long long t0 = clock64();
-    while ((int)(ld_acquire(f.bar + 1) - target) < 0) {
+    while ((int)(ld_acquire(counter) - target) < 0)
       if (clock64() - t0 > f.barrier_cycles) {
         flag_error(flag, 5);
-        ok_s = 0;
+        ok = 0;
         break;
       }
-      __nanosleep(32);
-    }
   }
-  __syncthreads();
-  epoch = target;
-  return ok_s != 0;
+  return __syncthreads_and(ok) != 0;
 }
 
-// Barrier without partials.
-__device__ __forceinline__ bool group_sync(const Fit& f, int* flag, unsigned& epoch) {
-  return group_sync(f, flag, epoch, 0, [](int, double) {}, [] {});
+// Barrier of the fit's CTAs with a deterministic reduction: sums[k] (shared)
+// = the sum over the CTAs of slot k (k < count) of their partial rows, in
+// every CTA. partials() gives the row to write before the call; rows are
+// double-buffered by turn, since a CTA that has passed one summing barrier may
+// write its next row while another still reads this one (and cannot pass the
+// next summing barrier before that one arrives there).
+//
+// Where the rows are few (C count <= kFlatLoads doubles) every CTA reads and
+// sums them all, Q threads per slot over strided CTAs and then a warp over the
+// Q sums: no CTA waits for another's result. With the last arriver summing and
+// publishing to global memory a component of the 4513 x 10000 fold fit (288
+// CTAs) took 126 us, 20 components 2.64 ms; so 2.48 ms.
+// Wider reductions go through two levels: the first CTA of each group of
+// kBarGroup sums its group's rows into gpart (thread k: slot k, the CTAs in
+// order) and every CTA, after a second barrier, the group rows in order.
+constexpr int kBarGroup = 32;
+constexpr int kFlatLoads = 12288;
+__device__ __forceinline__ double* partials(const Fit& f, const Passed& by) {
+  return f.cpart + ((long)((by.turn + 1u) & 1u) * f.C + ((int)blockIdx.x - f.cta0)) * f.cslots;
+}
+__device__ bool reduce_sync(const Fit& f, int* flag, Passed& by, int count, double* sums) {
+  extern __shared__ __align__(16) double dyn_smem[];
+  double* const part_s = dyn_smem + kPartOffset;  // PT doubles of the idle ring
+  const int cta = (int)blockIdx.x - f.cta0;
+  ++by.turn;
+  if (!arrive_and_wait(f, flag, f.bars, ++by.full * (unsigned)f.C)) return false;
+  const double* rows = f.cpart + (long)(by.turn & 1u) * f.C * f.cslots;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (f.C * count <= kFlatLoads && count <= PT) {
+    const int Q = max(1, min(PT / count, (f.C + 7) / 8));
+    const int t = threadIdx.x;
+    if (t < Q * count) {
+      const int k = t % count, q = t / count;
+      double sum = 0.0;
+#pragma unroll 8
+      for (int c = q; c < f.C; c += Q) sum += __ldcg(rows + (long)c * f.cslots + k);
+      part_s[t] = sum;
+    }
+    __syncthreads();
+    for (int k = warp; k < count; k += PT / 32) {
+      double sum = 0.0;
+      for (int q = lane; q < Q; q += 32) sum += part_s[q * count + k];
+      sum = warp_sum(sum);
+      if (lane == 0) sums[k] = sum;
+    }
+    __syncthreads();
+    return true;
+  }
+  const int ngroups = (f.C + kBarGroup - 1) / kBarGroup;
+  if (cta % kBarGroup == 0) {
+    const int g = cta / kBarGroup, gsize = min(kBarGroup, f.C - cta);
+    const double* src = rows + (long)cta * f.cslots;
+    for (int k = threadIdx.x; k < count; k += PT) {
+      double sum = 0.0;
+#pragma unroll 8
+      for (int c = 0; c < gsize; ++c) sum += __ldcg(src + (long)c * f.cslots + k);
+      f.gpart[(long)g * f.cslots + k] = sum;
+    }
+  }
+  if (!arrive_and_wait(f, flag, f.bars + 1, ++by.wide * (unsigned)ngroups, cta % kBarGroup == 0))
+    return false;
+  for (int k = threadIdx.x; k < count; k += PT) {
+    double sum = 0.0;
+    for (int g = 0; g < ngroups; ++g) sum += __ldcg(f.gpart + (long)g * f.cslots + k);
+    sums[k] = sum;
+  }
+  __syncthreads();
+  return true;
 }
 
 // CTA-level sum; every thread receives it.
@@ -238,11 +220,9 @@ struct NoExtra {
 };
 constexpr int kMaxRingStages = 8;
 static_assert(kBlockRows == 2 * PT, "the scores pass gives each thread two rows of a block");
-static_assert(Ring<bf16>::kBytes >= (kSmemDoubles + kPersistMaxComponents + PT) * 8 &&
-                  Ring<float>::kBytes >= (kSmemDoubles + kPersistMaxComponents + PT) * 8 &&
-                  Ring<double>::kBytes >= (kSmemDoubles + kPersistMaxComponents + PT) * 8,
-              "the vector phases and barriers use the first kSmemDoubles + kPersistMaxComponents + PT "
-              "doubles of the ring");
+static_assert(Ring<bf16>::kBytes >= kPhaseDoubles * 8 && Ring<float>::kBytes >= kPhaseDoubles * 8 &&
+                  Ring<double>::kBytes >= kPhaseDoubles * 8,
+              "the vector phases and barriers use the first kPhaseDoubles doubles of the ring");
 static_assert(Ring<bf16>::kCols <= 32 && Ring<float>::kCols <= 32 && Ring<double>::kCols <= 32 &&
                   Ring<float>::kCols % (PT / 32) == 0 && Ring<double>::kCols % (PT / 32) == 0 &&
                   Ring<bf16>::kCols % (PT / 32) == 0,
@@ -487,12 +467,11 @@ __device__ bool stream_region(const Fit& f, const T* X, const Region& g, bool ba
 }
 
 // Dominant eigenpair of the m x m Gram in A (shared, symmetric; whole CTA;
-// B, C, v shared scratch): scal[SC_Z..] = s z / sqrt(lambda), sign fixed so
-// the largest |z| entry is positive (as direction_kernel), and
-// scal[SC_C] = z . u with u (shared, m) = S^T (mean / scale).
-__device__ void direction_step(const Fit& f, const double* A, double* B, double* C, double* v,
-                               const double* u, int* flag) {
-  const int m = f.m;
+// B, C, v shared scratch): zs (shared) = s z / sqrt(lambda), sign fixed so the
+// largest |z| entry is positive (as direction_kernel), and *offset (shared) =
+// zs . u with u (shared, m) = S^T (mean / scale).
+__device__ void direction_step(int m, const double* A, double* B, double* C, double* v,
+                               const double* u, int* flag, double* zs, double* offset) {
   double lam = 0.0;
   const bool found = dominant_pair(A, B, C, v, m, lam);
   if (threadIdx.x == 0) {
@@ -507,10 +486,10 @@ __device__ void direction_step(const Fit& f, const double* A, double* B, double*
     double cz = 0.0;
     for (int k = 0; k < m; ++k) {
       const double zk = found ? sgn * v[k] * inv : 0.0;
-      f.scal[SC_Z + k] = zk;
+      zs[k] = zk;
       cz = fma(zk, u[k], cz);
     }
-    f.scal[SC_C] = cz;
+    *offset = cz;
   }
   __syncthreads();
 }
@@ -518,9 +497,9 @@ __device__ void direction_step(const Fit& f, const double* A, double* B, double*
 // Over this CTA's columns [j0, j1): when a >= 0, V[:, a] = v / |v| and the
 // deflation S -= V[:, a] (S^T v / |v|)^T; then the partials of the Gram of S
 // (slots 0 .. G-1, packed lower triangle) and of u = S^T (mean / scale)
-// (slots G .. G+m-1) into the CTA's partial row. Whole CTA.
-__device__ void gram_u_partials(const Fit& f, int cta, int j0, int j1, int a, double inv_v,
-                                const double* sv, double* sm) {
+// (slots G .. G+m-1) into out (the CTA's partial row). Whole CTA.
+__device__ void gram_u_partials(const Fit& f, int j0, int j1, int a, double inv_v,
+                                const double* sv, double* sm, double* out) {
   const int m = f.m, p = f.p;
   const int G = m * (m + 1) / 2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -564,7 +543,7 @@ __device__ void gram_u_partials(const Fit& f, int cta, int j0, int j1, int a, do
     }
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < G + m; k += PT) f.cpart[(long)cta * f.cslots + k] = gacc[k];
+  for (int k = threadIdx.x; k < G + m; k += PT) out[k] = gacc[k];
 }
 
 template <class T>
@@ -577,8 +556,7 @@ __global__ void __launch_bounds__(PT, 2)
   __shared__ unsigned ring_done[kMaxRingStages], ring_issued;
   __shared__ double red[32];
   __shared__ double zs[kPersistMaxResponses];
-  __shared__ double sv[kPersistMaxResponses];
-  __shared__ double scal_s[4];
+  __shared__ double offset_s, inv_s;
   int fi = 0;
   while (fi + 1 < nfits && (int)blockIdx.x >= fits[fi + 1].cta0) ++fi;
   const Fit& f = fits[fi];  // read through the read-only path as needed (fewer live registers)
@@ -595,7 +573,8 @@ __global__ void __launch_bounds__(PT, 2)
   double* const aux = reinterpret_cast<double*>(ring + Ring<T>::kBytes);
   const Region rg = region_of<T>(f, cta);
   unsigned seq = 0;  // stages streamed by this CTA so far
-  unsigned bar_epoch = 0;  // group barriers passed
+  Passed by;
+  double* const sums = psm + kSumsOffset;
   if (tid == 0) {
     for (int k = 0; k < Ring<T>::kStages; ++k) {
       ring_bar_init(ring_bars + k);
@@ -607,33 +586,28 @@ __global__ void __launch_bounds__(PT, 2)
   const int G = m * (m + 1) / 2;
   // partials of the Gram of S and of u = S^T (mean / scale) over this CTA's
   // columns, before the first component (S = S0)
-  gram_u_partials(f, cta, j0, j1, -1, 0.0, sv, psm);
+  gram_u_partials(f, j0, j1, -1, 0.0, nullptr, psm, partials(f, by));
   for (int a = 0; a < f.a; ++a) {
     // B0: Gram and u of the (deflated) S, the direction z / sqrt(lambda), and
     // the score offset c = mean . (S z / scale) = z . u
+    if (!reduce_sync(f, flag, by, G + m, sums)) return;
     {
       double* A = psm;               // m x m Gram
       double* B = A + m * m;         // squaring scratch
       double* Cs = B + m * m;        // m^2 + 1
       double* vd = Cs + m * m + 1;   // dominant eigenvector (m + 1)
-      double* us = vd + m + 1;       // u
-      auto store = [&](int k, double v) {
-        if (k < G) {
-          int c = (int)((sqrt(8.0 * k + 1.0) - 1.0) * 0.5);
-          while (c * (c + 1) / 2 > k) --c;
-          while ((c + 1) * (c + 2) / 2 <= k) ++c;
-          const int d = k - c * (c + 1) / 2;
-          A[c + d * m] = v;
-          A[d + c * m] = v;
-          f.gpk[k] = v;
-        } else {
-          us[k - G] = v;
-        }
-      };
-      if (!group_sync(f, flag, bar_epoch, G + m, store, [&] { direction_step(f, A, B, Cs, vd, us, flag); })) return;
+      for (int k = tid; k < G; k += PT) {
+        int c = (int)((sqrt(8.0 * k + 1.0) - 1.0) * 0.5);
+        while (c * (c + 1) / 2 > k) --c;
+        while ((c + 1) * (c + 2) / 2 <= k) ++c;
+        const int d = k - c * (c + 1) / 2;
+        A[c + d * m] = sums[k];
+        A[d + c * m] = sums[k];
+        if (cta == 0) f.gpk[k] = sums[k];
+      }
+      __syncthreads();
+      direction_step(m, A, B, Cs, vd, sums + G, flag, zs, &offset_s);
     }
-    for (int c = tid; c < m; c += PT) zs[c] = __ldcg(f.scal + SC_Z + c);
-    __syncthreads();
     // P2: score partials of the region, t_part[crg][rows] = X[rows, cols] rt[cols]
     // with rt = (S z) / scale (S is not deflated until P7)
     {
@@ -694,30 +668,71 @@ __global__ void __launch_bounds__(PT, 2)
       if (tid < rg.rows) out[tid] = (acc0[0] + acc0[1]) + (acc0[2] + acc0[3]);
       if (r1 < rg.rows) out[r1] = (acc1[0] + acc1[1]) + (acc1[2] + acc1[3]);
     }
-    if (!group_sync(f, flag, bar_epoch)) return;
+    // B2: the column ranges of this row block
+    if (!arrive_and_wait(f, flag, f.bars + 2 + rg.rbk, (unsigned)(a + 1) * (unsigned)f.Cc)) return;
     // P4: loading partials of the region, p_part[rbk][cols] = X[rows, cols]^T t[rows],
     // the stages backward. While the first stages are in flight each CTA
     // forms t for its row block: t = sum of the column ranges' partials - c
     // (the CTAs of column range 0 also store T[:, a] and the |t|^2, sum t
     // partials of their block).
     {
-      const double cc = __ldcg(f.scal + SC_C);
+      const double cc = offset_s;
       double* tcol = f.T + (long)a * n + rg.r0;
       auto tv = [&] {
         double s2 = 0.0, s1 = 0.0;
-        for (int r = tid; r < rg.rows; r += PT) {
-          const long i = rg.r0 + r;
-          // eight interleaved partial sums (more loads in flight), fixed order
-          double q[8];
+        // both of the thread's rows at once; per row eight interleaved sums
+        // over the column ranges in a fixed order, sixteen loads a row in
+        // flight (one row of eight at a time was 8 us at 49 column ranges)
+        double q[2][8];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) q[u] = 0.0;
-          int k = 0;
-          for (; k + 7 < f.Cc; k += 8) {
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int u = 0; u < 8; ++u) q[u] += __ldcg(f.tpart + (long)(k + u) * n + i);
-          }
-          for (; k < f.Cc; ++k) q[0] += __ldcg(f.tpart + (long)k * n + i);
-          const double t = (((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]))) - cc;
+          for (int u = 0; u < 8; ++u) q[h][u] = 0.0;
+        const double* src = f.tpart + rg.r0 + tid;
+        const bool in[2] = {tid < rg.rows, tid + PT < rg.rows};
+        int k = 0;
+        for (; k + 15 < f.Cc; k += 16) {
+          double v[2][16];
+#pragma unroll
+          for (int u = 0; u < 16; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) v[h][u] = in[h] ? __ldcg(src + (long)(k + u) * n + h * PT) : 0.0;
+#pragma unroll
+          for (int u = 0; u < 16; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) q[h][u & 7] += v[h][u];
+        }
+        for (; k + 7 < f.Cc; k += 8) {
+          double v[2][8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) v[h][u] = in[h] ? __ldcg(src + (long)(k + u) * n + h * PT) : 0.0;
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) q[h][u] += v[h][u];
+        }
+        if (k < f.Cc) {
+          // the last ranges into sum 0, in order, loaded together
+          double v[2][7];
+#pragma unroll
+          for (int u = 0; u < 7; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              v[h][u] = in[h] && k + u < f.Cc ? __ldcg(src + (long)(k + u) * n + h * PT) : 0.0;
+#pragma unroll
+          for (int u = 0; u < 7; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              if (k + u < f.Cc) q[h][0] += v[h][u];
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (!in[h]) continue;
+          const int r = tid + h * PT;
+          const double* e = q[h];
+          const double t = (((e[0] + e[1]) + (e[2] + e[3])) + ((e[4] + e[5]) + (e[6] + e[7]))) - cc;
           aux[r] = t;
           if (rg.crg == 0) {
             tcol[r] = t;
@@ -731,8 +746,9 @@ __global__ void __launch_bounds__(PT, 2)
           s1 = cta_sum(s1, red);
         }
         if (tid == 0) {
-          f.cpart[(long)cta * f.cslots] = rg.crg == 0 ? s2 : 0.0;
-          f.cpart[(long)cta * f.cslots + 1] = rg.crg == 0 ? s1 : 0.0;
+          double* row = partials(f, by);
+          row[0] = rg.crg == 0 ? s2 : 0.0;
+          row[1] = rg.crg == 0 ? s1 : 0.0;
         }
       };
       const int lane = tid & 31, warp = tid >> 5;
@@ -801,13 +817,13 @@ __global__ void __launch_bounds__(PT, 2)
       });
       if (!ok) return;
     }
-    if (!group_sync(f, flag, bar_epoch, 2, [&](int k, double v) { f.scal[k == 0 ? SC_T2 : SC_ST] = v; }, [] {}))
-      return;
+    if (!reduce_sync(f, flag, by, 2, sums)) return;
     // P5: p, R[:, a] = (S z) / |t|; partial V^T p (a) and S0^T R[:, a] (m).
-    // The column partials are loaded while thread 0 fetches |t|^2 and sum t.
     if (tid == 0) {
-      scal_s[0] = __ldcg(f.scal + SC_T2);
-      scal_s[1] = __ldcg(f.scal + SC_ST);
+      const double tn = sqrt(sums[0]);
+      const bool ok = tn > 0.0 && isfinite(tn);
+      if (!ok && cta == 0) flag_error(flag, 1);
+      inv_s = ok ? 1.0 / tn : 0.0;
     }
     double* ps = psm;          // p values of this CTA's columns (<= 2048)
     double* rs = psm + 2048;   // R values
@@ -842,14 +858,7 @@ __global__ void __launch_bounds__(PT, 2)
       rs[jl] = rv;
     }
     __syncthreads();
-    if (tid == 0) {
-      const double tn = sqrt(scal_s[0]);
-      const bool ok = tn > 0.0 && isfinite(tn);
-      if (!ok && cta == 0) flag_error(flag, 1);
-      scal_s[2] = ok ? 1.0 / tn : 0.0;
-    }
-    __syncthreads();
-    const double inv_t = scal_s[2], sum_t = scal_s[1];
+    const double inv_t = inv_s, sum_t = sums[1];
     for (int jl = tid; jl < j1 - j0; jl += PT) {
       const int j = j0 + jl;
       const double pj = (ps[jl] - f.mean[j] * sum_t) / f.scale[j] * inv_t;
@@ -866,6 +875,7 @@ __global__ void __launch_bounds__(PT, 2)
       const int lane = tid & 31, warp = tid >> 5;
       const int cols = j1 - j0;
       constexpr int W = PT / 32;
+      double* row = partials(f, by);
       for (int kb = warp; kb < a + m; kb += 3 * W) {
         double sd[3] = {0.0, 0.0, 0.0};
 #pragma unroll
@@ -880,25 +890,15 @@ __global__ void __launch_bounds__(PT, 2)
         for (int e = 0; e < 3; ++e) {
           const int k = kb + e * W;
           const double v = warp_sum(sd[e]);
-          if (lane == 0 && k < a + m) f.cpart[(long)cta * f.cslots + k] = v;
+          if (lane == 0 && k < a + m) row[k] = v;
         }
       }
     }
-    if (!group_sync(f, flag, bar_epoch, a + m,
-                    [&](int k, double v) {
-                      if (k < a) {
-                        f.scal[SC_H + k] = v;
-                      } else {
-                        f.scal[SC_Q + k - a] = v;
-                        f.Q[(k - a) + (long)a * m] = v;
-                      }
-                    },
-                    [] {}))
-      return;
+    if (!reduce_sync(f, flag, by, a + m, sums)) return;
+    if (cta == 0)
+      for (int c = tid; c < m; c += PT) f.Q[c + (long)a * m] = sums[a + c];
     // P6: v = p - V h; partial v.v and S^T v
-    double* const hs = psm + kSmemDoubles;  // V^T p (a), beside psm in the idle ring
-    for (int k = tid; k < a; k += PT) hs[k] = __ldcg(f.scal + SC_H + k);
-    __syncthreads();
+    const double* const hs = sums;  // V^T p (a)
     double* vs = psm;  // v of this CTA's columns
     double vvp = 0.0;
     for (int jl = tid; jl < j1 - j0; jl += PT) {
@@ -914,33 +914,27 @@ __global__ void __launch_bounds__(PT, 2)
     {
       const int lane = tid & 31, warp = tid >> 5;
       const int cols = j1 - j0;
+      double* row = partials(f, by);
       for (int c = warp; c < m; c += PT / 32) {
         const double* sc = f.S + (long)c * p + j0;
         double s = 0.0;
         for (int jl = lane; jl < cols; jl += 32) s = fma(__ldcg(sc + jl), vs[jl], s);
         s = warp_sum(s);
-        if (lane == 0) f.cpart[(long)cta * f.cslots + 1 + c] = s;
+        if (lane == 0) row[1 + c] = s;
       }
-      if (tid == 0) f.cpart[(long)cta * f.cslots] = vvp;
+      if (tid == 0) row[0] = vvp;
     }
-    if (!group_sync(f, flag, bar_epoch, 1 + m,
-                    [&](int k, double v) {
-                      if (k == 0) f.scal[SC_VV] = v;
-                      else f.scal[SC_SV + k - 1] = v;
-                    },
-                    [] {}))
-      return;
+    if (!reduce_sync(f, flag, by, 1 + m, sums)) return;
     // P7: V[:, a], deflate S, partials of the Gram and u of the deflated S;
     // T[:, a] /= |t|
     if (tid == 0) {
-      const double vn = sqrt(__ldcg(f.scal + SC_VV));
+      const double vn = sqrt(sums[0]);
       const bool ok = vn > 0.0 && isfinite(vn);
       if (!ok && cta == 0) flag_error(flag, 1);
-      scal_s[2] = ok ? 1.0 / vn : 0.0;
+      inv_s = ok ? 1.0 / vn : 0.0;
     }
-    for (int c = tid; c < m; c += PT) sv[c] = __ldcg(f.scal + SC_SV + c);
     __syncthreads();
-    gram_u_partials(f, cta, j0, j1, a, scal_s[2], sv, psm);
+    gram_u_partials(f, j0, j1, a, inv_s, sums + 1, psm, partials(f, by));
     double* tcol = f.T + (long)a * n;
     for (int i = cta * PT + tid; i < n; i += C * PT) tcol[i] = __ldcg(tcol + i) * inv_t;
   }
@@ -1072,9 +1066,15 @@ namespace {
 // not fit the persistent launch.
 bool persistent_grid(int n, int p, int& Cr, int& Cc, int& rb, int& pc) {
   const long elems = (long)n * p;
-  // about 2^15 elements per CTA: one CTA streams a few tens of GB/s, so
-  // even small fits spread over many SMs (the barriers cost little more)
-  const int c0 = (int)std::max(1L, std::min<long>(2L * num_sms(), (elems + (1L << 15) - 1) >> 15));
+  // Elements per CTA: a CTA streams a few tens of GB/s, so small fits spread
+  // until the barriers cost what the passes save -- 2^13 elements up to 32 CTAs,
+  // 2^14 beyond (fit in us at 2^15 / 2^14 / 2^13 / 2^12 elements: 97 x 311 FP64,
+  // 4 components 533 / 351 / 252 / 224; 200 x 300 FP32, 6: 404 / 328 / 292 /
+  // 311; 500 x 2000 FP64, 10: 630 / 545 / 587 / 659; 541 x 1500 FP64, 8: 607 /
+  // 466 / 477 / 421). Fewer CTAs per fit also leave room for other fits of a
+  // batch in one launch.
+  const int shift = elems <= (32L << 13) ? 13 : 14;
+  const int c0 = (int)std::max(1L, std::min<long>(2L * num_sms(), (elems + (1L << shift) - 1) >> shift));
   Cr = (n + kBlockRows - 1) / kBlockRows;
   rb = round_up((n + Cr - 1) / Cr, 8);
   Cr = (n + rb - 1) / rb;
@@ -1173,14 +1173,12 @@ bool plan_simpls_persistent(const T* X, int n, int p, long ld, int m, int a, Dev
   f.tpart = plan.part.get();
   f.ppart = f.tpart + (size_t)Cc * n;
   const int ngroups = (C + kBarGroup - 1) / kBarGroup;
-  plan.cpart.allocate((size_t)(C + ngroups) * f.cslots, stream);
-  plan.scal.allocate((size_t)SC_H + kPersistMaxComponents + 8, stream);
-  plan.bar.allocate(2 + ngroups, stream);
-  plan.bar.zero(stream);
+  plan.cpart.allocate((size_t)(2 * C + ngroups) * f.cslots, stream);
+  plan.bars.allocate(2 + Cr, stream);
+  plan.bars.zero(stream);
   f.cpart = plan.cpart.get();
-  f.gpart = f.cpart + (size_t)C * f.cslots;
-  f.scal = plan.scal.get();
-  f.bar = plan.bar.get();
+  f.gpart = f.cpart + (size_t)2 * C * f.cslots;
+  f.bars = plan.bars.get();
   model.a = a;
   return true;
 }

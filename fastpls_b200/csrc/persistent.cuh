@@ -27,10 +27,9 @@ struct PersistentFit {
   double *pv, *v;           // p
   double* tpart;            // Cc x n (scores pass, one row per column range)
   double* ppart;            // Cr x p (loading pass, one row per row block)
-  double* cpart;            // C x cslots (per-CTA partials)
+  double* cpart;            // 2 x C x cslots (per-CTA partials, by turn)
   double* gpart;            // ceil(C / 32) x cslots (per-group sums)
-  double* scal;             // scalar slots
-  unsigned* bar;            // [groups arrived, generation, CTAs arrived per group...]
+  unsigned* bars;           // arrivals: all CTAs, second level, per row block
   int* flag;                // the fit's error flag
   int cta0, C;              // CTA range of this fit in the launch
   int Cr, rb;               // row blocks of X and their rows (C = Cr Cc)
@@ -46,8 +45,8 @@ struct PersistentFit {
 struct PersistentPlan {
   PersistentFit fit{};
   int elem = 0;  // bytes per stored element of X (2 BF16, 4 FP32, 8 FP64)
-  DeviceArray<double> S, part, cpart, scal;
-  DeviceArray<unsigned> bar;
+  DeviceArray<double> S, part, cpart;
+  DeviceArray<unsigned> bars;
 };
 
 // Whether the persistent path takes a fit with m responses and a components.

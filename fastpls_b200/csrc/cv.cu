@@ -4,17 +4,23 @@
 // Behavioural contract: src/cuda_resident_api.cuh:538-1023 of the reference
 // (validation and messages, fold status codes 1/2/4, metric assembly in long
 // double, prediction and score output layouts). X and Y are uploaded once;
-// each fold's training and held-out rows are gathered on the device and the
-// fold model is fitted by the resident engine (fit.cu / plssvd.cu).
-// Folds run one after another here; the many-fold / many-permutation batched
-// engine lives in batched.cu.
+// each fold's training and held-out rows are split on the device and the
+// fold model is fitted by the resident engine (fit.cu / plssvd.cu). Folds run
+// in batches: every fold of a batch is prepared on one of a few streams, the
+// SIMPLS folds that take the persistent form run their component loops in one
+// launch with the co-resident CTAs shared between them (a fold alone leaves
+// most SMs idle: ten folds of 541 x 1500 FP64 were ten launches of 24 CTAs, 527
+// us each), and the held-out predictions follow on the streams; one wait per
+// batch. The many-fold / many-permutation batched engine lives in batched.cu.
 #include "upload.cuh"
 #include "cv.cuh"
 #include "handle.cuh"
 #include "lda.cuh"
+#include "persistent.cuh"
 
 #include <algorithm>
 #include <cmath>
+#include <exception>
 #include <limits>
 #include <vector>
 
@@ -46,13 +52,6 @@ __global__ void fold_sums_kernel(const double* __restrict__ pred,
   }
 }
 
-template <class T>
-__global__ void to_f64_kernel(const T* __restrict__ in, long count, double* out) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count;
-       i += (long)gridDim.x * blockDim.x)
-    out[i] = as_f64(in[i]);
-}
-
 struct Folds {
   int count = 0;
   std::vector<std::vector<int>> test;
@@ -71,14 +70,196 @@ Folds partition(const int* folds, int n) {
   return f;
 }
 
+// Rows of X (n x p) and of Y (n x q, may be null) into the training and
+// held-out matrices of one fold: pos[r] >= 0 is row r's training row, ~pos[r]
+// its held-out row. Reads every element once, coalesced along the rows.
 template <class T>
-void fit_method(int method, const T* X, int n, int p, const double* Yc,
-                const double* ycsum, int m, int a, int scaling,
-                DeviceModel& model, Workspace& ws, cudaStream_t s) {
-  if (method == kPlssvd) fit_plssvd<T>(X, n, p, n, Yc, ycsum, m, a, scaling, model, ws, s);
-  else fit_simpls<T>(X, n, p, n, Yc, ycsum, m, a, scaling, model, ws, s,
-                     simpls_block_size(n, p, m, a, model.classification, std::is_same<T, float>::value),
-                     simpls_gram_route(n, p, a, model.classification));
+__global__ void split_rows_kernel(const T* __restrict__ X, const T* __restrict__ Y, int n, int p, int q,
+                                  const int* __restrict__ pos, int ntr, int nte, T* __restrict__ Xtr,
+                                  T* __restrict__ Xte, T* __restrict__ Ytr, double* __restrict__ Yte) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  const int at = pos[r];
+  for (int c = blockIdx.y; c < p + q; c += gridDim.y) {
+    if (c < p) {
+      const T v = X[r + (long)c * n];
+      if (at >= 0) Xtr[at + (long)c * ntr] = v;
+      else Xte[~at + (long)c * nte] = v;
+    } else {
+      const T v = Y[r + (long)(c - p) * n];
+      if (at >= 0) Ytr[at + (long)(c - p) * ntr] = v;
+      else Yte[~at + (long)(c - p) * nte] = as_f64(v);
+    }
+  }
+}
+
+// One fold of a batch, its device state allocated on its stream.
+template <class T>
+struct Fold {
+  int f = 0, ntr = 0, nte = 0, m = 0;  // fold, rows, responses or active classes
+  cudaStream_t st = nullptr;
+  Workspace ws;
+  DeviceModel model;
+  std::unique_ptr<PersistentPlan> plan;
+  DeviceArray<T> Xtr, Xte, Ytr;
+  DeviceArray<double> Yte, Yc, ycsum, scores, pred, sums;
+  DeviceArray<int> top;
+  const int *pos = nullptr, *lab = nullptr;  // into the batch's arrays
+  std::unique_ptr<LdaState> lda;
+  std::vector<int> active, host_labels;
+  std::vector<double> host_pred, host_sums;
+  int bad = 0;
+};
+
+constexpr int kLanes = 4;
+
+// The streams of one call: `main` (uploads, shared launches) and the lanes
+// that prepare and finish the folds.
+struct Lanes {
+  cudaStream_t main = nullptr, lane[kLanes] = {};
+  cudaEvent_t ev = nullptr;
+  explicit Lanes(int lanes) {
+    FPLS_CHECK(cudaStreamCreateWithFlags(&main, cudaStreamNonBlocking));
+    FPLS_CHECK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    for (int k = 0; k < std::min(lanes, kLanes); ++k)
+      FPLS_CHECK(cudaStreamCreateWithFlags(&lane[k], cudaStreamNonBlocking));
+  }
+  ~Lanes() {
+    for (cudaStream_t s : lane)
+      if (s) {
+        cudaStreamSynchronize(s);
+        cudaStreamDestroy(s);
+      }
+    if (main) {
+      cudaStreamSynchronize(main);
+      cudaStreamDestroy(main);
+    }
+    if (ev) cudaEventDestroy(ev);
+  }
+  Lanes(const Lanes&) = delete;
+  Lanes& operator=(const Lanes&) = delete;
+  void after(cudaStream_t later, cudaStream_t earlier) {
+    FPLS_CHECK(cudaEventRecord(ev, earlier));
+    FPLS_CHECK(cudaStreamWaitEvent(later, ev, 0));
+  }
+  void lanes_after_main() {
+    FPLS_CHECK(cudaEventRecord(ev, main));
+    for (cudaStream_t s : lane)
+      if (s) FPLS_CHECK(cudaStreamWaitEvent(s, ev, 0));
+  }
+  void main_after_lanes() {
+    for (cudaStream_t s : lane)
+      if (s) after(main, s);
+  }
+  void sync() {
+    for (cudaStream_t s : lane)
+      if (s) FPLS_CHECK(cudaStreamSynchronize(s));
+    FPLS_CHECK(cudaStreamSynchronize(main));
+  }
+};
+
+// Declared after what the lanes use: nothing is freed while they run, on an
+// error too.
+struct Settle {
+  Lanes& lanes;
+  ~Settle() {
+    for (cudaStream_t s : lanes.lane)
+      if (s) cudaStreamSynchronize(s);
+    cudaStreamSynchronize(lanes.main);
+  }
+};
+
+// Folds per batch and the persistent CTAs each may take: as many as device
+// memory (a quarter of what is free, at most 8 GB, at least one fold) and the
+// co-resident CTAs hold, in batches of equal size.
+template <class T>
+void batch_shape(int method, const Folds& fp, int n, int p, int m, int a, int folds, size_t pred_bytes,
+                 int* per_batch, int* max_ctas) {
+  size_t free_b = 0, total_b = 0;
+  FPLS_CHECK(cudaMemGetInfo(&free_b, &total_b));
+  const double one = (double)n * p * sizeof(T) + 8.0 * ((double)p * (2.0 * a + 4.0 * m + 16.0) +
+                                                      (double)n * (2.0 * a + 3.0 * m + 8.0)) +
+                     (double)pred_bytes + 64.0 * 1024 * 1024;
+  int most = (int)std::max(1.0, std::min((double)folds, std::min(8e9, 0.25 * (double)free_b) / one));
+  *max_ctas = 0;
+  if (method != kPlssvd) {
+    const int cap = persistent_capacity((int)sizeof(T));
+    while (most > 1 && most * persistent_ctas(fp.max_train, p, cap / most) > cap) --most;
+    if ((long)fp.max_train * p > kPersistMaxElements) most = 1;
+    if (cap > 0) *max_ctas = cap / most;
+  }
+  const int batches = (folds + most - 1) / most;
+  *per_batch = (folds + batches - 1) / batches;
+}
+
+// The fit of a prepared fold on its stream; a SIMPLS fold that takes the
+// persistent form leaves its plan for the batch's launch.
+template <class T>
+void fit_fold(int method, Fold<T>& d, int p, int a, int scaling, int max_ctas) {
+  const int n = d.ntr, m = d.m;
+  if (method == kPlssvd) {
+    fit_plssvd<T>(d.Xtr.get(), n, p, n, d.Yc.get(), d.ycsum.get(), m, a, scaling, d.model, d.ws, d.st);
+    return;
+  }
+  struct Sink {
+    explicit Sink(std::unique_ptr<PersistentPlan>* plan, int ctas) { persistent_deferral() = {plan, ctas}; }
+    ~Sink() { persistent_deferral() = {}; }
+  } sink(&d.plan, max_ctas);
+  fit_simpls<T>(d.Xtr.get(), n, p, n, d.Yc.get(), d.ycsum.get(), m, a, scaling, d.model, d.ws, d.st,
+                simpls_block_size(n, p, m, a, d.model.classification, std::is_same<T, float>::value),
+                simpls_gram_route(n, p, a, d.model.classification));
+}
+
+// The component loops of the batch's deferred folds, as many per launch as
+// are co-resident.
+template <class T>
+void launch_plans(std::vector<std::unique_ptr<Fold<T>>>& batch, Lanes& lanes) {
+  std::vector<PersistentPlan*> plans;
+  int ctas = 0;
+  const int cap = persistent_capacity((int)sizeof(T));
+  bool any = false;
+  for (auto& d : batch) any = any || d->plan;
+  if (!any) return;
+  lanes.main_after_lanes();
+  for (auto& d : batch) {
+    if (!d->plan) continue;
+    if (ctas + d->plan->fit.C > cap) {
+      launch_persistent(plans, lanes.main);
+      plans.clear();
+      ctas = 0;
+    }
+    plans.push_back(d->plan.get());
+    ctas += d->plan->fit.C;
+  }
+  launch_persistent(plans, lanes.main);
+  lanes.lanes_after_main();
+}
+
+// Position of every row in the training (k) or held-out (~k) matrix of the
+// fold that holds out `held`, into pos (n).
+void fold_positions(const std::vector<int>& held, int n, int* pos) {
+  std::fill(pos, pos + n, 0);
+  for (size_t k = 0; k < held.size(); ++k) pos[held[k]] = ~(int)k;
+  int at = 0;
+  for (int i = 0; i < n; ++i)
+    if (pos[i] >= 0) pos[i] = at++;
+}
+
+template <class T>
+void split_fold(Fold<T>& d, const T* X, const T* Y, int n, int p, int q) {
+  d.Xtr.allocate((size_t)d.ntr * p, d.st);
+  d.Xte.allocate((size_t)d.nte * p, d.st);
+  if (Y) {
+    d.Ytr.allocate((size_t)d.ntr * q, d.st);
+    d.Yte.allocate((size_t)d.nte * q, d.st);
+  }
+  const int cols = p + (Y ? q : 0);
+  const unsigned gx = ceil_div(n, 256);
+  const unsigned gy = (unsigned)std::max(1L, std::min<long>(cols, std::min<long>(65535, 16L * num_sms() / gx)));
+  split_rows_kernel<T><<<dim3(gx, gy), 256, 0, d.st>>>(X, Y, n, p, Y ? q : 0, d.pos, d.ntr, d.nte,
+                                                       d.Xtr.get(), d.Xte.get(), d.Ytr.get(), d.Yte.get());
+  count_launch();
+  FPLS_LAUNCH("split_rows");
 }
 
 }  // namespace
@@ -119,101 +300,121 @@ void cv_regression(int method, const T* predictors, const T* responses,
     total_ss += ss - s * s / n;
   }
 
-  cudaStream_t s = nullptr;
-  FPLS_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-  struct StreamGuard {
-    cudaStream_t s;
-    ~StreamGuard() {
-      if (s) {
-        cudaStreamSynchronize(s);
-        cudaStreamDestroy(s);
-      }
-    }
-  } guard{s};
+  Lanes lanes(fp.count);
   {
-    DeviceArray<T> X((size_t)n * p, s), Y((size_t)n * q, s);
-    upload_h2d(X.get(), predictors, sizeof(T) * n * p, s);
-    FPLS_CHECK(cudaMemcpyAsync(Y.get(), responses, sizeof(T) * n * q, cudaMemcpyHostToDevice, s));
-    DeviceArray<double> Y64((size_t)n * q, s);
-    to_f64_kernel<T><<<std::min<unsigned>(ceil_div((size_t)n * q, 256), 4 * num_sms()), 256, 0, s>>>(Y.get(), (long)n * q, Y64.get());
-    count_launch();
-    DeviceArray<T> Xtr((size_t)fp.max_train * p, s), Xte((size_t)fp.max_test * p, s);
-    DeviceArray<T> Ytr((size_t)fp.max_train * q, s);
-    DeviceArray<double> Yte((size_t)fp.max_test * q, s);
-    DeviceArray<int> idx_tr(fp.max_train, s), idx_te(fp.max_test, s);
-    DeviceArray<double> Yc((size_t)fp.max_train * q, s), ycsum(q, s);
-    DeviceArray<double> scores((size_t)fp.max_test * maximum_prefix, s);
-    const int step = prefixes_at_once((size_t)fp.max_test * q * sizeof(double), prefix_count);
-    DeviceArray<double> pred((size_t)fp.max_test * q * step, s);
-    DeviceArray<double> sums((size_t)2 * q * prefix_count, s);
-    Workspace ws;
-    ws.ensure(fp.max_train, p, q, maximum_prefix, s);
-
+    DeviceArray<T> X((size_t)n * p, lanes.main), Y((size_t)n * q, lanes.main);
+    upload_h2d(X.get(), predictors, sizeof(T) * n * p, lanes.main);
+    FPLS_CHECK(cudaMemcpyAsync(Y.get(), responses, sizeof(T) * n * q, cudaMemcpyHostToDevice, lanes.main));
+    lanes.lanes_after_main();
+    const size_t block = (size_t)fp.max_test * q;
+    const int step = prefixes_at_once(block * sizeof(double), prefix_count);
+    int per_batch = 1, max_ctas = 0;
+    batch_shape<T>(method, fp, n, p, q, maximum_prefix, fp.count, block * step * sizeof(double), &per_batch,
+                   &max_ctas);
     std::fill(metrics, metrics + prefix_count, 0.0);
     std::vector<double> counts(prefix_count, 0.0), fold_ss(prefix_count, 0.0);
-    std::vector<double> host_sums((size_t)2 * q * prefix_count);
-    std::vector<double> host_pred;
-    std::vector<int> train;
-    for (int f = 0; f < fp.count; ++f) {
-      const auto& held = fp.test[f];
-      if (held.empty()) {
-        status[f] = 2;
-        continue;
-      }
-      std::vector<char> flag(n, 0);
-      for (int r : held) flag[r] = 1;
-      train.clear();
-      for (int i = 0; i < n; ++i)
-        if (!flag[i]) train.push_back(i);
-      const int ntr = (int)train.size(), nte = (int)held.size();
-      if (maximum_prefix > std::min(ntr - 1, p))
-        throw std::invalid_argument("CUDA CV component count exceeds a fold rank");
-      FPLS_CHECK(cudaMemcpyAsync(idx_tr.get(), train.data(), sizeof(int) * ntr, cudaMemcpyHostToDevice, s));
-      FPLS_CHECK(cudaMemcpyAsync(idx_te.get(), held.data(), sizeof(int) * nte, cudaMemcpyHostToDevice, s));
-      gather_rows<T>(X.get(), n, p, idx_tr.get(), ntr, Xtr.get(), ntr, s);
-      gather_rows<T>(X.get(), n, p, idx_te.get(), nte, Xte.get(), nte, s);
-      gather_rows<T>(Y.get(), n, q, idx_tr.get(), ntr, Ytr.get(), ntr, s);
-      gather_rows<double>(Y64.get(), n, q, idx_te.get(), nte, Yte.get(), nte, s);
-      FPLS_CHECK(cudaMemsetAsync(ws.flag.get(), 0, sizeof(int), s));
-      DeviceModel model;
-      model.ymean.allocate(q, s);
-      prepare_responses<T>(Ytr.get(), nullptr, ntr, q, Yc.get(), model.ymean.get(), ycsum.get(), ws.flag.get(), s);
-      fit_method<T>(method, Xtr.get(), ntr, p, Yc.get(), ycsum.get(), q, maximum_prefix, scaling, model, ws, s);
-      project_rows<T>(model, Xte.get(), nte, nte, maximum_prefix, scores.get(), nte, ws, s);
-      if (store_predictions) host_pred.resize((size_t)nte * q * prefix_count);
-      for (int j = 0; j < prefix_count; j += step) {
-        const int w = std::min(step, prefix_count - j);
-        predict_prefixes<double>(model, scores.get(), nte, nte, prefixes + j, w, pred.get(), s);
-        if (store_predictions)
-          FPLS_CHECK(cudaMemcpyAsync(host_pred.data() + (size_t)j * nte * q, pred.get(),
-                                     sizeof(double) * nte * q * w, cudaMemcpyDeviceToHost, s));
-        fold_sums_kernel<<<dim3(q, w), 256, 0, s>>>(pred.get(), Yte.get(), model.ymean.get(), nte, q,
-                                                    sums.get() + (size_t)2 * q * j);
-        count_launch();
-        FPLS_LAUNCH("fold_sums");
-      }
-      FPLS_CHECK(cudaMemcpyAsync(host_sums.data(), sums.get(), sizeof(double) * 2 * q * prefix_count,
-                                 cudaMemcpyDeviceToHost, s));
-      raise_on_flag(ws, s, method == kPlssvd
-          ? "resident PLS-SVD failed: invalid labels, decomposition or score Gram"
-          : "resident SIMPLS failed: invalid labels, decomposition or component norm");
-      for (int j = 0; j < prefix_count; ++j) {
-        long double sse = 0.0L, tss = 0.0L;
-        for (int c = 0; c < q; ++c) {
-          sse += host_sums[(size_t)2 * q * j + 2 * c];
-          tss += host_sums[(size_t)2 * q * j + 2 * c + 1];
+    std::exception_ptr failed;
+    for (int f0 = 0; f0 < fp.count && !failed; f0 += per_batch) {
+      const int f1 = std::min(fp.count, f0 + per_batch);
+      // row positions of the batch's folds: one copy (a copy from pageable
+      // memory waits for its stream)
+      std::vector<int> host_pos((size_t)(f1 - f0) * n);
+      for (int f = f0; f < f1; ++f) fold_positions(fp.test[f], n, host_pos.data() + (size_t)(f - f0) * n);
+      DeviceArray<int> pos(host_pos.size(), lanes.main);
+      FPLS_CHECK(cudaMemcpyAsync(pos.get(), host_pos.data(), sizeof(int) * host_pos.size(),
+                                 cudaMemcpyHostToDevice, lanes.main));
+      lanes.lanes_after_main();
+      std::vector<std::unique_ptr<Fold<T>>> batch;
+      Settle settle{lanes};
+      try {
+        for (int f = f0; f < f1; ++f) {
+          const auto& held = fp.test[f];
+          if (held.empty()) {
+            status[f] = 2;
+            continue;
+          }
+          if (maximum_prefix > std::min(n - (int)held.size() - 1, p))
+            throw std::invalid_argument("CUDA CV component count exceeds a fold rank");
+          std::unique_ptr<Fold<T>> fold(new Fold<T>());
+          Fold<T>& d = *fold;
+          d.f = f;
+          d.m = q;
+          d.st = lanes.lane[batch.size() % std::min(fp.count, kLanes)];
+          d.nte = (int)held.size();
+          d.ntr = n - d.nte;
+          d.pos = pos.get() + (size_t)(f - f0) * n;
+          split_fold(d, X.get(), Y.get(), n, p, q);
+          d.ws.ensure(d.ntr, p, q, maximum_prefix, d.st);
+          FPLS_CHECK(cudaMemsetAsync(d.ws.flag.get(), 0, sizeof(int), d.st));
+          d.Yc.allocate((size_t)d.ntr * q, d.st);
+          d.ycsum.allocate(q, d.st);
+          d.model.ymean.allocate(q, d.st);
+          prepare_responses<T>(d.Ytr.get(), nullptr, d.ntr, q, d.Yc.get(), d.model.ymean.get(), d.ycsum.get(),
+                               d.ws.flag.get(), d.st);
+          fit_fold<T>(method, d, p, maximum_prefix, scaling, max_ctas);
+          batch.push_back(std::move(fold));
         }
-        metrics[j] += (double)sse;
-        fold_ss[j] += (double)tss;
-        counts[j] += (double)nte * q;
-        if (store_predictions)
-          for (int c = 0; c < q; ++c)
-            for (int i = 0; i < nte; ++i)
-              prediction_output[(size_t)j * n * q + (size_t)c * n + held[i]] =
-                  host_pred[(size_t)j * nte * q + (size_t)c * nte + i];
+      } catch (...) {
+        failed = std::current_exception();  // after the folds before it
       }
-      status[f] = 1;
+      launch_plans(batch, lanes);
+      for (auto& fold : batch) {
+        Fold<T>& d = *fold;
+        d.scores.allocate((size_t)d.nte * maximum_prefix, d.st);
+        d.pred.allocate((size_t)d.nte * q * step, d.st);
+        d.sums.allocate((size_t)2 * q * prefix_count, d.st);
+        d.host_sums.resize((size_t)2 * q * prefix_count);
+        if (store_predictions) d.host_pred.resize((size_t)d.nte * q * prefix_count);
+        project_rows<T>(d.model, d.Xte.get(), d.nte, d.nte, maximum_prefix, d.scores.get(), d.nte, d.ws, d.st);
+        for (int j = 0; j < prefix_count; j += step) {
+          const int w = std::min(step, prefix_count - j);
+          predict_prefixes<double>(d.model, d.scores.get(), d.nte, d.nte, prefixes + j, w, d.pred.get(), d.st);
+          fold_sums_kernel<<<dim3(q, w), 256, 0, d.st>>>(d.pred.get(), d.Yte.get(), d.model.ymean.get(), d.nte,
+                                                         q, d.sums.get() + (size_t)2 * q * j);
+          count_launch();
+          FPLS_LAUNCH("fold_sums");
+          if (store_predictions && step < prefix_count)
+            FPLS_CHECK(cudaMemcpyAsync(d.host_pred.data() + (size_t)j * d.nte * q, d.pred.get(),
+                                       sizeof(double) * d.nte * q * w, cudaMemcpyDeviceToHost, d.st));
+        }
+      }
+      // copies to pageable memory wait for their stream: after every fold is enqueued
+      for (auto& fold : batch) {
+        Fold<T>& d = *fold;
+        if (store_predictions && step == prefix_count)
+          FPLS_CHECK(cudaMemcpyAsync(d.host_pred.data(), d.pred.get(), sizeof(double) * d.host_pred.size(),
+                                     cudaMemcpyDeviceToHost, d.st));
+        FPLS_CHECK(cudaMemcpyAsync(d.host_sums.data(), d.sums.get(), sizeof(double) * d.host_sums.size(),
+                                   cudaMemcpyDeviceToHost, d.st));
+        FPLS_CHECK(cudaMemcpyAsync(&d.bad, d.ws.flag.get(), sizeof(int), cudaMemcpyDeviceToHost, d.st));
+      }
+      lanes.sync();
+      for (auto& fold : batch) {
+        Fold<T>& d = *fold;
+        if (d.bad)
+          throw std::runtime_error(method == kPlssvd
+              ? "resident PLS-SVD failed: invalid labels, decomposition or score Gram"
+              : "resident SIMPLS failed: invalid labels, decomposition or component norm");
+        const auto& held = fp.test[d.f];
+        for (int j = 0; j < prefix_count; ++j) {
+          long double sse = 0.0L, tss = 0.0L;
+          for (int c = 0; c < q; ++c) {
+            sse += d.host_sums[(size_t)2 * q * j + 2 * c];
+            tss += d.host_sums[(size_t)2 * q * j + 2 * c + 1];
+          }
+          metrics[j] += (double)sse;
+          fold_ss[j] += (double)tss;
+          counts[j] += (double)d.nte * q;
+          if (store_predictions)
+            for (int c = 0; c < q; ++c)
+              for (int i = 0; i < d.nte; ++i)
+                prediction_output[(size_t)j * n * q + (size_t)c * n + held[i]] =
+                    d.host_pred[((size_t)j * q + c) * d.nte + i];
+        }
+        status[d.f] = 1;
+      }
     }
+    if (failed) std::rethrow_exception(failed);
     const double nan = std::numeric_limits<double>::quiet_NaN();
     for (int j = 0; j < prefix_count; ++j) {
       const double sse = metrics[j];
@@ -225,7 +426,6 @@ void cv_regression(int method, const T* predictors, const T* responses,
       if (observed_r2_values) observed_r2_values[j] = r2;
       metrics[j] = metric == 4 ? rmsd : metric == 3 ? q2 : r2;
     }
-    FPLS_CHECK(cudaStreamSynchronize(s));
   }
 }
 
@@ -258,133 +458,178 @@ void cv_classification(int method, const T* predictors, const int* labels,
   if (fp.max_test < 1 || fp.max_train < 2)
     throw std::invalid_argument("CUDA CV contains an empty train or test fold");
 
-  cudaStream_t s = nullptr;
-  FPLS_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-  struct StreamGuard {
-    cudaStream_t s;
-    ~StreamGuard() {
-      if (s) {
-        cudaStreamSynchronize(s);
-        cudaStreamDestroy(s);
-      }
-    }
-  } guard{s};
+  Lanes lanes(fp.count);
   {
-    DeviceArray<T> X((size_t)n * p, s);
-    upload_h2d(X.get(), predictors, sizeof(T) * n * p, s);
-    DeviceArray<T> Xtr((size_t)fp.max_train * p, s), Xte((size_t)fp.max_test * p, s);
-    DeviceArray<int> idx_tr(fp.max_train, s), idx_te(fp.max_test, s);
-    const int step = prefixes_at_once((size_t)fp.max_test * classes * sizeof(double), prefix_count);
-    DeviceArray<int> lab_tr(fp.max_train, s), top((size_t)fp.max_test * step, s);
-    DeviceArray<double> Yc((size_t)fp.max_train * classes, s), ycsum(classes, s);
-    DeviceArray<double> scores((size_t)fp.max_test * maximum_prefix, s);
-    DeviceArray<double> pred((size_t)fp.max_test * classes * step, s);
-    Workspace ws;
-    ws.ensure(fp.max_train, p, classes, maximum_prefix, s);
+    DeviceArray<T> X((size_t)n * p, lanes.main);
+    upload_h2d(X.get(), predictors, sizeof(T) * n * p, lanes.main);
+    lanes.lanes_after_main();
+    const size_t block = (size_t)fp.max_test * classes;
+    const int step = prefixes_at_once(block * sizeof(double), prefix_count);
+    int per_batch = 1, max_ctas = 0;
+    batch_shape<T>(method, fp, n, p, classes, maximum_prefix, fp.count, 2 * block * step * sizeof(double),
+                   &per_batch, &max_ctas);
     std::fill(metrics, metrics + prefix_count, 0.0);
     std::vector<double> counts(prefix_count, 0.0);
     if (store_scores) std::fill(score_output, score_output + (size_t)n * classes * prefix_count, T(0));
-    std::vector<int> train, host_labels;
-    std::vector<double> host_scores;
-    for (int f = 0; f < fp.count; ++f) {
-      const auto& held = fp.test[f];
-      if (held.empty()) {
-        status[f] = 2;
-        continue;
+    std::exception_ptr failed;
+    for (int f0 = 0; f0 < fp.count && !failed; f0 += per_batch) {
+      const int f1 = std::min(fp.count, f0 + per_batch);
+      // row positions and compacted training labels of the batch's folds: one
+      // copy each (a copy from pageable memory waits for its stream)
+      std::vector<int> host_pos((size_t)(f1 - f0) * n), host_lab(host_pos.size(), 1);
+      std::vector<std::vector<int>> counts_of(f1 - f0, std::vector<int>(classes, 0));
+      for (int f = f0; f < f1; ++f) {
+        int* at = host_pos.data() + (size_t)(f - f0) * n;
+        int* lab = host_lab.data() + (size_t)(f - f0) * n;
+        std::vector<int>& cnt = counts_of[f - f0];
+        fold_positions(fp.test[f], n, at);
+        for (int i = 0; i < n; ++i)
+          if (at[i] >= 0) ++cnt[labels[i] - 1];
+        std::vector<int> map(classes, 0);
+        int next = 0;
+        for (int c = 0; c < classes; ++c)
+          if (cnt[c] > 0) map[c] = ++next;
+        for (int i = 0; i < n; ++i)
+          if (at[i] >= 0) lab[at[i]] = map[labels[i] - 1];
       }
-      std::vector<char> flag(n, 0);
-      for (int r : held) flag[r] = 1;
-      train.clear();
-      std::vector<int> cnt(classes, 0);
-      for (int i = 0; i < n; ++i)
-        if (!flag[i]) {
-          train.push_back(i);
-          ++cnt[labels[i] - 1];
+      DeviceArray<int> pos(host_pos.size(), lanes.main), lab(host_lab.size(), lanes.main);
+      FPLS_CHECK(cudaMemcpyAsync(pos.get(), host_pos.data(), sizeof(int) * host_pos.size(),
+                                 cudaMemcpyHostToDevice, lanes.main));
+      FPLS_CHECK(cudaMemcpyAsync(lab.get(), host_lab.data(), sizeof(int) * host_lab.size(),
+                                 cudaMemcpyHostToDevice, lanes.main));
+      lanes.lanes_after_main();
+      std::vector<std::unique_ptr<Fold<T>>> batch;
+      Settle settle{lanes};
+      try {
+        for (int f = f0; f < f1; ++f) {
+          const auto& held = fp.test[f];
+          if (held.empty()) {
+            status[f] = 2;
+            continue;
+          }
+          const std::vector<int>& cnt = counts_of[f - f0];
+          std::vector<int> active;
+          for (int c = 0; c < classes; ++c)
+            if (cnt[c] > 0) active.push_back(c + 1);
+          if (active.size() <= 1) {
+            const int fallback = active.empty() ? 1 : active.front();
+            for (int j = 0; j < prefix_count; ++j)
+              for (int r : held) {
+                if (store_predictions) prediction_output[(size_t)j * n + r] = fallback;
+                metrics[j] += labels[r] == fallback ? 1.0 : 0.0;
+                counts[j] += 1.0;
+              }
+            status[f] = 4;
+            continue;
+          }
+          if (maximum_prefix > std::min(n - (int)held.size() - 1, p))
+            throw std::invalid_argument("CUDA CV component count exceeds a fold rank");
+          std::unique_ptr<Fold<T>> fold(new Fold<T>());
+          Fold<T>& d = *fold;
+          d.f = f;
+          d.m = (int)active.size();
+          d.active = active;
+          d.st = lanes.lane[batch.size() % std::min(fp.count, kLanes)];
+          d.nte = (int)held.size();
+          d.ntr = n - d.nte;
+          d.pos = pos.get() + (size_t)(f - f0) * n;
+          d.lab = lab.get() + (size_t)(f - f0) * n;
+          split_fold(d, X.get(), static_cast<const T*>(nullptr), n, p, 0);
+          d.ws.ensure(d.ntr, p, d.m, maximum_prefix, d.st);
+          FPLS_CHECK(cudaMemsetAsync(d.ws.flag.get(), 0, sizeof(int), d.st));
+          d.Yc.allocate((size_t)d.ntr * d.m, d.st);
+          d.ycsum.allocate(d.m, d.st);
+          d.model.classification = true;
+          d.model.label_view = d.lab;
+          for (int c : active) d.model.class_counts.push_back(cnt[c - 1]);
+          d.model.ymean.allocate(d.m, d.st);
+          prepare_responses<T>(nullptr, d.lab, d.ntr, d.m, d.Yc.get(), d.model.ymean.get(),
+                               d.ycsum.get(), d.ws.flag.get(), d.st);
+          fit_fold<T>(method, d, p, maximum_prefix, scaling, max_ctas);
+          batch.push_back(std::move(fold));
         }
-      std::vector<int> active, active_map(classes, -1);
-      for (int c = 0; c < classes; ++c)
-        if (cnt[c] > 0) {
-          active_map[c] = (int)active.size();
-          active.push_back(c + 1);
+      } catch (...) {
+        failed = std::current_exception();  // after the folds before it
+      }
+      launch_plans(batch, lanes);
+      std::vector<std::vector<double>> host_scores(batch.size());
+      for (size_t b = 0; b < batch.size(); ++b) {
+        Fold<T>& d = *batch[b];
+        const int c = d.m;
+        d.scores.allocate((size_t)d.nte * maximum_prefix, d.st);
+        d.pred.allocate((size_t)d.nte * c * step, d.st);
+        if (use_lda && store_scores) d.sums.allocate((size_t)d.nte * c * step, d.st);
+        d.top.allocate((size_t)d.nte * step, d.st);
+        project_rows<T>(d.model, d.Xte.get(), d.nte, d.nte, maximum_prefix, d.scores.get(), d.nte, d.ws, d.st);
+        if (use_lda) {
+          d.lda.reset(new LdaState());
+          d.lda->train(d.model.T.get(), d.ntr, d.ntr, maximum_prefix, d.lab, c, d.model.class_counts,
+                       d.ws.flag.get(), d.st);
         }
-      if (active.size() <= 1) {
-        const int fallback = active.empty() ? 1 : active.front();
-        for (int j = 0; j < prefix_count; ++j)
-          for (int r : held) {
-            if (store_predictions) prediction_output[(size_t)j * n + r] = fallback;
-            metrics[j] += labels[r] == fallback ? 1.0 : 0.0;
+        d.host_labels.assign((size_t)d.nte * prefix_count, 0);
+        if (store_scores) host_scores[b].resize((size_t)d.nte * c * prefix_count);
+        for (int j = 0; j < prefix_count; j += step) {
+          const int w = std::min(step, prefix_count - j);
+          // class indicators (stored, or decoded by the argmax head) and the
+          // LDA discriminants
+          double* resp = use_lda ? d.sums.get() : d.pred.get();
+          if (store_scores || !use_lda)
+            predict_prefixes<double>(d.model, d.scores.get(), d.nte, d.nte, prefixes + j, w, resp, d.st);
+          if (use_lda) d.lda->discriminants(d.scores.get(), d.nte, d.nte, prefixes + j, w, d.pred.get(), d.st);
+          topk_rows(d.pred.get(), d.nte, c, 1, w, d.top.get(), d.nte, d.st);
+          if (step < prefix_count) {
+            if (store_scores)
+              FPLS_CHECK(cudaMemcpyAsync(host_scores[b].data() + (size_t)j * d.nte * c, resp,
+                                         sizeof(double) * d.nte * c * w, cudaMemcpyDeviceToHost, d.st));
+            FPLS_CHECK(cudaMemcpyAsync(d.host_labels.data() + (size_t)j * d.nte, d.top.get(),
+                                       sizeof(int) * d.nte * w, cudaMemcpyDeviceToHost, d.st));
+          }
+        }
+      }
+      // copies to pageable memory wait for their stream: after every fold is enqueued
+      for (size_t b = 0; b < batch.size(); ++b) {
+        Fold<T>& d = *batch[b];
+        if (step == prefix_count) {
+          if (store_scores)
+            FPLS_CHECK(cudaMemcpyAsync(host_scores[b].data(), use_lda ? d.sums.get() : d.pred.get(),
+                                       sizeof(double) * host_scores[b].size(), cudaMemcpyDeviceToHost, d.st));
+          FPLS_CHECK(cudaMemcpyAsync(d.host_labels.data(), d.top.get(), sizeof(int) * d.host_labels.size(),
+                                     cudaMemcpyDeviceToHost, d.st));
+        }
+        FPLS_CHECK(cudaMemcpyAsync(&d.bad, d.ws.flag.get(), sizeof(int), cudaMemcpyDeviceToHost, d.st));
+      }
+      lanes.sync();
+      for (size_t b = 0; b < batch.size(); ++b) {
+        Fold<T>& d = *batch[b];
+        const int c = d.m;
+        const auto& held = fp.test[d.f];
+        if (d.bad)
+          throw std::runtime_error(method == kPlssvd
+              ? "resident PLS-SVD failed: invalid labels, decomposition or score Gram"
+              : "resident SIMPLS failed: invalid labels, decomposition or component norm");
+        for (int j = 0; j < prefix_count; ++j) {
+          for (int i = 0; i < d.nte; ++i) {
+            const int predicted = d.active[d.host_labels[(size_t)j * d.nte + i] - 1];
+            const int row = held[i];
+            if (store_predictions) prediction_output[(size_t)j * n + row] = predicted;
+            metrics[j] += predicted == labels[row] ? 1.0 : 0.0;
             counts[j] += 1.0;
           }
-        status[f] = 4;
-        continue;
-      }
-      const int ntr = (int)train.size(), nte = (int)held.size();
-      const int c = (int)active.size();
-      if (maximum_prefix > std::min(ntr - 1, p))
-        throw std::invalid_argument("CUDA CV component count exceeds a fold rank");
-      std::vector<int> compact(ntr);
-      std::vector<int> ccount(c, 0);
-      for (int i = 0; i < ntr; ++i) {
-        compact[i] = active_map[labels[train[i]] - 1] + 1;
-        ++ccount[compact[i] - 1];
-      }
-      FPLS_CHECK(cudaMemcpyAsync(idx_tr.get(), train.data(), sizeof(int) * ntr, cudaMemcpyHostToDevice, s));
-      FPLS_CHECK(cudaMemcpyAsync(idx_te.get(), held.data(), sizeof(int) * nte, cudaMemcpyHostToDevice, s));
-      FPLS_CHECK(cudaMemcpyAsync(lab_tr.get(), compact.data(), sizeof(int) * ntr, cudaMemcpyHostToDevice, s));
-      gather_rows<T>(X.get(), n, p, idx_tr.get(), ntr, Xtr.get(), ntr, s);
-      gather_rows<T>(X.get(), n, p, idx_te.get(), nte, Xte.get(), nte, s);
-      FPLS_CHECK(cudaMemsetAsync(ws.flag.get(), 0, sizeof(int), s));
-      DeviceModel model;
-      model.classification = true;
-      model.label_view = lab_tr.get();
-      model.ymean.allocate(c, s);
-      prepare_responses<T>(nullptr, lab_tr.get(), ntr, c, Yc.get(), model.ymean.get(), ycsum.get(), ws.flag.get(), s);
-      fit_method<T>(method, Xtr.get(), ntr, p, Yc.get(), ycsum.get(), c, maximum_prefix, scaling, model, ws, s);
-      project_rows<T>(model, Xte.get(), nte, nte, maximum_prefix, scores.get(), nte, ws, s);
-      std::unique_ptr<LdaState> lda;
-      if (use_lda) {
-        lda.reset(new LdaState());
-        lda->train(model.T.get(), ntr, ntr, maximum_prefix, lab_tr.get(), c, ccount, ws.flag.get(), s);
-      }
-      host_labels.resize((size_t)nte * prefix_count);
-      if (store_scores) host_scores.resize((size_t)nte * c * prefix_count);
-      for (int j = 0; j < prefix_count; j += step) {
-        const int w = std::min(step, prefix_count - j);
-        if (store_scores || !use_lda)
-          predict_prefixes<double>(model, scores.get(), nte, nte, prefixes + j, w, pred.get(), s);
-        if (store_scores)
-          FPLS_CHECK(cudaMemcpyAsync(host_scores.data() + (size_t)j * nte * c, pred.get(),
-                                     sizeof(double) * nte * c * w, cudaMemcpyDeviceToHost, s));
-        if (use_lda) lda->discriminants(scores.get(), nte, nte, prefixes + j, w, pred.get(), s);
-        topk_rows(pred.get(), nte, c, 1, w, top.get(), nte, s);
-        FPLS_CHECK(cudaMemcpyAsync(host_labels.data() + (size_t)j * nte, top.get(),
-                                   sizeof(int) * nte * w, cudaMemcpyDeviceToHost, s));
-      }
-      raise_on_flag(ws, s, method == kPlssvd
-          ? "resident PLS-SVD failed: invalid labels, decomposition or score Gram"
-          : "resident SIMPLS failed: invalid labels, decomposition or component norm");
-      for (int j = 0; j < prefix_count; ++j) {
-        for (int i = 0; i < nte; ++i) {
-          const int predicted = active[host_labels[(size_t)j * nte + i] - 1];
-          const int row = held[i];
-          if (store_predictions) prediction_output[(size_t)j * n + row] = predicted;
-          metrics[j] += predicted == labels[row] ? 1.0 : 0.0;
-          counts[j] += 1.0;
+          if (store_scores)
+            for (int ai = 0; ai < c; ++ai) {
+              const int dest = d.active[ai] - 1;
+              for (int i = 0; i < d.nte; ++i)
+                score_output[(size_t)j * n * classes + (size_t)dest * n + held[i]] =
+                    static_cast<T>(host_scores[b][((size_t)j * c + ai) * d.nte + i]);
+            }
         }
-        if (store_scores)
-          for (int ai = 0; ai < c; ++ai) {
-            const int dest = active[ai] - 1;
-            for (int i = 0; i < nte; ++i)
-              score_output[(size_t)j * n * classes + (size_t)dest * n + held[i]] =
-                  static_cast<T>(host_scores[(size_t)j * nte * c + (size_t)ai * nte + i]);
-          }
+        status[d.f] = 1;
       }
-      status[f] = 1;
     }
+    if (failed) std::rethrow_exception(failed);
     for (int j = 0; j < prefix_count; ++j)
       metrics[j] = counts[j] > 0.0 ? metrics[j] / counts[j]
                                    : std::numeric_limits<double>::quiet_NaN();
-    FPLS_CHECK(cudaStreamSynchronize(s));
   }
 }
 

@@ -587,9 +587,10 @@ void fit_simpls(const T* X, int n, int p, long ld, const double* Yc,
   // (or handed to the caller's batch when it collects plans)
   if (block <= 1 && !gram_route) {
     std::unique_ptr<PersistentPlan> plan(new PersistentPlan());
-    if (plan_simpls_persistent<T>(X, n, p, ld, m, a_max, model, S, gpk, ws, stream, *plan)) {
-      if (std::unique_ptr<PersistentPlan>* sink = persistent_deferral()) {
-        *sink = std::move(plan);
+    const PersistentDeferral& defer = persistent_deferral();
+    if (plan_simpls_persistent<T>(X, n, p, ld, m, a_max, model, S, gpk, ws, stream, *plan, defer.max_ctas)) {
+      if (defer.sink) {
+        *defer.sink = std::move(plan);
       } else {
         launch_persistent({plan.get()}, stream);
       }

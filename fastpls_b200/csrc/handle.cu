@@ -254,8 +254,8 @@ class TypedHandle final : public ResidentHandle {
       FPLS_CHECK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
       if (defer && rq_.method == kSimpls) {
         struct Sink {
-          explicit Sink(std::unique_ptr<PersistentPlan>* s) { persistent_deferral() = s; }
-          ~Sink() { persistent_deferral() = nullptr; }
+          explicit Sink(std::unique_ptr<PersistentPlan>* s) { persistent_deferral() = {s, 0}; }
+          ~Sink() { persistent_deferral() = {}; }
         } sink(&pending_);
         fit_begin();
       } else {

@@ -92,11 +92,6 @@ void xtv_product(const T* X, int n, int p, long ld, const double* V, long ldv,
                  int nb, double* out, long ldo, DeviceArray<double>& scratch,
                  cudaStream_t stream);
 
-// Copy rows idx[0..count) of a column-major (rows x cols) matrix.
-template <class T>
-void gather_rows(const T* src, long ld_src, int cols, const int* idx, int count,
-                 T* dst, long ld_dst, cudaStream_t stream);
-
 // ---------------------------------------------------------------- misc
 // One-based top-k per row of `count` consecutive column-major (rows x classes)
 // FP64 matrices (out: ldo x top each); the lower class index wins ties

@@ -1054,17 +1054,17 @@ PersistentWaitTest& persistent_wait_test() {
   return t;
 }
 
-std::unique_ptr<PersistentPlan>*& persistent_deferral() {
-  thread_local std::unique_ptr<PersistentPlan>* sink = nullptr;
-  return sink;
+PersistentDeferral& persistent_deferral() {
+  thread_local PersistentDeferral deferral;
+  return deferral;
 }
 
 namespace {
 
 // Regions of a fit of n x p: Cr row blocks of rb rows times Cc column ranges
-// of pc columns (a function of the shape only); false when the shape does
+// of pc columns (a function of the shape and max_ctas only); false when the shape does
 // not fit the persistent launch.
-bool persistent_grid(int n, int p, int& Cr, int& Cc, int& rb, int& pc) {
+bool persistent_grid(int n, int p, int max_ctas, int& Cr, int& Cc, int& rb, int& pc) {
   const long elems = (long)n * p;
   // Elements per CTA: a CTA streams a few tens of GB/s, so small fits spread
   // until the barriers cost what the passes save -- 2^13 elements up to 32 CTAs,
@@ -1074,7 +1074,8 @@ bool persistent_grid(int n, int p, int& Cr, int& Cc, int& rb, int& pc) {
   // 466 / 477 / 421). Fewer CTAs per fit also leave room for other fits of a
   // batch in one launch.
   const int shift = elems <= (32L << 13) ? 13 : 14;
-  const int c0 = (int)std::max(1L, std::min<long>(2L * num_sms(), (elems + (1L << shift) - 1) >> shift));
+  const long most = max_ctas > 0 ? std::min<long>(max_ctas, 2L * num_sms()) : 2L * num_sms();
+  const int c0 = (int)std::max(1L, std::min<long>(most, (elems + (1L << shift) - 1) >> shift));
   Cr = (n + kBlockRows - 1) / kBlockRows;
   rb = round_up((n + Cr - 1) / Cr, 8);
   Cr = (n + rb - 1) / rb;
@@ -1085,9 +1086,9 @@ bool persistent_grid(int n, int p, int& Cr, int& Cc, int& rb, int& pc) {
 
 }  // namespace
 
-int persistent_ctas(int n, int p) {
+int persistent_ctas(int n, int p, int max_ctas) {
   int Cr, Cc, rb, pc;
-  return persistent_grid(n, p, Cr, Cc, rb, pc) ? Cr * Cc : 0;
+  return persistent_grid(n, p, max_ctas, Cr, Cc, rb, pc) ? Cr * Cc : 0;
 }
 
 namespace {
@@ -1119,7 +1120,7 @@ int persistent_capacity(int elem) {
 template <class T>
 bool plan_simpls_persistent(const T* X, int n, int p, long ld, int m, int a, DeviceModel& model,
                             DeviceArray<double>& S, double* gpk, Workspace& ws, cudaStream_t stream,
-                            PersistentPlan& plan) {
+                            PersistentPlan& plan, int max_ctas) {
   if (!persistent_enabled() || !persistent_supported(m, a) || n < 2 || p < 1) return false;
   // Large fits take the per-kernel loop: its streaming kernels keep more
   // loads in flight (many CTAs per SM) and a component's two passes over X
@@ -1127,7 +1128,7 @@ bool plan_simpls_persistent(const T* X, int n, int p, long ld, int m, int a, Dev
   // passes are short and the per-component launches dominate.
   if ((long)n * p > kPersistMaxElements) return false;
   int Cr, Cc, rb, pc;
-  if (!persistent_grid(n, p, Cr, Cc, rb, pc)) return false;
+  if (!persistent_grid(n, p, max_ctas, Cr, Cc, rb, pc)) return false;
   const int C = Cr * Cc;
   const int cap = capacity_of<T>();
   if (cap == 0 || C > cap) return false;
@@ -1298,12 +1299,12 @@ template bool xr_ring<bf16>(const bf16*, int, int, long, const double*, long, in
 
 template bool plan_simpls_persistent<float>(const float*, int, int, long, int, int, DeviceModel&,
                                             DeviceArray<double>&, double*, Workspace&, cudaStream_t,
-                                            PersistentPlan&);
+                                            PersistentPlan&, int);
 template bool plan_simpls_persistent<double>(const double*, int, int, long, int, int, DeviceModel&,
                                              DeviceArray<double>&, double*, Workspace&, cudaStream_t,
-                                             PersistentPlan&);
+                                             PersistentPlan&, int);
 template bool plan_simpls_persistent<bf16>(const bf16*, int, int, long, int, int, DeviceModel&,
                                            DeviceArray<double>&, double*, Workspace&, cudaStream_t,
-                                           PersistentPlan&);
+                                           PersistentPlan&, int);
 
 }  // namespace fpls

@@ -51,9 +51,11 @@ struct PersistentPlan {
 
 // Whether the persistent path takes a fit with m responses and a components.
 bool persistent_supported(int m, int a);
-// CTAs a fit of n x p gets (a function of the shape only; 0: the shape does
-// not fit a persistent launch).
-int persistent_ctas(int n, int p);
+// CTAs a fit of n x p gets (a function of the shape and of max_ctas only; 0:
+// the shape does not fit a persistent launch). max_ctas > 0: a caller that
+// runs several fits in one launch gives each its share, as far as the shape
+// allows.
+int persistent_ctas(int n, int p, int max_ctas = 0);
 // CTAs one launch can hold co-resident for a storage type (0: unavailable).
 int persistent_capacity(int elem);
 
@@ -66,16 +68,21 @@ int persistent_capacity(int elem);
 template <class T>
 bool plan_simpls_persistent(const T* X, int n, int p, long ld, int m, int a, DeviceModel& model,
                             DeviceArray<double>& S, double* gpk, Workspace& ws, cudaStream_t stream,
-                            PersistentPlan& plan);
+                            PersistentPlan& plan, int max_ctas = 0);
 
 // One cooperative launch for the planned fits (one storage type, total CTAs
 // within persistent_capacity) on `stream`, which must already be ordered
 // after the work that produced each plan.
 void launch_persistent(const std::vector<PersistentPlan*>& plans, cudaStream_t stream);
 
-// When set on this thread, a SIMPLS fit that plans a persistent launch hands
-// the plan to *sink instead of launching it (the caller batches plans).
-std::unique_ptr<PersistentPlan>*& persistent_deferral();
+// When its sink is set on this thread, a SIMPLS fit that plans a persistent
+// launch (with the caller's max_ctas) hands the plan to *sink instead of
+// launching it (the caller batches plans).
+struct PersistentDeferral {
+  std::unique_ptr<PersistentPlan>* sink = nullptr;
+  int max_ctas = 0;
+};
+PersistentDeferral& persistent_deferral();
 
 // Process-wide switch (1 = use the persistent path where it applies).
 int& persistent_enabled();

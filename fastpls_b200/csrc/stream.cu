@@ -491,19 +491,6 @@ void xr_launch(const T* X, int n, int p, long ld, const double* R, long ldr,
   FPLS_LAUNCH("xr_finish");
 }
 
-template <class T>
-__global__ void gather_rows_kernel(const T* __restrict__ src, long ld_src,
-                                   int cols, const int* __restrict__ idx,
-                                   int count, T* __restrict__ dst, long ld_dst) {
-  const long total = (long)count * cols;
-  for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < total;
-       k += (long)gridDim.x * blockDim.x) {
-    const int r = (int)(k % count);
-    const long c = k / count;
-    dst[r + c * ld_dst] = src[idx[r] + c * ld_src];
-  }
-}
-
 __global__ void topk_kernel(const double* __restrict__ v, int rows, int classes,
                             int top, int* __restrict__ out, long ldo) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -703,17 +690,6 @@ void xr_product(const T* X, int n, int p, long ld, const double* R, long ldr,
   else xr_launch<T, 2>(X, n, p, ld, R, ldr, nb, offset, offset_parts, out, ldo, scratch, stream);
 }
 
-template <class T>
-void gather_rows(const T* src, long ld_src, int cols, const int* idx, int count,
-                 T* dst, long ld_dst, cudaStream_t stream) {
-  if (count <= 0 || cols <= 0) return;
-  const long total = (long)count * cols;
-  const unsigned blocks = (unsigned)std::min<long>((total + 255) / 256, 16L * num_sms());
-  gather_rows_kernel<T><<<blocks, 256, 0, stream>>>(src, ld_src, cols, idx, count, dst, ld_dst);
-  count_launch();
-  FPLS_LAUNCH("gather_rows");
-}
-
 void topk_rows(const double* values, int rows, int classes, int top, int count, int* out,
                long ldo, cudaStream_t stream) {
   if (rows <= 0 || count <= 0) return;
@@ -734,14 +710,11 @@ void topk_rows(const double* values, int rows, int classes, int top, int count, 
                                cudaStream_t);                                 \
   template void xr_product<T>(const T*, int, int, long, const double*, long,  \
                               int, const double*, int, double*, long,         \
-                              DeviceArray<double>&, cudaStream_t);            \
-  template void gather_rows<T>(const T*, long, int, const int*, int, T*,      \
-                               long, cudaStream_t);
+                              DeviceArray<double>&, cudaStream_t);
+
 FPLS_INSTANTIATE(float)
 FPLS_INSTANTIATE(double)
 FPLS_INSTANTIATE(bf16)
-template void gather_rows<int>(const int*, long, int, const int*, int, int*,
-                               long, cudaStream_t);
 #undef FPLS_INSTANTIATE
 
 }  // namespace fpls

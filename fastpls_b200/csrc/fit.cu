@@ -34,14 +34,22 @@ namespace fpls {
 namespace {
 
 constexpr int TB = 256;
+// Rows (predictors) per block of the p-vector kernels, whose TB threads share
+// them: 157 blocks at p = 10000, where 256 rows a block left 108 SMs idle.
+constexpr int PB = 64;
+constexpr int kGemmCrossResponses = 5;
 
+// One block per response: bound by the latency of its loads (1024 threads; 256
+// took 83 us at 40003 rows, 12 classes, 29 now).
+constexpr int kCenterThreads = 1024;
 template <class T>
-__global__ void center_dense(const T* __restrict__ Y, int n, int m,
+__global__ void __launch_bounds__(kCenterThreads) center_dense(const T* __restrict__ Y, int n, int m,
                              double* __restrict__ Yc, double* ymean,
                              double* ycsum, int* flag) {
   __shared__ double scratch[32];
   const int c = blockIdx.x;
   double s = 0.0;
+#pragma unroll 4
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double y = as_f64(Y[i + (long)c * n]);
     if (!isfinite(y)) flag_error(flag, 3);
@@ -49,6 +57,7 @@ __global__ void center_dense(const T* __restrict__ Y, int n, int m,
   }
   const double mu = block_sum(s, scratch) / n;
   double r = 0.0;
+#pragma unroll 4
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double v = as_f64(Y[i + (long)c * n]) - mu;
     Yc[i + (long)c * n] = v;
@@ -61,12 +70,13 @@ __global__ void center_dense(const T* __restrict__ Y, int n, int m,
   }
 }
 
-__global__ void center_labels(const int* __restrict__ labels, int n, int m,
+__global__ void __launch_bounds__(kCenterThreads) center_labels(const int* __restrict__ labels, int n, int m,
                               double* __restrict__ Yc, double* ymean,
                               double* ycsum, int* flag) {
   __shared__ double scratch[32];
   const int c = blockIdx.x;
   double cnt = 0.0;
+#pragma unroll 4
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const int l = labels[i];
     if (l < 1 || l > m) flag_error(flag, 2);
@@ -74,6 +84,7 @@ __global__ void center_labels(const int* __restrict__ labels, int n, int m,
   }
   const double prior = block_sum(cnt, scratch) / n;
   double r = 0.0;
+#pragma unroll 4
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double v = (labels[i] == c + 1 ? 1.0 : 0.0) - prior;
     Yc[i + (long)c * n] = v;
@@ -119,14 +130,14 @@ __global__ void finish_moments(const double* __restrict__ sum,
 // triangle), by decreasing eigenvalue (ties: lower index first):
 // zs[k + j m] = z_j / sqrt(lambda_j), sign fixed so the largest-magnitude
 // entry of z_j is positive; lambda_out = lambda_0.
-__global__ void direction_kernel(const double* __restrict__ gpk, int m,
-                                 double* zs, double* lambda_out, int* flag, int count) {
-  extern __shared__ double sm[];
+// Whole block; sm: direction_smem(m) doubles.
+__device__ void direction(const double* gpk, int m, double* zs, double* lambda_out, int* flag, int count,
+                          double* sm) {
   double* A = sm;
   double* E = sm + m * m;
   for (int c = threadIdx.x; c < m; c += blockDim.x)
     for (int d = 0; d <= c; ++d) {
-      const double v = gpk[c * (c + 1) / 2 + d];
+      const double v = __ldcg(gpk + c * (c + 1) / 2 + d);
       A[c + d * m] = v;
       A[d + c * m] = v;
     }
@@ -181,6 +192,17 @@ __global__ void direction_kernel(const double* __restrict__ gpk, int m,
   }
 }
 
+// A, B, C, v of the dominant pair (one direction), or A, E of the Jacobi sweeps
+__host__ __device__ inline size_t direction_smem(int m) {
+  return m <= kDominantMaxOrder ? 3 * (size_t)m * m + m + 2 : 2 * (size_t)m * m;
+}
+
+__global__ void direction_kernel(const double* __restrict__ gpk, int m,
+                                 double* zs, double* lambda_out, int* flag, int count) {
+  extern __shared__ double sm[];
+  direction(gpk, m, zs, lambda_out, flag, count, sm);
+}
+
 // r = S zs ; rt = r / scale ; scal[0] = mean . rt
 __global__ void rvec_kernel(const double* __restrict__ S, int p, int m,
                             const double* __restrict__ zs,
@@ -206,47 +228,40 @@ __global__ void rvec_kernel(const double* __restrict__ S, int p, int m,
   last_block_reduce(vals, 1, partial, counter, scal);
 }
 
-// scal[1] = sum t^2, scal[2] = sum t
-__global__ void tstats_kernel(const double* __restrict__ t, int n,
-                              double* partial, unsigned* counter,
-                              double* scal) {
-  __shared__ double scratch[32];
-  __shared__ double vals[2];
-  double a = 0.0, b = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += gridDim.x * blockDim.x) {
-    a = fma(t[i], t[i], a);
-    b += t[i];
-  }
-  a = block_sum(a, scratch);
-  b = block_sum(b, scratch);
-  if (threadIdx.x == 0) {
-    vals[0] = a;
-    vals[1] = b;
-  }
-  __syncthreads();
-  last_block_reduce(vals, 2, partial, counter, scal + 1);
-}
-
-// Warp-strided block reduction of `count` dot products over the block's row
-// range: out[k] = sum_{j in block} col_k[j] * w[j] (w in shared memory).
+// Dot products over the block's rows: out[k] = sum_{j in block} col_k[j] w[j]
+// (w in shared memory), a warp per column, four columns of a warp at once so
+// that their loads overlap.
 __device__ inline void block_dots(const double* __restrict__ M, long ldm,
                                   int j0, int rows, const double* w, int count,
                                   double* out) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int warps = blockDim.x >> 5;
-  for (int k = warp; k < count; k += warps) {
-    double acc = 0.0;
-    for (int j = lane; j < rows; j += 32) acc = fma(M[j0 + j + (long)k * ldm], w[j], acc);
-    acc = warp_sum(acc);
-    if (lane == 0) out[k] = acc;
+  constexpr int W = TB / 32, U = 4;
+  for (int kb = warp; kb < count; kb += U * W) {
+    double acc[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      acc[u] = 0.0;
+      const int k = kb + u * W;
+      if (k < count)
+#pragma unroll
+        for (int j = 0; j < PB; j += 32)
+          if (j + lane < rows) acc[u] = fma(M[j0 + j + lane + (long)k * ldm], w[j + lane], acc[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const double s = warp_sum(acc[u]);
+      if (lane == 0 && kb + u * W < count) out[kb + u * W] = s;
+    }
   }
 }
 
 // p = (praw - mean * sum t) / (scale * ||t||) ; R[:,a] = r / ||t||
-// out (last block): h = V^T p (a_cur), q = S0^T R[:,a] (m)
+// out (last block): h = V^T p (a_cur), q = S0^T R[:,a] (m), also Q[:,a]
 // When `loading` is given (cached-Gram route) p = loading / ||t|| directly.
-__global__ void tail1_kernel(const double* __restrict__ praw,
+// Latency-bound (p (a + m) doubles read once): 31 us at p = 10000, a + m = 35
+// with 256-row blocks and serial partial sums, 16 us now.
+__global__ void __launch_bounds__(TB)
+    tail1_kernel(const double* __restrict__ praw,
                              const double* __restrict__ mean,
                              const double* __restrict__ scale,
                              const double* __restrict__ scal,
@@ -255,13 +270,14 @@ __global__ void tail1_kernel(const double* __restrict__ praw,
                              const double* __restrict__ V, int p, int m,
                              int a_cur, double* pvec, double* Rcol,
                              double* partial, unsigned* counter, double* hq,
-                             int* flag, const double* __restrict__ loading = nullptr) {
+                             int* flag, double* Qcol, double* tnorm2,
+                             const double* __restrict__ loading = nullptr) {
   extern __shared__ double sm[];
-  double* ps = sm;            // TB
-  double* rs = sm + TB;       // TB
-  double* vals = sm + 2 * TB; // a_cur + m
-  const int j0 = blockIdx.x * TB;
-  const int rows = min(TB, p - j0);
+  double* ps = sm;            // PB
+  double* rs = sm + PB;       // PB
+  double* vals = sm + 2 * PB; // a_cur + m
+  const int j0 = blockIdx.x * PB;
+  const int rows = min(PB, p - j0);
   const double tn = sqrt(scal[1]);
   if (!(tn > 0.0) || !isfinite(tn)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) flag_error(flag, 1);
@@ -281,29 +297,44 @@ __global__ void tail1_kernel(const double* __restrict__ praw,
   block_dots(V, p, j0, rows, ps, a_cur, vals);
   block_dots(S0, p, j0, rows, rs, m, vals + a_cur);
   __syncthreads();
-  last_block_reduce(vals, a_cur + m, partial, counter, hq);
+  if (!last_block_reduce(vals, a_cur + m, partial, counter, hq)) return;
+  // Q[:, a] and ||t||^2 (for the scaling of T after the last component)
+  __syncthreads();
+  for (int c = t; c < m; c += TB) Qcol[c] = hq[a_cur + c];
+  if (t == 0) *tnorm2 = scal[1];
 }
 
-// v = p - V h ; out (last block): [v.v, S^T v (m)]
-__global__ void tail2_kernel(const double* __restrict__ pvec,
+// v = p - V h ; out (last block): [v.v, S^T v (m)]. A row's sum over the
+// components is shared by TB / PB threads. 24 us at p = 10000, a = 25 before,
+// 12 us now.
+__global__ void __launch_bounds__(TB)
+    tail2_kernel(const double* __restrict__ pvec,
                              const double* __restrict__ V,
                              const double* __restrict__ hq,
                              const double* __restrict__ S, int p, int m,
                              int a_cur, double* v, double* partial,
                              unsigned* counter, double* vr) {
   extern __shared__ double sm[];
-  double* vs = sm;             // TB
-  double* vals = sm + TB;      // 1 + m
+  double* vs = sm;             // PB
+  double* vals = sm + PB;      // 1 + m
   __shared__ double scratch[32];
-  const int j0 = blockIdx.x * TB;
-  const int rows = min(TB, p - j0);
-  const int t = threadIdx.x;
+  __shared__ double part[TB];
+  constexpr int G = TB / PB;
+  const int j0 = blockIdx.x * PB;
+  const int rows = min(PB, p - j0);
+  const int t = threadIdx.x, row = t % PB, g = t / PB;
+  double q = 0.0;
+  if (row < rows) {
+#pragma unroll 8
+    for (int k = g; k < a_cur; k += G) q = fma(V[j0 + row + (long)k * p], hq[k], q);
+  }
+  part[t] = q;
+  __syncthreads();
   double vj = 0.0;
   if (t < rows) {
-    const int j = j0 + t;
-    vj = pvec[j];
-    for (int k = 0; k < a_cur; ++k) vj = fma(-V[j + (long)k * p], hq[k], vj);
-    v[j] = vj;
+    for (int u = 1; u < G; ++u) q += part[t + u * PB];
+    vj = pvec[j0 + t] - q;
+    v[j0 + t] = vj;
     vs[t] = vj;
   }
   __syncthreads();
@@ -316,17 +347,20 @@ __global__ void tail2_kernel(const double* __restrict__ pvec,
 
 // V[:,a] = v / ||v|| ; S -= V[:,a] (row / ||v||) ; G partials of updated S
 // (packed lower triangle) reduced by the last block into gpk.
-// When `update` is false only the Gram of S is formed.
-__global__ void tail3_kernel(const double* __restrict__ v,
+// When `update` is false only the Gram of S is formed. With zs the last block
+// goes on to the next direction (direction()), which was a launch of its own
+// (15 us at 10 responses).
+__global__ void __launch_bounds__(TB)
+    tail3_kernel(const double* __restrict__ v,
                              const double* __restrict__ vr, double* S, int p,
                              int m, double* Vcol, bool update, double* partial,
-                             unsigned* counter, double* gpk, int* flag) {
+                             unsigned* counter, double* gpk, int* flag, double* zs,
+                             double* lambda_out) {
   extern __shared__ double sm[];
-  const int jb = blockDim.x;
-  double* ss = sm;                 // jb x m
-  double* vals = sm + jb * m;      // m(m+1)/2
-  const int j0 = blockIdx.x * jb;
-  const int rows = min(jb, p - j0);
+  double* ss = sm;                 // PB x m
+  double* vals = sm + PB * m;      // m(m+1)/2
+  const int j0 = blockIdx.x * PB;
+  const int rows = min(PB, p - j0);
   const int t = threadIdx.x;
   double vn = 1.0;
   if (update) {
@@ -337,48 +371,49 @@ __global__ void tail3_kernel(const double* __restrict__ v,
     }
   }
   const double inv = vn > 0.0 ? 1.0 / vn : 0.0;
-  if (t < rows) {
-    const int j = j0 + t;
+  const int row = t % PB;
+  if (row < rows) {
+    const int j = j0 + row;
     const double vj = update ? v[j] * inv : 0.0;
-    if (update) Vcol[j] = vj;
-    for (int c = 0; c < m; ++c) {
+    if (update && t < PB) Vcol[j] = vj;
+#pragma unroll 4
+    for (int c = t / PB; c < m; c += TB / PB) {
       double s = S[j + (long)c * p];
       if (update) {
         s = fma(-vj, vr[1 + c] * inv, s);
         S[j + (long)c * p] = s;
       }
-      ss[t + c * jb] = s;
+      ss[row + c * PB] = s;
     }
   }
   __syncthreads();
   const int pairs = m * (m + 1) / 2;
-  const int lane = t & 31, warp = t >> 5, warps = jb >> 5;
-  for (int k = warp; k < pairs; k += warps) {
+  const int lane = t & 31, warp = t >> 5;
+  for (int k = warp; k < pairs; k += TB / 32) {
     // k -> (c, d) with d <= c, k = c(c+1)/2 + d
-    int c = (int)((sqrt(8.0 * k + 1.0) - 1.0) * 0.5);
+    int c = (int)((sqrtf(8.0f * k + 1.0f) - 1.0f) * 0.5f);
     while (c * (c + 1) / 2 > k) --c;
     while ((c + 1) * (c + 2) / 2 <= k) ++c;
     const int d = k - c * (c + 1) / 2;
     double acc = 0.0;
-    for (int j = lane; j < rows; j += 32) acc = fma(ss[j + c * jb], ss[j + d * jb], acc);
+#pragma unroll
+    for (int j = 0; j < PB; j += 32)
+      if (j + lane < rows) acc = fma(ss[j + lane + c * PB], ss[j + lane + d * PB], acc);
     acc = warp_sum(acc);
     if (lane == 0) vals[k] = acc;
   }
   __syncthreads();
-  last_block_reduce(vals, pairs, partial, counter, gpk);
+  if (!last_block_reduce(vals, pairs, partial, counter, gpk) || !zs) return;
+  __syncthreads();
+  direction(gpk, m, zs, lambda_out, flag, 1, sm);
 }
 
-// T[:,a] /= ||t|| ; Q[:,a] = q
-__global__ void finish_component(double* Tcol, int n, const double* scal,
-                                 const double* hq, int a_cur, int m,
-                                 double* Qcol) {
-  const double tn = sqrt(scal[1]);
+// T[:, a] /= ||t_a|| for every component, one pass after the last.
+__global__ void scale_scores(double* T, int n, const double* __restrict__ tnorm2) {
+  const double tn = sqrt(tnorm2[blockIdx.y]);
   const double inv = (tn > 0.0 && isfinite(tn)) ? 1.0 / tn : 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += gridDim.x * blockDim.x)
-    Tcol[i] *= inv;
-  if (blockIdx.x == 0)
-    for (int c = threadIdx.x; c < m; c += blockDim.x) Qcol[c] = hq[a_cur + c];
+  double* col = T + (long)blockIdx.y * n;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) col[i] *= inv;
 }
 
 // Gs[j, k] = (G[j, k] - n mean_j mean_k) / (scale_j scale_k): the Gram of
@@ -410,7 +445,16 @@ __global__ void gram_tstats(const double* __restrict__ r, const double* __restri
   last_block_reduce(vals, 2, partial, counter, scal + 1);
 }
 
-int tail3_block(int m) { return m <= 16 ? 256 : (m <= 32 ? 128 : 64); }
+// The dynamic shared memory any response count needs (one setting: callers on
+// several threads launch these with different counts).
+void configure_small_kernels() {
+  static const bool configured = [] {
+    FPLS_CHECK(cudaFuncSetAttribute(tail3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    FPLS_CHECK(cudaFuncSetAttribute(direction_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    return true;
+  }();
+  (void)configured;
+}
 
 }  // namespace
 
@@ -442,8 +486,9 @@ template <class T>
 void prepare_responses(const T* Y, const int* labels, int n, int m, double* Yc,
                        double* ymean, double* ycsum, int* flag,
                        cudaStream_t stream) {
-  if (labels) center_labels<<<m, TB, 0, stream>>>(labels, n, m, Yc, ymean, ycsum, flag);
-  else center_dense<T><<<m, TB, 0, stream>>>(Y, n, m, Yc, ymean, ycsum, flag);
+  const int threads = std::min(kCenterThreads, std::max(64, (n + 31) / 32 * 32));
+  if (labels) center_labels<<<m, threads, 0, stream>>>(labels, n, m, Yc, ymean, ycsum, flag);
+  else center_dense<T><<<m, threads, 0, stream>>>(Y, n, m, Yc, ymean, ycsum, flag);
   count_launch();
   FPLS_LAUNCH("prepare_responses");
 }
@@ -459,10 +504,8 @@ __global__ void s_times_z(const double* __restrict__ S, int p, int m,
 
 void dominant_direction(const double* S, int p, int m, const double* gpk,
                         double* zs, double* w, Workspace& ws, cudaStream_t s) {
-  // A, B, C, v of the dominant pair (one direction), or A, E of the Jacobi sweeps
-  const size_t smem_dir = (m <= kDominantMaxOrder ? 3 * (size_t)m * m + m + 2 : 2 * (size_t)m * m) * sizeof(double);
-  if (smem_dir > 48 * 1024)
-    FPLS_CHECK(cudaFuncSetAttribute(direction_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dir));
+  const size_t smem_dir = direction_smem(m) * sizeof(double);
+  configure_small_kernels();
   direction_kernel<<<1, jacobi_threads(m), smem_dir, s>>>(gpk, m, zs, nullptr, ws.flag.get(), 1);
   s_times_z<<<std::min<unsigned>(ceil_div(p, TB), 4 * num_sms()), TB, 0, s>>>(S, p, m, zs, w);
   count_launch(2);
@@ -484,7 +527,27 @@ void compute_crossprod(const T* X, int n, int p, long ld, const double* Yc,
   if (model.label_view && m <= kClassMomentsMaxClasses)
     class_moments<T>(X, n, p, ld, model.label_view, m, model.ymean.get(), sum, sumsq, cross,
                      ws.stream_partial, stream);
-  else
+  else if (m >= kGemmCrossResponses && (long)n * p >= (1L << 22)) {
+    // several responses: the moments alone (one pass) and X^T Yc as a DMMA
+    // product (a second one). With the responses in the moments pass the sums
+    // and warp reductions of m columns bound it: 30011 x 10000 BF16, 10
+    // responses 1.35 ms, 0.50 ms in two passes; 4513 x 10000 FP32, 3 responses 0.11
+    // ms in one.
+    column_moments<T>(X, n, p, ld, nullptr, 0, sum, sumsq, nullptr, ws.stream_partial, stream);
+    GemmArgs g;
+    g.M = p;
+    g.N = m;
+    g.K = n;
+    g.A = X;
+    g.lda = ld;
+    g.a_type = gemm_type<T>::value;
+    g.trans_a = true;
+    g.B = Yc;
+    g.ldb = n;
+    g.C = cross;
+    g.ldc = p;
+    gemm_f64(g, stream);
+  } else
     column_moments<T>(X, n, p, ld, Yc, m, sum, sumsq, cross, ws.stream_partial, stream);
   const unsigned gp = std::min<unsigned>(ceil_div(p, TB), 8 * num_sms());
   finish_moments<<<gp, TB, 0, stream>>>(sum, sumsq, cross, ycsum, n, p, m,
@@ -497,15 +560,13 @@ void compute_crossprod(const T* X, int n, int p, long ld, const double* Yc,
 
 void gram_of_columns(double* S, int p, int m, double* gpk, Workspace& ws,
                      cudaStream_t stream) {
-  const int jb3 = tail3_block(m);
-  const unsigned g3 = ceil_div(p, jb3);
-  const size_t smem3 = ((size_t)jb3 * m + (size_t)m * (m + 1) / 2) * sizeof(double);
-  if (smem3 > 48 * 1024)
-    FPLS_CHECK(cudaFuncSetAttribute(tail3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3));
-  tail3_kernel<<<g3, jb3, smem3, stream>>>(nullptr, nullptr, S, p, m, nullptr,
+  const unsigned g3 = ceil_div(p, PB);
+  const size_t smem3 = ((size_t)PB * m + (size_t)m * (m + 1) / 2) * sizeof(double);
+  configure_small_kernels();
+  tail3_kernel<<<g3, TB, smem3, stream>>>(nullptr, nullptr, S, p, m, nullptr,
                                            false, ws.block_partial.get(),
                                            ws.counters.get() + 5, gpk,
-                                           ws.flag.get());
+                                           ws.flag.get(), nullptr, nullptr);
   count_launch();
   FPLS_LAUNCH("gram_of_columns");
 }
@@ -545,16 +606,10 @@ void fit_simpls(const T* X, int n, int p, long ld, const double* Yc,
   unsigned* ctr = ws.counters.get();
   double* part = ws.block_partial.get();
 
-  const int jb3 = tail3_block(m);
-  const unsigned g3 = ceil_div(p, jb3);
-  const size_t smem3 = ((size_t)jb3 * m + (size_t)m * (m + 1) / 2) * sizeof(double);
+  const unsigned g3 = ceil_div(p, PB);
   const unsigned g1 = ceil_div(p, TB);
-  // A, B, C, v of the dominant pair (one direction), or A, E of the Jacobi sweeps
-  const size_t smem_dir = (m <= kDominantMaxOrder ? 3 * (size_t)m * m + m + 2 : 2 * (size_t)m * m) * sizeof(double);
-  if (smem3 > 48 * 1024)
-    FPLS_CHECK(cudaFuncSetAttribute(tail3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3));
-  if (smem_dir > 48 * 1024)
-    FPLS_CHECK(cudaFuncSetAttribute(direction_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dir));
+  const size_t smem_dir = direction_smem(m) * sizeof(double);
+  configure_small_kernels();
 
   // cached-Gram route (FP32 / FP64 storage): Gs = X_s^T X_s once
   gram_route = gram_route && !std::is_same<T, bf16>::value;
@@ -610,10 +665,18 @@ void fit_simpls(const T* X, int n, int p, long ld, const double* Yc,
     Sblk.allocate((size_t)p * m, stream);
   }
   int use = 0, jb = 0;
+  // with one direction a block (and where both fit its last block's shared
+  // memory) the deflation of a component yields the next direction
+  const bool chained = block == 1 && m <= kDominantMaxOrder;
+  const size_t smem3 = std::max((size_t)PB * m + (size_t)m * (m + 1) / 2, chained ? direction_smem(m) : 0) *
+                       sizeof(double);
+  DeviceArray<double> tnorm2(a_max, stream);
   for (int a = 0; a < a_max; ++a) {
     if (jb == use) {
       use = std::min(block, a_max - a);
       jb = 0;
+    }
+    if (jb == 0 && !(chained && a > 0)) {
       direction_kernel<<<1, jacobi_threads(m), smem_dir, stream>>>(gpk, m, use > 1 ? zblk.get() : zs, scal + 3,
                                                     ws.flag.get(), use);
       count_launch();
@@ -638,36 +701,33 @@ void fit_simpls(const T* X, int n, int p, long ld, const double* Yc,
       count_launch();
       FPLS_LAUNCH("gram_tstats");
     } else {
-      xr_product<T>(X, n, p, ld, rt, p, 1, scal, 1, tcol, n, ws.stream_partial, stream);
-      tstats_kernel<<<std::min<unsigned>(ceil_div(n, TB), 2 * num_sms()), TB, 0, stream>>>(
-          tcol, n, part, ctr + 1, scal);
-      count_launch();
-      FPLS_LAUNCH("tstats");
-      xtv_product<T>(X, n, p, ld, tcol, n, 1, praw, p, ws.stream_partial, stream);
+      const XrStats stats{part, ctr + 1, scal + 1};  // sum t^2, sum t
+      xr_product<T>(X, n, p, ld, rt, p, 1, scal, 1, tcol, n, ws.stream_partial, stream, &stats, true);
+      xtv_product<T>(X, n, p, ld, tcol, n, 1, praw, p, ws.stream_partial, stream, true);
     }
-    tail1_kernel<<<g1, TB, (2 * TB + a + m) * sizeof(double), stream>>>(
+    tail1_kernel<<<g3, TB, (2 * PB + a + m) * sizeof(double), stream>>>(
         praw, model.mean.get(), model.scale.get(), scal, r, model.S0.get(),
         model.V.get(), p, m, a, pvec, model.R.get() + (size_t)a * p, part,
-        ctr + 2, hq, ws.flag.get(), gram_route ? loading.get() : nullptr);
-    tail2_kernel<<<g1, TB, (TB + 1 + m) * sizeof(double), stream>>>(
+        ctr + 2, hq, ws.flag.get(), model.Q.get() + (size_t)a * m, tnorm2.get() + a,
+        gram_route ? loading.get() : nullptr);
+    tail2_kernel<<<g3, TB, (PB + 1 + m) * sizeof(double), stream>>>(
         pvec, model.V.get(), hq, S.get(), p, m, a, v, part, ctr + 3, vr);
-    tail3_kernel<<<g3, jb3, smem3, stream>>>(v, vr, S.get(), p, m,
+    tail3_kernel<<<g3, TB, smem3, stream>>>(v, vr, S.get(), p, m,
                                              model.V.get() + (size_t)a * p,
-                                             true, part, ctr + 4, gpk,
-                                             ws.flag.get());
-    if (!gram_route)
-      finish_component<<<std::min<unsigned>(ceil_div(n, TB), 2 * num_sms()), TB, 0, stream>>>(
-          tcol, n, scal, hq, a, m, model.Q.get() + (size_t)a * m);
-    else
-      finish_component<<<1, TB, 0, stream>>>(tcol, 0, scal, hq, a, m,
-                                             model.Q.get() + (size_t)a * m);
-    count_launch(4);
+                                             true, part, ctr + 4, gpk, ws.flag.get(),
+                                             chained && a + 1 < a_max ? zs : nullptr, scal + 3);
+    count_launch(3);
     FPLS_LAUNCH("simpls component");
   }
   model.a = a_max;
   if (gram_route) {
     // training scores T = X_s R (normalised: R holds r / ||t||), one pass
     project_rows<T>(model, X, n, ld, a_max, model.T.get(), n, ws, stream);
+  } else {
+    scale_scores<<<dim3(std::min<unsigned>(ceil_div(n, TB), 4 * num_sms()), a_max), TB, 0, stream>>>(
+        model.T.get(), n, tnorm2.get());
+    count_launch();
+    FPLS_LAUNCH("scale_scores");
   }
 }
 

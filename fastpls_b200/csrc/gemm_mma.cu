@@ -1,7 +1,7 @@
 // FP64 GEMM on the FP64 tensor-core path (DMMA, mma.sync m16n8k8 f64).
 //
 //   C[M x N] = alpha * op(A)[M x K] * op(B)[K x N] (+ beta C), column-major;
-//   op(X) = X or X^T, A and B both FP64 or both FP32, or (A X-like predictors,
+//   op(X) = X or X^T, A and B both FP64 or both FP32, or (A predictors, B
 //   not transposed) A FP32 or BF16 and B FP64; narrow types are widened
 //   exactly as the fragments are loaded, every product and sum is FP64.
 //
@@ -17,8 +17,8 @@
 // which a SIMT kernel took before), zero-filled outside the matrix either
 // way. Shared layouts are padded so that fragment loads are conflict-free:
 // k-major [16][T + pad] for operands contiguous along M or N (row stride
-// 4 mod 16 doubles or 8 mod 32 floats), row-major [T][20] for operands
-// contiguous along K. `lower` restricts the grid to the lower triangle of
+// 4 mod 16 doubles or 8 mod 32 floats), row-major [T][20] ([T][24]
+// for BF16) for operands contiguous along K. `lower` restricts the grid to the lower triangle of
 // square block tiles (symmetric products such as the Gram X X^T).
 //
 // The tile and the K splits come from gemm_plan (gemm.cu): most products of
@@ -43,11 +43,14 @@ template <class T>
 constexpr int row_pad(int t) {
   return t + (sizeof(T) == 8 ? 4 : 8);
 }
-constexpr int LDK = TK + 4;
+template <class T>
+constexpr int row_stride() {  // 16-byte multiples, conflict-free
+  return TK + (sizeof(T) == 2 ? 8 : 4);
+}
 
 template <class T>
 constexpr int slab_elems(bool kcontig, int t) {
-  return kcontig ? t * LDK : TK * row_pad<T>(t);
+  return kcontig ? t * row_stride<T>() : TK * row_pad<T>(t);
 }
 
 // Copies of 16 bytes (or one element) with the bytes past `bytes` zero-filled.
@@ -98,7 +101,7 @@ __device__ __forceinline__ void load_slab(T* s, const T* __restrict__ X, long ld
       if (KCONTIG) {
         const int r = c / (TK / V), k = (c % (TK / V)) * V;
         const int left = r0 + r < rows ? min(V, max(0, kend - (k0 + k))) : 0;
-        cp_async16(s + r * LDK + k, left ? X + (k0 + k) + (long)(r0 + r) * ld : X, left * (int)sizeof(T));
+        cp_async16(s + r * row_stride<T>() + k, left ? X + (k0 + k) + (long)(r0 + r) * ld : X, left * (int)sizeof(T));
       } else {
         const int k = c / (TR / V), r = (c % (TR / V)) * V;
         const int left = k0 + k < kend ? min(V, max(0, rows - (r0 + r))) : 0;
@@ -115,7 +118,7 @@ __device__ __forceinline__ void load_slab(T* s, const T* __restrict__ X, long ld
       if (KCONTIG) {
         const int r = c / TK, k = c % TK;
         const bool ok = r0 + r < rows && k0 + k < kend;
-        cp_async1(s + r * LDK + k, ok ? X + (k0 + k) + (long)(r0 + r) * ld : X, ok);
+        cp_async1(s + r * row_stride<T>() + k, ok ? X + (k0 + k) + (long)(r0 + r) * ld : X, ok);
       } else {
         const int k = c / TR, r = c % TR;
         const bool ok = r0 + r < rows && k0 + k < kend;
@@ -127,7 +130,7 @@ __device__ __forceinline__ void load_slab(T* s, const T* __restrict__ X, long ld
 
 template <class T, bool KCONTIG, int TR>
 __device__ __forceinline__ double slab_at(const T* s, int r, int k) {
-  return as_f64(KCONTIG ? s[r * LDK + k] : s[k * row_pad<T>(TR) + r]);
+  return as_f64(KCONTIG ? s[r * row_stride<T>() + k] : s[k * row_pad<T>(TR) + r]);
 }
 
 // A_T: A stored K x M (contiguous along K); B_T: B stored N x K (contiguous
@@ -302,9 +305,14 @@ void gemm_mma_launch(const GemmArgs& g, const GemmPlan& plan, double* C, long ld
     else by_layout<double>(g, plan, t, stream);
     return;
   }
-  require(g.b_type == GemmType::kF64 && !g.trans_a && !g.trans_b, "FP64 GEMM: unsupported operand types");
-  if (g.a_type == GemmType::kF32) by_tile<float, double, false, false>(g, plan, t, stream);
-  else by_tile<bf16, double, false, false>(g, plan, t, stream);
+  require(g.b_type == GemmType::kF64 && !g.trans_b, "FP64 GEMM: unsupported operand types");
+  if (g.a_type == GemmType::kF32) {
+    if (g.trans_a) by_tile<float, double, true, false>(g, plan, t, stream);
+    else by_tile<float, double, false, false>(g, plan, t, stream);
+  } else {
+    if (g.trans_a) by_tile<bf16, double, true, false>(g, plan, t, stream);
+    else by_tile<bf16, double, false, false>(g, plan, t, stream);
+  }
 }
 
 }  // namespace fpls

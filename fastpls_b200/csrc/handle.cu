@@ -187,6 +187,17 @@ __global__ void variance_finish_kernel(const double* __restrict__ sequential,
   }
 }
 
+// Column stride of the resident training predictors: a multiple of 8 rows, so
+// that every column starts on 16 bytes and the streaming kernels take their
+// vector loads (30011 x 10000 BF16: 153 us a pass with 2-byte loads, 123 to 128 us
+// with 16-byte ones). Only from 8192 rows, where the strided DMA of a column
+// (16 KB and more) runs at the flat copy's rate (54 GB/s; 29 GB/s at 4 KB), and
+// up to 2^21, whose columns still fit a staging slot; the line depends on the
+// rows alone, so that every storage type takes the same kernels.
+long training_ld(int n) {
+  return n >= 8192 && n <= (1 << 21) ? ((long)n + 7) / 8 * 8 : n;
+}
+
 void check_path(const int* prefixes, int count, int a) {
   require(prefixes != nullptr && count >= 1, "invalid resident prediction-path request");
   int previous = 0;
@@ -474,8 +485,9 @@ class TypedHandle final : public ResidentHandle {
     if (cls && q < 2) throw std::invalid_argument("classification requires at least two classes");
     timer_.reset(new FitTimer(stream_));
     FitTimer& timer = *timer_;
-    xtrain_.allocate((size_t)n * p, stream_);
-    upload_h2d(xtrain_.get(), rq_.x, sizeof(T) * n * p, stream_);
+    const long ld = train_ld_ = training_ld(n);
+    xtrain_.allocate((size_t)ld * p, stream_);
+    upload_columns_h2d(xtrain_.get(), ld, rq_.x, n, p, sizeof(T), stream_);
     DeviceArray<TO> y;
     if (cls) {
       model_.labels.allocate(n, stream_);
@@ -498,18 +510,18 @@ class TypedHandle final : public ResidentHandle {
     prepare_responses<TO>(y.get(), model_.labels.get(), n, q, yc.get(),
                          model_.ymean.get(), ycsum.get(), ws_.flag.get(), stream_);
     if (rq_.method == kPlssvd)
-      fit_plssvd<T>(xtrain_.get(), n, p, n, yc.get(), ycsum.get(), q, a, rq_.scaling, model_, ws_, stream_);
+      fit_plssvd<T>(xtrain_.get(), n, p, ld, yc.get(), ycsum.get(), q, a, rq_.scaling, model_, ws_, stream_);
     else if (rq_.method == kOpls)
-      fit_opls<T>(xtrain_.get(), n, p, n, yc.get(), ycsum.get(), q, a, rq_.scaling, rq_.north, model_, ws_,
+      fit_opls<T>(xtrain_.get(), n, p, ld, yc.get(), ycsum.get(), q, a, rq_.scaling, rq_.north, model_, ws_,
                   design_, stream_);
     else if (rq_.method == kKernelPls)
-      fit_kernelpls<T>(xtrain_.get(), n, p, n, yc.get(), ycsum.get(), q, a, rq_.scaling, rq_.kernel,
+      fit_kernelpls<T>(xtrain_.get(), n, p, ld, yc.get(), ycsum.get(), q, a, rq_.scaling, rq_.kernel,
                        rq_.gamma, rq_.degree, rq_.coef0, model_, ws_, design_, stream_);
     else
     {
       used_block_ = simpls_block_size(n, p, q, a, cls, std::is_same<T, float>::value);
       used_gram_ = simpls_gram_route(n, p, a, cls) && !std::is_same<T, bf16>::value;
-      fit_simpls<T>(xtrain_.get(), n, p, n, yc.get(), ycsum.get(), q, a, rq_.scaling, model_, ws_, stream_,
+      fit_simpls<T>(xtrain_.get(), n, p, ld, yc.get(), ycsum.get(), q, a, rq_.scaling, model_, ws_, stream_,
                     used_block_, used_gram_);
     }
   }
@@ -629,11 +641,11 @@ class TypedHandle final : public ResidentHandle {
       DeviceArray<double> zero(fp, stream_), one(fp, stream_);
       zero.zero(stream_);
       fill_ones(one.get(), fp);
-      variance_from<double>(design_.get(), fp, zero.get(), one.get());
+      variance_from<double>(design_.get(), model_.n, fp, zero.get(), one.get());
       return;
     }
     if (!xtrain_) throw std::invalid_argument("resident variance requires the training predictors (call before compaction)");
-    variance_from<T>(xtrain_.get(), model_.p, model_.mean.get(), model_.scale.get());
+    variance_from<T>(xtrain_.get(), train_ld_, model_.p, model_.mean.get(), model_.scale.get());
   }
 
   void fill_ones(double* ptr, int count) {
@@ -646,15 +658,15 @@ class TypedHandle final : public ResidentHandle {
   // mean/scale) and the training scores (variance_loadings/variance_finish,
   // src/cuda_resident_variance.cuh:10-94)
   template <class TX>
-  void variance_from(const TX* X, int p, const double* mean, const double* scale) {
+  void variance_from(const TX* X, long ld, int p, const double* mean, const double* scale) {
     const int n = model_.n, a = model_.a;
     DeviceArray<double> cross((size_t)p * a, stream_), seq((size_t)p * a, stream_);
     DeviceArray<double> gram((size_t)a * a, stream_), tsum(a, stream_);
     DeviceArray<double> mom((size_t)2 * p, stream_);
     loadings_.allocate((size_t)p * a, stream_);
     var_ss_.allocate(a + 1, stream_);
-    xtv_product<TX>(X, n, p, n, model_.T.get(), n, a, cross.get(), p, ws_.stream_partial, stream_);
-    column_moments<TX>(X, n, p, n, nullptr, 0, mom.get(), mom.get() + p, nullptr, ws_.stream_partial, stream_);
+    xtv_product<TX>(X, n, p, ld, model_.T.get(), n, a, cross.get(), p, ws_.stream_partial, stream_);
+    column_moments<TX>(X, n, p, ld, nullptr, 0, mom.get(), mom.get() + p, nullptr, ws_.stream_partial, stream_);
     column_sums_kernel<<<a, 256, 0, stream_>>>(model_.T.get(), n, n, tsum.get());
     count_launch();
     standardize_cross<<<std::min<unsigned>(ceil_div((size_t)p * a, 256), 8 * num_sms()), 256, 0, stream_>>>(
@@ -710,6 +722,7 @@ class TypedHandle final : public ResidentHandle {
   std::unique_ptr<LdaState> lda_;
   std::unique_ptr<PersistentPlan> pending_;
   std::unique_ptr<FitTimer> timer_;
+  long train_ld_ = 0;  // column stride of xtrain_
   int used_block_ = 1;
   bool used_gram_ = false;
 };

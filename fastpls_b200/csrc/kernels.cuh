@@ -7,7 +7,7 @@ namespace fpls {
 
 // ---------------------------------------------------------------- gemm.cu
 // A and B of one type (FP64 or FP32, any transposes), or A FP32 / BF16 and B
-// FP64 (neither transposed).
+// FP64 (B not transposed).
 enum class GemmType { kF64, kF32, kBf16 };
 template <class T> struct gemm_type;
 template <> struct gemm_type<double> { static constexpr GemmType value = GemmType::kF64; };
@@ -68,14 +68,26 @@ void class_moments(const T* X, int n, int p, long ld, const int* labels, int m,
                    const double* prior, double* sum, double* sumsq, double* cross,
                    DeviceArray<double>& scratch, cudaStream_t stream);
 
+// Sum of squares and sum of the (one) column xr_product writes, into out[0]
+// and out[1]; partial: scratch of kXrStatsPartial doubles, counter: a
+// last_block_reduce ticket.
+constexpr int kXrStatsPartial = 4096;
+struct XrStats {
+  double* partial;
+  unsigned* counter;
+  double* out;
+};
+
 // out[i + c*n] = sum_j X[i,j] * R[j + c*ldr] - offset_c   (c < nb)
 // (scores of a scaled/centred X folded into R and offset); offset_c is the sum
 // of offset[c * offset_parts ..] (offset null: 0). FP64 result, nb = 1 or 2
-// (HBM-bound); wider products are FP64-bound and run as GEMMs.
+// (HBM-bound); wider products are FP64-bound and run as GEMMs. finite: X holds
+// no infinity or NaN (finite_f64; one column).
 template <class T>
 void xr_product(const T* X, int n, int p, long ld, const double* R, long ldr,
                 int nb, const double* offset, int offset_parts, double* out, long ldo,
-                DeviceArray<double>& scratch, cudaStream_t stream);
+                DeviceArray<double>& scratch, cudaStream_t stream, const XrStats* stats = nullptr,
+                bool finite = false);
 
 // The one-pass form of xr_product for 3 <= nb <= 16 columns (persistent.cu):
 // X streamed once through the single fit's bulk-copy stages, each stage also
@@ -86,11 +98,12 @@ bool xr_ring(const T* X, int n, int p, long ld, const double* R, long ldr, int n
              const double* offset, int offset_parts, double* out, long ldo, int* flag,
              cudaStream_t stream);
 
-// out[j + c*p] = sum_i X[i,j] * V[i + c*ldv]   (c < nb, FP64)
+// out[j + c*p] = sum_i X[i,j] * V[i + c*ldv]   (c < nb, FP64). finite: X holds
+// no infinity or NaN (finite_f64; used at one column).
 template <class T>
 void xtv_product(const T* X, int n, int p, long ld, const double* V, long ldv,
                  int nb, double* out, long ldo, DeviceArray<double>& scratch,
-                 cudaStream_t stream);
+                 cudaStream_t stream, bool finite = false);
 
 // ---------------------------------------------------------------- misc
 // One-based top-k per row of `count` consecutive column-major (rows x classes)

@@ -104,15 +104,40 @@ __global__ void fold_filter(double* R, int fp, int a, const double* __restrict__
   }
 }
 
-__global__ void row_sqnorms(const double* __restrict__ X, int n, int p, double* out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+// Per-row reductions of a column-major matrix: a block takes 32 rows (a lane
+// each, coalesced) and its 8 warps every eighth column, eight loads in flight;
+// the warps' sums are added in order. One thread per row left 1 to 8 blocks of
+// serial loads at 200 to 2001 rows (150 to 280 us each, 21 to 34 us so).
+constexpr int RR = 32;
+template <class F, class G>
+__device__ __forceinline__ void row_reduce(int rows, int cols, F&& term, G&& store) {
+  __shared__ double part[8][RR];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r0 = blockIdx.x * RR; r0 < rows; r0 += gridDim.x * RR) {
+    const int i = r0 + lane;
     double s = 0.0;
-    for (int j = 0; j < p; ++j) {
-      const double v = X[i + (long)j * n];
-      s = fma(v, v, s);
+    if (i < rows) {
+#pragma unroll 8
+      for (int j = warp; j < cols; j += 8) s = term(s, i, j);
     }
-    out[i] = s;
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && i < rows) {
+      for (int w = 1; w < 8; ++w) s += part[w][lane];
+      store(i, s);
+    }
+    __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(256) row_sqnorms(const double* __restrict__ X, int n, int p, double* out) {
+  row_reduce(
+      n, p,
+      [&](double s, int i, int j) {
+        const double v = X[i + (long)j * n];
+        return fma(v, v, s);
+      },
+      [&](int i, double s) { out[i] = s; });
 }
 
 __global__ void kernel_transform(double* K, int rows, int cols, long ld, int kind,
@@ -151,14 +176,12 @@ __global__ void col_means(const double* __restrict__ K, int rows, int cols, long
   }
 }
 
-// mean of each row (thread per row, coalesced over rows)
-__global__ void row_means_kernel(const double* __restrict__ K, int rows, int cols,
-                                 long ld, double* out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int j = 0; j < cols; ++j) s += K[i + (long)j * ld];
-    out[i] = s / cols;
-  }
+// mean of each row
+__global__ void __launch_bounds__(256)
+    row_means_kernel(const double* __restrict__ K, int rows, int cols, long ld, double* out) {
+  row_reduce(
+      rows, cols, [&](double s, int i, int j) { return s + K[i + (long)j * ld]; },
+      [&](int i, double s) { out[i] = s / cols; });
 }
 
 __global__ void grand_mean(const double* __restrict__ m, int len, double* out) {
@@ -303,7 +326,7 @@ void fit_kernelpls(const T* X, int n, int p, long ld, const double* Yc,
   DeviceArray<double> mean, scale;
   standardized_copy<T>(X, n, p, ld, scaling, mean, scale, model.reference, ws, s);
   model.ref_norms.allocate(n, s);
-  row_sqnorms<<<grid_for(n), TB, 0, s>>>(model.reference.get(), n, p, model.ref_norms.get());
+  row_sqnorms<<<std::min<unsigned>(ceil_div(n, RR), 8 * num_sms()), 256, 0, s>>>(model.reference.get(), n, p, model.ref_norms.get());
   count_launch();
   design.allocate((size_t)n * n, s);
   GemmArgs g;
@@ -353,7 +376,7 @@ void kernel_scores(const DeviceModel& model, const T* X, int rows, long ld, int 
   DeviceArray<double> xs((size_t)rows * p, s), norms(rows, s), kt((size_t)rows * n, s), rm(rows, s);
   standardize_f64<T><<<grid_for((long)rows * p), TB, 0, s>>>(X, rows, p, ld, model.in_mean.get(),
                                                               model.in_scale.get(), xs.get());
-  row_sqnorms<<<grid_for(rows), TB, 0, s>>>(xs.get(), rows, p, norms.get());
+  row_sqnorms<<<std::min<unsigned>(ceil_div(rows, RR), 8 * num_sms()), 256, 0, s>>>(xs.get(), rows, p, norms.get());
   count_launch(2);
   GemmArgs g;
   g.M = rows;
@@ -370,7 +393,7 @@ void kernel_scores(const DeviceModel& model, const T* X, int rows, long ld, int 
   kernel_transform<<<grid_for((long)rows * n), TB, 0, s>>>(kt.get(), rows, n, rows, model.kernel_kind,
                                                             model.gamma, model.degree, model.coef0,
                                                             norms.get(), model.ref_norms.get());
-  row_means_kernel<<<grid_for(rows), TB, 0, s>>>(kt.get(), rows, n, rows, rm.get());
+  row_means_kernel<<<std::min<unsigned>(ceil_div(rows, RR), 8 * num_sms()), 256, 0, s>>>(kt.get(), rows, n, rows, rm.get());
   double_center<<<grid_for((long)rows * n), TB, 0, s>>>(kt.get(), rows, n, rows, rm.get(),
                                                          model.kcol_means.get(), model.kcol_means.get() + n);
   count_launch(3);

@@ -104,7 +104,7 @@ void fastcor_impl(const T* a, const T* b, int rows_a, int cols_a, int rows_b,
   count_launch();
   if (b) {
     db.allocate((size_t)rows_b * cols_b, s);
-    FPLS_CHECK(cudaMemcpyAsync(db.get(), b, sizeof(T) * rows_b * cols_b, cudaMemcpyHostToDevice, s));
+    upload_h2d(db.get(), b, sizeof(T) * rows_b * cols_b, s);
     R.allocate((size_t)units_b * feats, s);
     unit_normalize<T><<<std::min(units_b, 8 * num_sms()), TB, 0, s>>>(db.get(), rows_b, cols_b, byrow,
                                                                         R.get(), units_b, feats);
@@ -648,7 +648,7 @@ void fastsvd_impl(const T* x, int n, int p, int k, int oversample, int power,
     }
   } guard{s};
   DeviceArray<T> xd((size_t)n * p, s);
-  FPLS_CHECK(cudaMemcpyAsync(xd.get(), x, sizeof(T) * n * p, cudaMemcpyHostToDevice, s));
+  upload_h2d(xd.get(), x, sizeof(T) * n * p, s);
   // FP64 copy so every product takes the FP64 tensor path
   DeviceArray<double> X((size_t)n * p, s);
   widen_kernel<T><<<grid_for((long)n * p), TB, 0, s>>>(xd.get(), (long)n * p, X.get());

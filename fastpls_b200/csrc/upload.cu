@@ -191,36 +191,65 @@ bool pinned(const void* p) {
 
 }  // namespace
 
-void upload_h2d(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-  if (bytes == 0) return;
-  Staging* st = nullptr;
-  if (bytes >= kUploadStagedMin && !pinned(src)) {
-    int dev = 0;
-    FPLS_CHECK(cudaGetDevice(&dev));
-    st = StagingPool::get().acquire(dev);
-  }
-  if (!st) {
-    FPLS_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
-    return;
-  }
+namespace {
+
+// Copies src to the device in pieces of `piece` bytes (at most kChunk), each
+// handed to dma(offset, length, host address) on the stream: from the staging
+// slots, or the caller's buffer whole (false) when it is pinned or small.
+template <class F>
+bool staged(const char* h, size_t bytes, size_t piece, cudaStream_t s, F&& dma) {
+  if (bytes < kUploadStagedMin || pinned(h)) return false;
+  int dev = 0;
+  FPLS_CHECK(cudaGetDevice(&dev));
+  Staging* st = StagingPool::get().acquire(dev);
+  if (!st) return false;
   struct Lend {
     Staging* st;
     ~Lend() { StagingPool::get().release(st); }
   } lend{st};
-  char* d = static_cast<char*>(dst);
-  const char* h = static_cast<const char*>(src);
   int k = 0;
-  for (size_t off = 0; off < bytes; off += kChunk, k = (k + 1) % kSlots) {
-    const size_t len = std::min(kChunk, bytes - off);
+  for (size_t off = 0; off < bytes; off += piece, k = (k + 1) % kSlots) {
+    const size_t len = std::min(piece, bytes - off);
     if (st->pending[k]) {
       FPLS_CHECK(cudaEventSynchronize(st->ev[k]));
       st->pending[k] = false;
     }
     CopyPool::get().copy(st->slot[k], h + off, len);
-    FPLS_CHECK(cudaMemcpyAsync(d + off, st->slot[k], len, cudaMemcpyHostToDevice, s));
+    dma(off, len, st->slot[k]);
     FPLS_CHECK(cudaEventRecord(st->ev[k], s));
     st->pending[k] = true;
   }
+  return true;
+}
+
+}  // namespace
+
+void upload_h2d(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  if (bytes == 0) return;
+  char* d = static_cast<char*>(dst);
+  const char* h = static_cast<const char*>(src);
+  if (!staged(h, bytes, kChunk, s, [&](size_t off, size_t len, const char* from) {
+        FPLS_CHECK(cudaMemcpyAsync(d + off, from, len, cudaMemcpyHostToDevice, s));
+      }))
+    FPLS_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+}
+
+void upload_columns_h2d(void* dst, size_t ld, const void* src, size_t rows, size_t cols, size_t elem,
+                        cudaStream_t s) {
+  const size_t row = rows * elem, pitch = ld * elem;
+  if (row == pitch || row > kChunk || cols < 2) {
+    for (size_t c = 0; c < (row == pitch ? 1 : cols); ++c)
+      upload_h2d(static_cast<char*>(dst) + c * pitch, static_cast<const char*>(src) + c * row,
+                 row == pitch ? row * cols : row, s);
+    return;
+  }
+  char* d = static_cast<char*>(dst);
+  const char* h = static_cast<const char*>(src);
+  const auto copy = [&](size_t off, size_t len, const char* from) {
+    FPLS_CHECK(cudaMemcpy2DAsync(d + off / row * pitch, pitch, from, row, row, len / row,
+                                 cudaMemcpyHostToDevice, s));
+  };
+  if (!staged(h, row * cols, kChunk / row * row, s, copy)) copy(0, row * cols, h);
 }
 
 }  // namespace fpls

@@ -17,5 +17,9 @@ namespace fpls {
 // DMA of the last chunks may still be running on s.
 constexpr size_t kUploadStagedMin = size_t(8) << 20;
 void upload_h2d(void* dst, const void* src, size_t bytes, cudaStream_t s);
+// The same for a rows x cols matrix of `elem`-byte elements, columns
+// contiguous in src and `ld` elements apart in dst.
+void upload_columns_h2d(void* dst, size_t ld, const void* src, size_t rows, size_t cols, size_t elem,
+                        cudaStream_t s);
 
 }  // namespace fpls

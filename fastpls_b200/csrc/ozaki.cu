@@ -2,13 +2,13 @@
 // accumulators, TMA-fed shared memory), by the digit split described in
 // ozaki.cuh.
 //
-// Kernel layout (one CTA per 128 x 128 output tile, 320 threads):
-//   warp 0, lane 0   bulk-copy producer: per k-block of 32 bytes, the digit
+// Kernel layout (one CTA per 128 x BN output tile, 320 threads):
+//   warp 0           bulk-copy producer: per k-block of 32 bytes, the digit
 //                    planes 0..ns-1 of the A rows and of the B rows of the
 //                    tile (4 KB each, stored pre-tiled so that they are one
 //                    contiguous run per operand) by two cp.async.bulk copies
 //                    (TMA engine) into a ring of stages.
-//   warp 1, lane 0   MMA issuer: for every diagonal d of the pass and every
+//   warp 1           MMA issuer: for every diagonal d of the pass and every
 //                    digit pair (s, d - s), one tcgen05.mma (K = 32) into the
 //                    TMEM accumulator of d (128 lanes x 128 int32 columns);
 //                    tcgen05.commit releases the stage.
@@ -16,9 +16,18 @@
 //                    = warp % 4, column half = (warp - 2) / 4), exact int32 ->
 //                    FP64, weighted sum over the diagonals, power-of-two row
 //                    scales, one store to C.
+// What bounds it is how fast one thread issues MMAs (128 clocks each at BN =
+// 256, 96 at 192, 64 at 128 when nothing else is in the way) and copies. Both
+// loops are therefore run by their whole warp, with uniform values and only
+// the tcgen05 and bulk-copy instructions under the elected lane: behind
+// `if (lane == 0)` an MMA took about 100 clocks to issue, a commit and its
+// wait 180 more and a copy about 100. 5000 x 2010 x 5000, six digits, BN 192
+// and 256: 1297 and 1370 us, 838 and 952 us with this and the epilogue's
+// reads of C ahead of their use (1068 and 1125 us with the latter alone).
 // TMEM holds four 128-column accumulators, so the S diagonals run in passes
-// of four (S = 6: diagonals 0-3, then 4-5); the epilogue keeps the first
-// pass's 64 partial sums per thread in registers while the second pass runs.
+// of four (S = 6: diagonals 0-3, then 4-5); the epilogue parks the first
+// pass's FP64 sums in TMEM while the second pass runs, or of two (three passes) at BN = 192
+// and 256, each pass after the first adding to C.
 // Every wait on an mbarrier is bounded: on expiry the kernel sets flag = 4,
 // stops issuing, waits (bounded) for its copies and MMAs in flight, frees TMEM
 // and returns.
@@ -136,6 +145,7 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 __device__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort,
                           int* flag, bool ignore_abort = false,
                           long long limit = OZ_WAIT_CYCLES) {
+  if (mbar_test(bar, parity)) return true;
   const long long start = clock64();
   while (!mbar_test(bar, parity)) {
     if (!ignore_abort && *abort) return false;
@@ -146,6 +156,23 @@ __device__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort,
     }
   }
   return true;
+}
+
+// The same wait by a whole warp; every lane gets the same answer.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort,
+                                          int* flag, long long limit = OZ_WAIT_CYCLES) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort, flag, false, limit));
+}
+
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
 }
 
 // One contiguous global -> shared copy on the TMA engine, completing on an
@@ -182,6 +209,22 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t a_desc, uint
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// The same from the low descriptor words (address and leading offset; the high
+// word, stride offset and version, is constant), issued by the elected lane.
+constexpr uint32_t kCoreDescLo = (uint32_t)(128 >> 4) << 16;
+__device__ __forceinline__ void tc_mma_i8_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo,
+                                             uint32_t idesc, uint32_t accumulate, uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "mov.b64 a, {%1, %5};\n\t"
+      "mov.b64 b, {%2, %5};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"((256 >> 4) | (1 << 14)), "r"(elected)
       : "memory");
 }
 
@@ -257,7 +300,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   volatile int* abort = &abort_s;
 
   uint8_t* smem = oz_smem_raw + ((1024 - (smem_u32(oz_smem_raw) & 1023)) & 1023);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   int tm, tn;
   if (args.lower) {
     // blockIdx.x = tm (tm + 1) / 2 + tn, tn <= tm (BN == OZ_BM)
@@ -300,106 +343,113 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   const uint32_t tmem = tmem_base_s;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------------------------------------------------- producer
-      uint32_t it = 0;
-      bool ok = true;
-      for (int pass = 0; pass < npass && ok; ++pass) {
-        const int dhi = min(S - 1, pass * ACC + ACC - 1);
-        const int ns = min(S, dhi + 1);
-        // a stage has S plane slots of A and of B: a pass that needs ns < S
-        // digit planes packs S / ns k-blocks into each stage
-        const int kbs = S / ns;
-        for (int kb = 0; kb < args.kblocks; kb += kbs) {
-          const int nk = min(kbs, args.kblocks - kb);
-          const int st = it % stages;
-          if (args.skip_last && pass + 1 == npass && kb + kbs >= args.kblocks) {
-            ok = false;  // the stage is never issued: the MMA issuer's wait runs out
-            break;
-          }
-          if (it >= (uint32_t)stages &&
-              !mbar_wait(&empty_bar[st], ((it / stages) - 1) & 1, abort, args.flag)) {
-            ok = false;
-            break;
-          }
-          uint8_t* a_dst = smem + st * stage_bytes;
-          uint8_t* b_dst = a_dst + S * OZ_A_PLANE;
-          mbar_expect_tx(&full_bar[st], (uint32_t)(nk * ns) * (OZ_A_PLANE + Shape::B_PLANE));
-          for (int q = 0; q < nk; ++q) {
-            const long slab = (long)(args.kb0 + kb + q) * S;
-            for (int j = 0; j < ns; ++j) {
-              bulk_load(a_dst + (q * ns + j) * OZ_A_PLANE,
-                        digits_a + ((slab + j) * args.rows_pa + (long)tm * OZ_BM) * OZ_BK,
-                        (uint32_t)OZ_A_PLANE, &full_bar[st]);
-              bulk_load(b_dst + (q * ns + j) * Shape::B_PLANE,
-                        digits_b + ((slab + j) * args.rows_pb + (long)tn * BN) * OZ_BK,
-                        (uint32_t)Shape::B_PLANE, &full_bar[st]);
-            }
-          }
-          ++it;
+    // ------------------------------------------------------------ producer
+    const bool elected = elect_one();
+    uint32_t it = 0;
+    bool ok = true;
+    for (int pass = 0; pass < npass && ok; ++pass) {
+      const int dhi = min(S - 1, pass * ACC + ACC - 1);
+      const int ns = min(S, dhi + 1);
+      // a stage has S plane slots of A and of B: a pass that needs ns < S
+      // digit planes packs S / ns k-blocks into each stage
+      const int kbs = S / ns;
+      for (int kb = 0; kb < args.kblocks; kb += kbs) {
+        const int nk = min(kbs, args.kblocks - kb);
+        const int st = it % stages;
+        if (args.skip_last && pass + 1 == npass && kb + kbs >= args.kblocks) {
+          ok = false;  // the stage is never issued: the MMA issuer's wait runs out
+          break;
         }
+        if (it >= (uint32_t)stages &&
+            !warp_wait(&empty_bar[st], ((it / stages) - 1) & 1, abort, args.flag)) {
+          ok = false;
+          break;
+        }
+        uint8_t* a_dst = smem + st * stage_bytes;
+        uint8_t* b_dst = a_dst + S * OZ_A_PLANE;
+        if (elected)
+          mbar_expect_tx(&full_bar[st], (uint32_t)(nk * ns) * (OZ_A_PLANE + Shape::B_PLANE));
+        for (int q = 0; q < nk; ++q) {
+          const long slab = (long)(args.kb0 + kb + q) * S;
+          const int8_t* a_src = digits_a + (slab * args.rows_pa + (long)tm * OZ_BM) * OZ_BK;
+          const int8_t* b_src = digits_b + (slab * args.rows_pb + (long)tn * BN) * OZ_BK;
+          for (int j = 0; j < ns; ++j) {
+            if (elected) {
+              bulk_load(a_dst, a_src, (uint32_t)OZ_A_PLANE, &full_bar[st]);
+              bulk_load(b_dst, b_src, (uint32_t)Shape::B_PLANE, &full_bar[st]);
+            }
+            a_dst += OZ_A_PLANE;
+            b_dst += Shape::B_PLANE;
+            a_src += (long)args.rows_pa * OZ_BK;
+            b_src += (long)args.rows_pb * OZ_BK;
+          }
+        }
+        ++it;
       }
-      // copies still in flight land before the CTA leaves (no-op when every
-      // stage was consumed)
-      for (uint32_t j = it > (uint32_t)stages ? it - stages : 0; j < it; ++j)
-        mbar_wait(&full_bar[j % stages], (j / stages) & 1, abort, args.flag, true);
     }
+    // copies still in flight land before the CTA leaves (no-op when every
+    // stage was consumed)
+    for (uint32_t j = it > (uint32_t)stages ? it - stages : 0; j < it; ++j)
+      mbar_wait(&full_bar[j % stages], (j / stages) & 1, abort, args.flag, true);
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // -------------------------------------------------------- MMA issuer
-      uint32_t it = 0;
-      bool ok = true;
-      for (int pass = 0; pass < npass && ok; ++pass) {
-        const int dlo = pass * ACC, dhi = min(S - 1, dlo + ACC - 1);
-        if (pass > 0) {
-          if (!mbar_wait(&acc_empty, (pass - 1) & 1, abort, args.flag)) break;
-          tc_fence_after();
+    // ---------------------------------------------------------- MMA issuer
+    const uint32_t elected = elect_one();
+    uint32_t it = 0;
+    bool ok = true;
+    for (int pass = 0; pass < npass && ok; ++pass) {
+      const int dlo = pass * ACC, dhi = min(S - 1, dlo + ACC - 1);
+      if (pass > 0) {
+        if (!warp_wait(&acc_empty, (pass - 1) & 1, abort, args.flag)) break;
+        tc_fence_after();
+      }
+      const int ns = min(S, dhi + 1);
+      const int kbs = S / ns;
+      for (int kb = 0; kb < args.kblocks; kb += kbs) {
+        const int nk = min(kbs, args.kblocks - kb);
+        const int st = it % stages;
+        if (!warp_wait(&full_bar[st], (it / stages) & 1, abort, args.flag, args.wait_cycles)) {
+          ok = false;
+          break;
         }
-        const int ns = min(S, dhi + 1);
-        const int kbs = S / ns;
-        for (int kb = 0; kb < args.kblocks; kb += kbs) {
-          const int nk = min(kbs, args.kblocks - kb);
-          const int st = it % stages;
-          if (!mbar_wait(&full_bar[st], (it / stages) & 1, abort, args.flag, false,
-                         args.wait_cycles)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a0 = smem_u32(smem + st * stage_bytes);
-          const uint32_t b0 = a0 + S * OZ_A_PLANE;
-          for (int q = 0; q < nk; ++q) {
-            if (args.interleave) {
-              // digit s outer, diagonal inner: consecutive MMAs write
-              // different accumulators (the int32 sums are exact, so the
-              // order does not change any result)
-              for (int s = 0; s <= dhi; ++s)
-                for (int d = max(dlo, s); d <= dhi; ++d) {
-                  const uint64_t ad = core_desc(a0 + (q * ns + s) * OZ_A_PLANE);
-                  const uint64_t bd = core_desc(b0 + (q * ns + d - s) * Shape::B_PLANE);
-                  const uint32_t acc = (kb + q > 0 || s > 0) ? 1u : 0u;
-                  tc_mma_i8(tmem + (uint32_t)((d - dlo) * BN), ad, bd, Shape::IDESC, acc);
-                }
-            } else {
-              for (int d = dlo; d <= dhi; ++d)
-                for (int s = 0; s <= d; ++s) {
-                  const uint64_t ad = core_desc(a0 + (q * ns + s) * OZ_A_PLANE);
-                  const uint64_t bd = core_desc(b0 + (q * ns + d - s) * Shape::B_PLANE);
-                  const uint32_t acc = (kb + q > 0 || s > 0) ? 1u : 0u;
-                  tc_mma_i8(tmem + (uint32_t)((d - dlo) * BN), ad, bd, Shape::IDESC, acc);
-                }
+        tc_fence_after();
+        constexpr uint32_t A_STEP = OZ_A_PLANE >> 4, B_STEP = Shape::B_PLANE >> 4;
+        const uint32_t a0 = smem_u32(smem + st * stage_bytes);
+        const uint32_t a_lo = (a0 >> 4) | kCoreDescLo;
+        const uint32_t b_lo = ((a0 + S * OZ_A_PLANE) >> 4) | kCoreDescLo;
+        if (args.interleave) {
+          // digit s outer, diagonal inner: consecutive MMAs write different
+          // accumulators (the int32 sums are exact, so the order does not
+          // change any result)
+          for (int q = 0; q < nk; ++q)
+            for (int s = 0; s <= dhi; ++s)
+              for (int d = max(dlo, s); d <= dhi; ++d)
+                tc_mma_i8_lo(tmem + (uint32_t)((d - dlo) * BN), a_lo + (q * ns + s) * A_STEP,
+                             b_lo + (q * ns + d - s) * B_STEP, Shape::IDESC, kb + q > 0 || s > 0,
+                             elected);
+        } else {
+          for (int d = dlo; d <= dhi; ++d) {
+            const uint32_t acc = tmem + (uint32_t)((d - dlo) * BN);
+            for (int q = 0; q < nk; ++q) {
+              uint32_t ad = a_lo + q * ns * A_STEP, bd = b_lo + (q * ns + d) * B_STEP;
+#pragma unroll 1
+              for (int s = 0; s <= d; ++s) {
+                tc_mma_i8_lo(acc, ad, bd, Shape::IDESC, kb + q > 0 || s > 0, elected);
+                ad += A_STEP;
+                bd -= B_STEP;
+              }
             }
           }
-          tc_commit(&empty_bar[st]);
-          ++it;
         }
-        if (ok) tc_commit(&acc_full);
+        if (elected) tc_commit(&empty_bar[st]);
+        ++it;
       }
-      // every MMA issued has completed before TMEM is freed
-      tc_commit(&drain_bar);
-      mbar_wait(&drain_bar, 0, abort, args.flag, true);
+      if (ok && elected) tc_commit(&acc_full);
     }
+    // every MMA issued has completed before TMEM is freed
+    if (elected) tc_commit(&drain_bar);
+    __syncwarp();
+    mbar_wait(&drain_bar, 0, abort, args.flag, true);
     __syncwarp();
   } else {
     // ------------------------------------------------------------ epilogue
@@ -423,18 +473,71 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       const int nd = dhi - dlo + 1;
       const bool last = pass + 1 == npass;
       int ready = 0;
-      if (lane == 0) ready = mbar_wait(&acc_full, pass & 1, abort, args.flag) ? 1 : 0;
+      if (lane == 0) {
+        // a pass takes tens of microseconds: leave the issue slots to the two
+        // issuing warps meanwhile (the bound is that of mbar_wait below)
+        for (int t = 0; t < 65536 && !*abort && !mbar_test(&acc_full, pass & 1); ++t) __nanosleep(256);
+        ready = mbar_wait(&acc_full, pass & 1, abort, args.flag) ? 1 : 0;
+      }
       ready = __shfl_sync(0xffffffffu, ready, 0);
       if (!ready) break;
       tc_fence_after();
       double w[ACC];
 #pragma unroll
       for (int a = 0; a < ACC; ++a) w[a] = a < nd ? kOzWeight[dlo + a] : 0.0;
+      if (!park) {
+        // C is read 16 columns ahead of its update: as one load, add and store
+        // per 4 columns the read-modify-write of the second and third pass was
+        // a chain of L2 latencies, 120 us of 370 us per wave of tiles (width
+        // 256, k = 5000); 35 us so.
+        const bool add = pass > 0 || args.accumulate;
+        constexpr int CH = 16;
+        static_assert(HALF % CH == 0, "column chunks");
+        const double* src = args.C + row + (long)col0 * args.ldc;
+        double next[CH];
+#pragma unroll
+        for (int j = 0; j < CH; ++j)
+          next[j] = add && row_ok && col0 + j < args.N ? __ldcg(src + (long)j * args.ldc) : 0.0;
+        for (int c = 0; c < HALF; c += CH) {
+          double cur[CH];
+#pragma unroll
+          for (int j = 0; j < CH; ++j) cur[j] = next[j];
+          if (c + CH < HALF) {
+#pragma unroll
+            for (int j = 0; j < CH; ++j)
+              next[j] = add && row_ok && col0 + c + CH + j < args.N
+                            ? __ldcg(src + (long)(c + CH + j) * args.ldc)
+                            : 0.0;
+          }
+#pragma unroll
+          for (int g = 0; g < CH; g += 4) {
+            double v[4];
+            pass_sum4<ACC, BN>(mine + (uint32_t)(c + g), nd, w, v);
+            if (row_ok) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const int col = col0 + c + g + j;
+                if (col < args.N) {
+                  const double val = __dmul_rn(__dmul_rn(v[j], sa), args.scale_b[col]);
+                  args.C[row + (long)col * args.ldc] = add ? __dadd_rn(cur[g + j], val) : val;
+                }
+              }
+            }
+          }
+        }
+      } else {
 #pragma unroll 2
-      for (int c = 0; c < HALF / 4; ++c) {
-        const uint32_t at = mine + (uint32_t)(c * 4);
-        double v[4];
-        if (last && park) {
+        for (int c = 0; c < HALF / 4; ++c) {
+          const uint32_t at = mine + (uint32_t)(c * 4);
+          double v[4];
+          if (!last) {
+            pass_sum4<ACC, BN>(at, nd, w, v);
+            tmem_st4(at + 2 * BN, (uint32_t)__double2loint(v[0]), (uint32_t)__double2hiint(v[0]),
+                     (uint32_t)__double2loint(v[1]), (uint32_t)__double2hiint(v[1]));
+            tmem_st4(at + 3 * BN, (uint32_t)__double2loint(v[2]), (uint32_t)__double2hiint(v[2]),
+                     (uint32_t)__double2loint(v[3]), (uint32_t)__double2hiint(v[3]));
+            continue;
+          }
           uint32_t p0[4], p1[4];
           tmem_ld4(at + 2 * BN, p0);
           tmem_ld4(at + 3 * BN, p1);
@@ -453,25 +556,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 const double f = __dmul_rn(__dmul_rn(first[j], sa), sb);
                 const double val = __dmul_rn(__dmul_rn(v[j], sa), sb);
                 *dst = args.accumulate ? __dadd_rn(__dadd_rn(*dst, f), val) : __dadd_rn(f, val);
-              }
-            }
-          }
-        } else {
-          pass_sum4<ACC, BN>(at, nd, w, v);
-          if (!last && park) {
-            tmem_st4(at + 2 * BN, (uint32_t)__double2loint(v[0]), (uint32_t)__double2hiint(v[0]),
-                     (uint32_t)__double2loint(v[1]), (uint32_t)__double2hiint(v[1]));
-            tmem_st4(at + 3 * BN, (uint32_t)__double2loint(v[2]), (uint32_t)__double2hiint(v[2]),
-                     (uint32_t)__double2loint(v[3]), (uint32_t)__double2hiint(v[3]));
-          } else if (row_ok) {
-            const bool add = pass > 0 || args.accumulate;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int col = col0 + c * 4 + j;
-              if (col < args.N) {
-                double* dst = args.C + row + (long)col * args.ldc;
-                const double val = __dmul_rn(__dmul_rn(v[j], sa), args.scale_b[col]);
-                *dst = add ? __dadd_rn(*dst, val) : val;
               }
             }
           }
@@ -968,7 +1052,7 @@ TileChoice pick_tile(int M, int N, int tile_n, int pair) {
     bool pair;
     double step_clk;
   };
-  const Cand cands[] = {{128, false, 177.0}, {192, false, 276.0}, {256, false, 288.0},
+  const Cand cands[] = {{128, false, 106.0}, {192, false, 137.0}, {256, false, 159.0},
                         {192, true, 327.0},  {256, true, 342.0}};
   TileChoice best{128, false};
   double best_cost = -1.0;
@@ -1084,7 +1168,7 @@ int ozaki_wide_tile(int a_rows, int b_rows) {
     const long tiles = (long)ceil_div(a_rows, OZ_BM) * ceil_div(b_rows, bn);
     return (double)((tiles + sms - 1) / sms) * step_clk;
   };
-  return cost(256, 288.0) <= cost(192, 276.0) ? 256 : 192;
+  return cost(256, 159.0) <= cost(192, 137.0) ? 256 : 192;
 }
 
 void ozaki_profile_read(double* ms, double* int8_ops, unsigned long long* launches) {

@@ -46,9 +46,20 @@ namespace fpls {
 namespace {
 
 constexpr int BT = 256;
-// The deflation runs one CTA per instance through dependent phases; 128
-// threads keep every instance of a lane (~670) resident in one wave.
-constexpr int DEFL_BT = 128;
+// The deflation runs one CTA per instance through dependent phases, bound by
+// how many loads are in flight: every thread carries 5 rows through a sweep
+// (10 loads per column of W and KW), its block has as many threads as that
+// takes, up to 512, two of which fill an SM at 64 registers. The rule looks at
+// n only, so an instance's sums do not depend on the group it runs in. Per
+// launch of 2010 instances, n = 5000, q = 3, after 0, 8 and 15 components: 286,
+// 593 and 838 us; one block of 1024 threads per SM 350, 608 and 887; blocks of
+// 256 threads that took a row at a time, eight columns unrolled, 391, 791 and
+// 1145. 700 instances, n = 803, q = 5: 34 us after 0 components,
+// 94 with a Jacobi diagonalisation and a row at a time.
+constexpr int kDeflateMaxThreads = 512;
+constexpr int kDeflateRows = 5;   // rows of a thread in flight
+constexpr int kDeflateDepth = 8;  // loads of a lane in flight in the dots
+
 
 struct InstanceView {
   int n, q, kmax, B;        // rows, responses, max components, perms per fold
@@ -190,32 +201,41 @@ __global__ void initial_gram(InstanceView v, const double* C0, const double* KC0
 
 // zs = z / sqrt(lambda) for the dominant eigenpair of the instance's q x q
 // Gram (packed lower triangle), sign fixed so the largest |z| entry is
-// positive. A, E: 2 q^2 doubles of shared memory.
+// positive. A, E: 2 q^2 doubles of shared memory, D: q^2 + q + 2. The pair
+// comes from repeated squaring, as in the fits (a Jacobi diagonalisation of
+// all q pairs, latency-bound in one warp, was half of a deflation launch of
+// 700 instances at n = 803, q = 5); where the trace or the pair's value is
+// not positive the Gram is diagonalised and its largest eigenvalue decides.
 __device__ void dominant_z(const InstanceView& v, int i, const double* G, int* flag,
-                           double* A, double* E, double* zs) {
+                           double* A, double* E, double* D, double* zs) {
   const int q = v.q;
   const double* g = G + (long)i * q * (q + 1) / 2;
-  for (int c = threadIdx.x; c < q; c += blockDim.x)
-    for (int d = 0; d <= c; ++d) {
-      A[c + d * q] = g[c * (c + 1) / 2 + d];
-      A[d + c * q] = g[c * (c + 1) / 2 + d];
-    }
+  for (int e = threadIdx.x; e < q * q; e += blockDim.x) {
+    const int c = max(e % q, e / q), d = min(e % q, e / q);
+    A[e] = g[c * (c + 1) / 2 + d];
+  }
   __syncthreads();
-  jacobi_eigen(A, E, q);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int best = 0;
+  double* z = D + q * q + 1;  // q + 1
+  double lam = 0.0;
+  int at = 0;
+  if (!dominant_pair(A, E, D, z, q, lam) || !(lam > 0.0)) {
+    __syncthreads();
+    jacobi_eigen(A, E, q);
+    __syncthreads();
     for (int k = 1; k < q; ++k)
-      if (A[k + k * q] > A[best + best * q]) best = k;
-    const double lam = A[best + best * q];
+      if (A[k + k * q] > A[at + at * q]) at = k;
+    lam = A[at + at * q];
+    z = E + at * q;
+  }
+  if (threadIdx.x == 0) {
     const bool ok = lam > 0.0 && isfinite(lam);
     if (!ok) flag_error(flag, 1);
     int arg = 0;
     for (int k = 1; k < q; ++k)
-      if (fabs(E[k + best * q]) > fabs(E[arg + best * q])) arg = k;
-    const double sgn = E[arg + best * q] < 0.0 ? -1.0 : 1.0;
+      if (fabs(z[k]) > fabs(z[arg])) arg = k;
+    const double sgn = z[arg] < 0.0 ? -1.0 : 1.0;
     const double inv = ok ? 1.0 / sqrt(lam) : 0.0;
-    for (int k = 0; k < q; ++k) zs[k] = sgn * E[k + best * q] * inv;
+    for (int k = 0; k < q; ++k) zs[k] = sgn * z[k] * inv;
   }
   __syncthreads();
 }
@@ -269,12 +289,12 @@ __device__ void block_z(const InstanceView& v, int i, const double* G, int* flag
 __device__ void direction_body(const InstanceView& v, int i, const double* G,
                                const double* C, double* U, const double* KC0,
                                double* Y1, int* flag, double* A, double* E,
-                               double* zs, double* scratch) {
+                               double* D, double* zs, double* scratch) {
   const int f = v.inst_fold[i];
   const int n = v.n, q = v.q;
   const int blk = v.blk ? v.blk[i] : 1;
   if (blk > 1) block_z(v, i, G, flag, blk, A, E, zs);
-  else dominant_z(v, i, G, flag, A, E, zs);
+  else dominant_z(v, i, G, flag, A, E, D, zs);
   const double* c = C + (long)i * n * q;
   double* cb = blk > 1 ? v.cblk + (long)i * n * q : nullptr;
   double* u = U + (long)i * n;
@@ -310,7 +330,8 @@ __global__ void direction_batched(InstanceView v, const double* G,
   extern __shared__ double sm[];
   __shared__ double scratch[32];
   __shared__ double zs[kBatchMaxResponses];
-  direction_body(v, blockIdx.x, G, C, U, KC0, Y1, flag, sm, sm + v.q * v.q, zs, scratch);
+  direction_body(v, blockIdx.x, G, C, U, KC0, Y1, flag, sm, sm + v.q * v.q,
+                 sm + 2 * v.q * v.q, zs, scratch);
 }
 
 // Scores from Y1 = K U: centre over training rows, normalise, emit the
@@ -385,6 +406,27 @@ __global__ void scores_batched(InstanceView v, const double* Y1, double* Tm,
   }
 }
 
+// A, E (q^2 each), row (q), h (kmax) and the partial dots, later the scratch of
+// dominant_z.
+inline size_t deflate_shared_bytes(int q, int kmax, int threads) {
+  const size_t qq = (size_t)q * q;
+  const size_t dots = std::max((size_t)kmax + 1 + 4 * (size_t)(threads / 32), qq + q + 2);
+  return (2 * qq + q + kmax + dots) * sizeof(double);
+}
+
+// Sum over the block of one double per thread, fixed order; every thread
+// receives it. One barrier: `part` (a double per warp) is not reused before
+// another one.
+__device__ __forceinline__ double deflate_sum(double v, double* part) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v = warp_sum(v);
+  if (lane == 0) part[warp] = v;
+  __syncthreads();
+  double tot = 0.0;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += part[w];
+  return tot;
+}
+
 // Deflation from Y2 = K t~ and the next direction, per instance:
 //   Kt = P_F Y2_F ; h = KW^T t ; w = t - W h ; Kw = Kt - KW h ;
 //   v = sqrt(w^T Kw) ; row = Kw^T C / v ; C -= (w / v) row ; G -= row row^T ;
@@ -392,84 +434,131 @@ __global__ void scores_batched(InstanceView v, const double* Y1, double* Tm,
 // W and KW hold the columns unnormalised, with the scale 1/v of column k in
 // wscale[k] (applied where the columns are read), so no pass rewrites them;
 // Kw^T C is accumulated in the same sweep that forms w and Kw, and the C
-// update shares its sweep with u = C z. Dynamic shared memory:
-// 2 q^2 + 2 kmax + q doubles. QMAX >= q bounds the per-thread Kw^T C sums.
-template <int QMAX>
-__global__ void deflate_batched(InstanceView v, const double* Y2,
-                                double* Tm, double* W, double* KW, double* wscale,
-                                double* C, double* G, int a, int* flag) {
+// update shares its sweep with u = C z. ONE: the block's rows cover n, so w and
+// u stay in registers between the sweeps. KW is read twice, by columns and by
+// rows.
+template <bool ONE>
+__global__ void __launch_bounds__(kDeflateMaxThreads, 2)
+    deflate_batched(InstanceView v, const double* Y2, double* Tm, double* W, double* KW,
+                    double* wscale, double* C, double* G, int a, int* flag) {
   extern __shared__ double sm[];
-  __shared__ double scratch[32];
-  __shared__ double rowpart[(BT / 32) * kBatchMaxResponses];
+  __shared__ double part_v[32], part_u[32];
+  __shared__ double rowpart[(kDeflateMaxThreads / 32) * kBatchMaxResponses];
   __shared__ double zs[kBatchMaxResponses];
+  constexpr int R = kDeflateRows;
   const int i = blockIdx.x;
   const int f = v.inst_fold[i];
   const int n = v.n, q = v.q, kmax = v.kmax;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   double* A = sm;
   double* E = A + q * q;
-  double* h = E + q * q;      // h_k * wscale_k (kmax)
-  double* hsc = h + kmax;     // scratch for the warp-per-column dots (kmax)
-  double* row = hsc + kmax;   // q
+  double* row = E + q * q;    // q
+  double* h = row + q;        // h_k * wscale_k (kmax)
+  double* dots = h + kmax;    // partial dots; later the scratch of dominant_z
   const double* y = Y2 + (long)i * n;
   double* t = Tm + (long)i * n;
   double* w = W + (long)i * n * kmax;
   double* kw = KW + (long)i * n * kmax;
   const double* ws = wscale + (long)i * kmax;
   double* c = C + (long)i * n * q;
-  double s = 0.0;
-  for (int r = threadIdx.x; r < n; r += blockDim.x)
-    if (v.fold_of_row[r] != f + 1) s += y[r];
-  const double mu = v.center ? block_sum(s, scratch) / v.ntrain[f] : 0.0;
-  // h = KW^T t (warp per column), times the column scales
-  for (int k = warp; k < a; k += warps) {
+  // h = KW^T t and, as column a, the sum of Y2 over the training rows: every
+  // column in `parts` row parts, one warp each, so that few columns still
+  // occupy all warps
+  const int parts = max(1, 4 * warps / (a + 1));
+  const int seg = ((n + parts - 1) / parts + 31) & ~31;
+  for (int e = warp; e < (a + 1) * parts; e += warps) {
+    const int k = e / parts, r0 = (e % parts) * seg + lane, r1 = min(n, (e % parts) * seg + seg);
     double acc = 0.0;
+    if (k < a) {
+      const double* col = kw + (long)k * n;
+      for (int r = r0; r < r1; r += 32 * kDeflateDepth) {
+        double x[kDeflateDepth];
+#pragma unroll
+        for (int j = 0; j < kDeflateDepth; ++j) x[j] = r + 32 * j < r1 ? col[r + 32 * j] : 0.0;
+#pragma unroll
+        for (int j = 0; j < kDeflateDepth; ++j)
+          if (r + 32 * j < r1) acc = fma(x[j], t[r + 32 * j], acc);
+      }
+    } else if (v.center) {
 #pragma unroll 4
-    for (int r = lane; r < n; r += 32) acc = fma(kw[r + (long)k * n], t[r], acc);
+      for (int r = r0; r < r1; r += 32) acc += v.fold_of_row[r] != f + 1 ? y[r] : 0.0;
+    }
     acc = warp_sum(acc);
-    if (lane == 0) hsc[k] = acc;
+    if (lane == 0) dots[e] = acc;
+  }
+  for (int e = threadIdx.x; e < warps * q; e += blockDim.x) rowpart[e] = 0.0;
+  __syncthreads();
+  for (int k = threadIdx.x; k <= a; k += blockDim.x) {
+    double acc = 0.0;
+    for (int e = 0; e < parts; ++e) acc += dots[k * parts + e];
+    if (k < a) h[k] = acc * ws[k] * ws[k];
+    else part_u[0] = v.center ? acc / v.ntrain[f] : 0.0;
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < a; k += blockDim.x) h[k] = hsc[k] * ws[k] * ws[k];
-  __syncthreads();
+  const double mu = part_u[0];
   // w = t - W h, Kw = (Y2 - mu) - KW h (training rows), stored unscaled;
   // w^T Kw and Kw^T C in the same sweep
   double* wa = w + (long)a * n;
   double* kwa = kw + (long)a * n;
   double vv = 0.0;
-  double rc[QMAX];
+  double wr[R];
+  unsigned train;
+  for (int base = threadIdx.x; ONE ? base == (int)threadIdx.x : base - (int)threadIdx.x < n;
+       base += R * blockDim.x) {
+    double kr[R];
+    train = 0u;
 #pragma unroll
-  for (int cc = 0; cc < QMAX; ++cc) rc[cc] = 0.0;
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
-    double wr = 0.0, kr = 0.0;
-    if (v.fold_of_row[r] != f + 1) {
-      wr = t[r];
-      kr = y[r] - mu;
-#pragma unroll 4
-      for (int k = 0; k < a; ++k) {
-        wr = fma(-w[r + (long)k * n], h[k], wr);
-        kr = fma(-kw[r + (long)k * n], h[k], kr);
-      }
-      vv = fma(wr, kr, vv);
-#pragma unroll
-      for (int cc = 0; cc < QMAX; ++cc)
-        if (cc < q) rc[cc] = fma(kr, c[r + (long)cc * n], rc[cc]);
+    for (int j = 0; j < R; ++j) {
+      const int r = base + j * blockDim.x;
+      const bool in = r < n && v.fold_of_row[r] != f + 1;
+      train |= (unsigned)in << j;
+      wr[j] = in ? t[r] : 0.0;
+      kr[j] = in ? y[r] - mu : 0.0;
     }
-    wa[r] = wr;
-    kwa[r] = kr;
+    const double* wk = w + base;
+    const double* kk = kw + base;
+#pragma unroll 1
+    for (int k = 0; k < a; ++k) {
+      double x[R], z[R];
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const bool in = train >> j & 1u;
+        x[j] = in ? __ldcs(wk + j * blockDim.x) : 0.0;
+        z[j] = in ? kk[j * blockDim.x] : 0.0;
+      }
+      const double hk = h[k];
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        wr[j] = fma(-x[j], hk, wr[j]);
+        kr[j] = fma(-z[j], hk, kr[j]);
+      }
+      wk += n;
+      kk += n;
+    }
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int r = base + j * blockDim.x;
+      vv = fma(wr[j], kr[j], vv);
+      if (r < n) {
+        wa[r] = wr[j];
+        kwa[r] = kr[j];
+      }
+    }
+    for (int cc = 0; cc < q; ++cc) {
+      const double* col = c + base + (long)cc * n;
+      double acc = 0.0;
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+        if (train >> j & 1u) acc = fma(kr[j], col[j * blockDim.x], acc);
+      acc = warp_sum(acc);
+      if (lane == 0) rowpart[warp * q + cc] += acc;
+    }
   }
-  vv = block_sum(vv, scratch);
+  vv = deflate_sum(vv, part_v);  // and rowpart is complete
   const double vn = sqrt(vv);
   const bool ok = vn > 0.0 && isfinite(vn);
   if (!ok && threadIdx.x == 0) flag_error(flag, 1);
   const double inv = ok ? 1.0 / vn : 0.0;
-#pragma unroll
-  for (int cc = 0; cc < QMAX; ++cc)
-    if (cc < q) {
-      const double part = warp_sum(rc[cc]);
-      if (lane == 0) rowpart[warp * q + cc] = part;
-    }
-  __syncthreads();
   if (threadIdx.x < q) {
     double tot = 0.0;
     for (int ww = 0; ww < warps; ++ww) tot += rowpart[ww * q + threadIdx.x];
@@ -477,10 +566,12 @@ __global__ void deflate_batched(InstanceView v, const double* Y2,
   }
   if (threadIdx.x == 0) wscale[(long)i * kmax + a] = inv;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  {
     double* g = G + (long)i * q * (q + 1) / 2;
-    for (int cc = 0; cc < q; ++cc)
-      for (int d = 0; d <= cc; ++d) g[cc * (cc + 1) / 2 + d] -= row[cc] * row[d];
+    for (int e = threadIdx.x; e < q * q; e += blockDim.x) {
+      const int cc = e / q, d = e % q;
+      if (d <= cc) g[cc * (cc + 1) / 2 + d] -= row[cc] * row[d];
+    }
   }
   __syncthreads();
   // next direction: the dominant pair of the deflated Gram, or within a
@@ -496,27 +587,61 @@ __global__ void deflate_batched(InstanceView v, const double* Y2,
     if (threadIdx.x < q) zs[threadIdx.x] = v.zblk[(long)i * q * q + (long)(nxt % blk) * q + threadIdx.x];
     __syncthreads();
   } else {
-    dominant_z(v, i, G, flag, A, E, zs);
+    dominant_z(v, i, G, flag, A, E, dots, zs);
   }
   double* cb = blk > 1 ? v.cblk + (long)i * n * q : nullptr;
   // C -= (w / v) row^T and the next direction u = C z (over t~)
   double su = 0.0;
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
-    const double wr = wa[r] * inv;
-    double u = 0.0;
-    for (int cc = 0; cc < q; ++cc) {
-      const double cv = fma(-wr, row[cc], c[r + (long)cc * n]);
-      c[r + (long)cc * n] = cv;
-      if (start) cb[r + (long)cc * n] = cv;
-      u = fma(inside ? cb[r + (long)cc * n] : cv, zs[cc], u);
+  double u[R];
+  for (int base = threadIdx.x; ONE ? base == (int)threadIdx.x : base - (int)threadIdx.x < n;
+       base += R * blockDim.x) {
+    if (!ONE) {
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const int r = base + j * blockDim.x;
+        wr[j] = r < n ? wa[r] : 0.0;
+      }
     }
-    t[r] = u;
-    su += u;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      wr[j] *= inv;
+      u[j] = 0.0;
+    }
+    for (int cc = 0; cc < q; ++cc) {
+      double* col = c + base + (long)cc * n;
+      const double rw = row[cc], zc = zs[cc];
+      double x[R];
+#pragma unroll
+      for (int j = 0; j < R; ++j) x[j] = base + j * (int)blockDim.x < n ? col[j * blockDim.x] : 0.0;
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+        if (base + j * (int)blockDim.x < n) {
+          const double cv = fma(-wr[j], rw, x[j]);
+          col[j * blockDim.x] = cv;
+          double* bl = cb + base + j * blockDim.x + (long)cc * n;
+          if (start) *bl = cv;
+          u[j] = fma(inside ? *bl : cv, zc, u[j]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int r = base + j * blockDim.x;
+      su += u[j];
+      if (r < n && (!ONE || !v.center)) t[r] = u[j];
+    }
   }
   if (v.center) {
-    const double mu_u = block_sum(su, scratch) / v.ntrain[f];
-    for (int r = threadIdx.x; r < n; r += blockDim.x)
-      if (v.fold_of_row[r] != f + 1) t[r] -= mu_u;
+    const double mu_u = deflate_sum(su, part_u) / v.ntrain[f];
+    if (ONE) {
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const int r = threadIdx.x + j * blockDim.x;
+        if (r < n) t[r] = train >> j & 1u ? u[j] - mu_u : u[j];
+      }
+    } else {
+      for (int r = threadIdx.x; r < n; r += blockDim.x)
+        if (v.fold_of_row[r] != f + 1) t[r] -= mu_u;
+    }
   }
 }
 
@@ -1137,8 +1262,14 @@ void BatchedCv<T>::gram_product(const double* rhs, int cols, double* out,
 // here allocates, synchronises or reads back, so it can be captured.
 template <class T>
 void BatchedCv<T>::enqueue_group(int I, int nlanes, int tile_n, cudaStream_t s) {
-  const size_t smem_dir = 2 * (size_t)q * q * sizeof(double);
-  const size_t smem_defl = (2 * (size_t)q * q + 2 * (size_t)kmax + q) * sizeof(double);
+  const size_t smem_dir = (3 * (size_t)q * q + q + 2) * sizeof(double);
+  const int defl_bt = std::min(kDeflateMaxThreads, (int)ceil_div(ceil_div(n, kDeflateRows), 32) * 32);
+  const bool one = defl_bt * kDeflateRows >= n;
+  const size_t smem_defl = deflate_shared_bytes(q, kmax, defl_bt);
+  if (smem_defl > 40 * 1024) {
+    FPLS_CHECK(cudaFuncSetAttribute(deflate_batched<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_defl));
+    FPLS_CHECK(cudaFuncSetAttribute(deflate_batched<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_defl));
+  }
   const size_t nq = (size_t)n * q;
   const int rpt = rows_per_thread(n);
   FPLS_CHECK(cudaEventRecord(ws->fork, s));
@@ -1210,12 +1341,12 @@ void BatchedCv<T>::enqueue_group(int I, int nlanes, int tile_n, cudaStream_t s) 
       double* Ws = ws->Ws.get() + o * kmax;
       double* C = ws->C.get() + o * nq;
       double* G = ws->G.get() + o * q * (q + 1) / 2;
-      if (q <= 4)
-        deflate_batched<4><<<c, DEFL_BT, smem_defl, st>>>(v, Y1, U, Wb, KWb, Ws, C, G, a,
-                                                          ws->flag.get());
+      if (one)
+        deflate_batched<true><<<c, defl_bt, smem_defl, st>>>(v, Y1, U, Wb, KWb, Ws, C, G, a,
+                                                             ws->flag.get());
       else
-        deflate_batched<kBatchMaxResponses><<<c, DEFL_BT, smem_defl, st>>>(
-            v, Y1, U, Wb, KWb, Ws, C, G, a, ws->flag.get());
+        deflate_batched<false><<<c, defl_bt, smem_defl, st>>>(v, Y1, U, Wb, KWb, Ws, C, G, a,
+                                                              ws->flag.get());
       count_launch();
       FPLS_LAUNCH("deflate_batched");
     }

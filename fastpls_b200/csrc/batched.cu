@@ -662,13 +662,13 @@ __device__ __forceinline__ void warp_partials_total(const double* part, int coun
   __syncthreads();
 }
 
-template <int RPT>
-__global__ void __launch_bounds__(BT)
+template <int RPT, int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT)
     scores_rows(InstanceView v, const double* Y1, double* Tm, const double* C0,
                 const double* ymean, double* yhat, int yhat_ld, int a,
                 const int* prefix_slot, int prefix_count, double* sse, int* flag) {
   __shared__ double scratch[32];
-  __shared__ double part[(BT / 32) * kBatchMaxResponses];
+  __shared__ double part[(NT / 32) * kBatchMaxResponses];
   __shared__ double qs[kBatchMaxResponses];
   const int i = blockIdx.x;
   const int f = v.inst_fold[i], b = v.inst_perm[i];
@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(BT)
   double s = 0.0;
 #pragma unroll
   for (int j = 0; j < RPT; ++j) {
-    const int r = threadIdx.x + j * BT;
+    const int r = threadIdx.x + j * NT;
     val[j] = 0.0;
     if (r < n && v.fold_of_row[r] != f + 1) {
       val[j] = y[r];
@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(BT)
   double* ttr = v.ttr ? v.ttr + ((long)i * v.kmax + a) * n : nullptr;
 #pragma unroll
   for (int j = 0; j < RPT; ++j) {
-    const int r = threadIdx.x + j * BT;
+    const int r = threadIdx.x + j * NT;
     val[j] = (train >> j & 1u) ? (val[j] - mu) * inv : 0.0;
     if (r < n) {
       t[r] = val[j];
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(BT)
     double acc = 0.0;
 #pragma unroll
     for (int j = 0; j < RPT; ++j) {
-      const int r = threadIdx.x + j * BT;
+      const int r = threadIdx.x + j * NT;
       if (r < n) acc = fma(c0[r + (long)c * n], val[j], acc);
     }
     acc = warp_sum(acc);
@@ -1006,11 +1006,13 @@ BatchedStats& last_batched_stats() {
 namespace {
 
 // Rows per thread of the register-resident score kernel for n rows (0: too
-// many, use the general kernel).
+// many, use the general kernel): blocks of 256 threads up to 1024 rows, of 512
+// above (2010 instances, n = 5000: 154 us a launch, 230 in blocks of 256 with 20
+// rows; 700 instances, n = 803: 29 and 25).
 int rows_per_thread(int n) {
-  const int need = (n + BT - 1) / BT;
-  for (int r : {8, 16, 20, 24, 32})
-    if (need <= r) return r;
+  if (n <= 1024) return n <= 768 ? 3 : 4;
+  for (int r : {5, 6, 8, 10, 12, 16})
+    if (n <= 512 * r) return r;
   return 0;
 }
 
@@ -1316,16 +1318,19 @@ void BatchedCv<T>::enqueue_group(int I, int nlanes, int tile_n, cudaStream_t s) 
       double* sse = ws->sse.get() + o * prefix_count;
       if (a > 0) gram_product(U, c, Y1, L.rhs, tile_n, st);  // Y1 = K u
       switch (rpt) {
-#define FPLS_SCORES(R)                                                                  \
+#define FPLS_SCORES(R, NT)                                                              \
   case R:                                                                               \
-    scores_rows<R><<<c, BT, 0, st>>>(v, Y1, U, C0, ym, yhat, max_test, a, ws->d_slot.get(), \
+    scores_rows<R, NT><<<c, NT, 0, st>>>(v, Y1, U, C0, ym, yhat, max_test, a, ws->d_slot.get(), \
                                      prefix_count, sse, ws->flag.get());                \
     break;
-        FPLS_SCORES(8)
-        FPLS_SCORES(16)
-        FPLS_SCORES(20)
-        FPLS_SCORES(24)
-        FPLS_SCORES(32)
+        FPLS_SCORES(3, 256)
+        FPLS_SCORES(4, 256)
+        FPLS_SCORES(5, 512)
+        FPLS_SCORES(6, 512)
+        FPLS_SCORES(8, 512)
+        FPLS_SCORES(10, 512)
+        FPLS_SCORES(12, 512)
+        FPLS_SCORES(16, 512)
 #undef FPLS_SCORES
         default:
           scores_batched<<<c, BT, 0, st>>>(v, Y1, U, C0, ym, yhat, max_test, a, ws->d_slot.get(),

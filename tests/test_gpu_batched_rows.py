@@ -1,6 +1,7 @@
 """The batched deflation at the edges of its block shapes: rows of one warp, of
 whole blocks and one past them, the largest single sweep (2560 rows) and the
-first size that takes two, against the oracle."""
+first size that takes two; the score kernel's row and block variants likewise,
+against the oracle."""
 import numpy as np
 import pytest
 
@@ -11,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("q", [1, 3, 9])
-@pytest.mark.parametrize("n", [31, 160, 161, 2560, 2561])
+@pytest.mark.parametrize("n", [31, 160, 161, 769, 1025, 2560, 2561, 5121])
 def test_deflation_row_edges(n, q):
     p = 120
     x, y = W.latent_regression(n, p, q, 4, 0.3, 71, dtype=np.float64)

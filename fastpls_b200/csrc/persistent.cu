@@ -261,6 +261,16 @@ __device__ __forceinline__ bool ring_wait(uint64_t* bar, unsigned parity) {
     if (clock64() - t0 > kBarrierCycles) return false;
   return true;
 }
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void bulk_to_smem(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -376,6 +386,31 @@ __device__ void issue_stage(const Fit& f, const T* X, const Region& g, int st, u
                             uint64_t* bar, const E& extra = E()) {
   const int lane = threadIdx.x & 31;
   const int nc = min(G::kCols, g.cols - st * G::kCols);
+  if (!g.ends && g.offc == 0) {
+    // every segment has the same alignment and length (a leading dimension that
+    // is a multiple of 16 bytes, as uploads of more than 8191 rows have): the
+    // converged warp steps the addresses and one lane issues. Copies issued by a
+    // lane each go out one at a time, about 100 clocks apart: fits of 4512 x
+    // 10000 FP32, 20 components 2475 us, 2397 so; 1504 x 4000 FP64 260 and 254.
+    const Segment sg = segment(f, X, g, g.c0 + st * G::kCols);
+    const unsigned bytes = sg.hi > sg.lo ? (unsigned)(sg.hi - sg.lo) : 0u;
+    const void* xsrc = nullptr;
+    unsigned xbytes = 0;
+    extra(st, xsrc, xbytes);
+    const bool el = elect_one();
+    if (el) ring_expect(bar, bytes * nc + xbytes);
+    unsigned long long src = (unsigned long long)sg.lo;
+    unsigned char* dst = slot + sg.off + ((long)sg.lo - (long)sg.g);
+    const long step = f.ld * (long)sizeof(T);
+#pragma unroll 1
+    for (int k = 0; k < nc; ++k) {
+      if (el && bytes) bulk_to_smem(dst, reinterpret_cast<const void*>(src), bytes, bar);
+      src += step;
+      dst += G::kColStride;
+    }
+    if (el && xbytes) bulk_to_smem(slot + G::kCols * G::kColStride, xsrc, xbytes, bar);
+    return;
+  }
   Segment sg;
   unsigned bytes = 0;
   const void* xsrc = nullptr;

@@ -22,8 +22,9 @@
 // the tcgen05 and bulk-copy instructions under the elected lane: behind
 // `if (lane == 0)` an MMA took about 100 clocks to issue, a commit and its
 // wait 180 more and a copy about 100. 5000 x 2010 x 5000, six digits, BN 192
-// and 256: 1297 and 1370 us, 838 and 952 us with this and the epilogue's
-// reads of C ahead of their use (1068 and 1125 us with the latter alone).
+// and 256: 1297 and 1370 us, 798 and 930 us with this and an epilogue that
+// reads C ahead and TMEM 16 columns at a time (1068 and 1125 us with the reads
+// of C alone).
 // TMEM holds four 128-column accumulators, so the S diagonals run in passes
 // of four (S = 6: diagonals 0-3, then 4-5); the epilogue parks the first
 // pass's FP64 sums in TMEM while the second pass runs, or of two (three passes) at BN = 192
@@ -54,8 +55,8 @@ OzakiWaitTest& ozaki_wait_test() {
 // MMA issue order of the int8 product within a stage: 0 = diagonal-major
 // (default: each diagonal's MMAs back to back into its accumulator), 1 =
 // digit-major (consecutive MMAs alternate between the accumulators).
-// Bit-identical results either way; digit-major measured 14% slower on the
-// benchmark's products (1.37 against 1.59 POP/s). The environment variable
+// Bit-identical results either way, and the same time (5000 x 2010 x 5000:
+// 820 us both). The environment variable
 // FASTPLS_B200_INT8_ORDER (0 or 1) selects the order.
 int ozaki_mma_order() {
   static const int order = [] {
@@ -196,24 +197,9 @@ __device__ __forceinline__ void tc_fence_after() {
 // Shared-memory matrix descriptor: K-major, no swizzle. A plane block holds
 // row groups of 2 k-chunks x 8 x 16-byte core matrices: k-adjacent core
 // matrices 128 bytes apart (leading offset), row groups 256 bytes apart
-// (stride offset); descriptor version 1.
-__device__ __forceinline__ uint64_t core_desc(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(128 >> 4) << 16) |
-         ((uint64_t)(256 >> 4) << 32) | ((uint64_t)1 << 46);
-}
-
-__device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same from the low descriptor words (address and leading offset; the high
-// word, stride offset and version, is constant), issued by the elected lane.
+// (stride offset); descriptor version 1. The low word is the address and the
+// leading offset, the high word (stride offset and version) is constant. Run
+// by a whole warp, issued by its elected lane.
 constexpr uint32_t kCoreDescLo = (uint32_t)(128 >> 4) << 16;
 __device__ __forceinline__ void tc_mma_i8_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo,
                                              uint32_t idesc, uint32_t accumulate, uint32_t elected) {
@@ -265,24 +251,91 @@ __device__ __forceinline__ void tmem_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Weighted sum over the nd accumulators of a pass for 4 columns of this
+template <int COLS>
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[COLS]) {
+  static_assert(COLS == 4 || COLS == 8 || COLS == 16, "columns of one load");
+  if constexpr (COLS == 4) {
+    tmem_ld4(taddr, r);
+  } else if constexpr (COLS == 8) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                   "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+  } else {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+        "%12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+          "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+  }
+}
+
+// Weighted sum over the nd accumulators of a pass for COLS columns of this
 // thread's TMEM lane, smallest weight first (exact int32 -> FP64).
-template <int ACC, int BN>
-__device__ __forceinline__ void pass_sum4(uint32_t addr, int nd, const double (&w)[ACC],
-                                          double (&v)[4]) {
-  uint32_t r[ACC][4];
+template <int ACC, int BN, int COLS>
+__device__ __forceinline__ void pass_sum(uint32_t addr, int nd, const double (&w)[ACC],
+                                         double (&v)[COLS]) {
+  uint32_t r[ACC][COLS];
 #pragma unroll
   for (int a = 0; a < ACC; ++a)
-    if (a < nd) tmem_ld4(addr + (uint32_t)(a * BN), r[a]);
+    if (a < nd) tmem_ld_cols<COLS>(addr + (uint32_t)(a * BN), r[a]);
   tmem_wait_ld();
 #pragma unroll
-  for (int j = 0; j < 4; ++j) v[j] = 0.0;
+  for (int j = 0; j < COLS; ++j) v[j] = 0.0;
 #pragma unroll
   for (int a = ACC - 1; a >= 0; --a)
     if (a < nd) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] = __dadd_rn(v[j], __dmul_rn(w[a], (double)(int)r[a][j]));
+      for (int j = 0; j < COLS; ++j) v[j] = __dadd_rn(v[j], __dmul_rn(w[a], (double)(int)r[a][j]));
     }
+}
+
+// The weighted sums of a pass for this thread's row and BN / 2 columns, stored
+// to C or added to it. C is read 16 columns ahead of its update: as one load,
+// add and store per 4 columns the read-modify-write of the second and third
+// pass was a chain of L2 latencies, 120 us of 370 us per wave of tiles (width
+// 256, k = 5000); 35 us so.
+template <int ACC, int BN>
+__device__ __forceinline__ void store_pass(const OzArgs& args, uint32_t mine, int nd,
+                                           const double (&w)[ACC], int row, int col0, double sa,
+                                           bool add) {
+  constexpr int HALF = BN / 2, CH = 16, G = ACC == 2 ? 16 : 8;
+  static_assert(HALF % CH == 0, "column chunks");
+  const bool row_ok = row < args.M;
+  const double* src = args.C + row + (long)col0 * args.ldc;
+  double next[CH];
+#pragma unroll
+  for (int j = 0; j < CH; ++j)
+    next[j] = add && row_ok && col0 + j < args.N ? __ldcg(src + (long)j * args.ldc) : 0.0;
+  for (int c = 0; c < HALF; c += CH) {
+    double cur[CH];
+#pragma unroll
+    for (int j = 0; j < CH; ++j) cur[j] = next[j];
+    if (c + CH < HALF) {
+#pragma unroll
+      for (int j = 0; j < CH; ++j)
+        next[j] = add && row_ok && col0 + c + CH + j < args.N
+                      ? __ldcg(src + (long)(c + CH + j) * args.ldc)
+                      : 0.0;
+    }
+#pragma unroll
+    for (int g = 0; g < CH; g += G) {
+      double v[G];
+      pass_sum<ACC, BN, G>(mine + (uint32_t)(c + g), nd, w, v);
+      if (row_ok) {
+#pragma unroll
+        for (int j = 0; j < G; ++j) {
+          const int col = col0 + c + g + j;
+          if (col < args.N) {
+            const double val = __dmul_rn(__dmul_rn(v[j], sa), args.scale_b[col]);
+            args.C[row + (long)col * args.ldc] = add ? __dadd_rn(cur[g + j], val) : val;
+          }
+        }
+      }
+    }
+  }
 }
 
 template <int BN>
@@ -486,52 +539,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 #pragma unroll
       for (int a = 0; a < ACC; ++a) w[a] = a < nd ? kOzWeight[dlo + a] : 0.0;
       if (!park) {
-        // C is read 16 columns ahead of its update: as one load, add and store
-        // per 4 columns the read-modify-write of the second and third pass was
-        // a chain of L2 latencies, 120 us of 370 us per wave of tiles (width
-        // 256, k = 5000); 35 us so.
-        const bool add = pass > 0 || args.accumulate;
-        constexpr int CH = 16;
-        static_assert(HALF % CH == 0, "column chunks");
-        const double* src = args.C + row + (long)col0 * args.ldc;
-        double next[CH];
-#pragma unroll
-        for (int j = 0; j < CH; ++j)
-          next[j] = add && row_ok && col0 + j < args.N ? __ldcg(src + (long)j * args.ldc) : 0.0;
-        for (int c = 0; c < HALF; c += CH) {
-          double cur[CH];
-#pragma unroll
-          for (int j = 0; j < CH; ++j) cur[j] = next[j];
-          if (c + CH < HALF) {
-#pragma unroll
-            for (int j = 0; j < CH; ++j)
-              next[j] = add && row_ok && col0 + c + CH + j < args.N
-                            ? __ldcg(src + (long)(c + CH + j) * args.ldc)
-                            : 0.0;
-          }
-#pragma unroll
-          for (int g = 0; g < CH; g += 4) {
-            double v[4];
-            pass_sum4<ACC, BN>(mine + (uint32_t)(c + g), nd, w, v);
-            if (row_ok) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const int col = col0 + c + g + j;
-                if (col < args.N) {
-                  const double val = __dmul_rn(__dmul_rn(v[j], sa), args.scale_b[col]);
-                  args.C[row + (long)col * args.ldc] = add ? __dadd_rn(cur[g + j], val) : val;
-                }
-              }
-            }
-          }
-        }
+        store_pass<ACC, BN>(args, mine, nd, w, row, col0, sa, pass > 0 || args.accumulate);
       } else {
 #pragma unroll 2
         for (int c = 0; c < HALF / 4; ++c) {
           const uint32_t at = mine + (uint32_t)(c * 4);
           double v[4];
           if (!last) {
-            pass_sum4<ACC, BN>(at, nd, w, v);
+            pass_sum<ACC, BN, 4>(at, nd, w, v);
             tmem_st4(at + 2 * BN, (uint32_t)__double2loint(v[0]), (uint32_t)__double2hiint(v[0]),
                      (uint32_t)__double2loint(v[1]), (uint32_t)__double2hiint(v[1]));
             tmem_st4(at + 3 * BN, (uint32_t)__double2loint(v[2]), (uint32_t)__double2hiint(v[2]),
@@ -541,7 +556,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           uint32_t p0[4], p1[4];
           tmem_ld4(at + 2 * BN, p0);
           tmem_ld4(at + 3 * BN, p1);
-          pass_sum4<ACC, BN>(at, nd, w, v);  // waits for all loads of this thread
+          pass_sum<ACC, BN, 4>(at, nd, w, v);  // waits for all loads of this thread
           const double first[4] = {__hiloint2double((int)p0[1], (int)p0[0]),
                                    __hiloint2double((int)p0[3], (int)p0[2]),
                                    __hiloint2double((int)p1[1], (int)p1[0]),
@@ -630,13 +645,17 @@ __device__ __forceinline__ void cluster_sync_all() {
                    : "memory");
 }
 
-__device__ __forceinline__ void tc_mma_i8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                               uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma_i8_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo,
+                                               uint32_t idesc, uint32_t accumulate,
+                                               uint32_t elected) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "mov.b64 a, {%1, %5};\n\t"
+      "mov.b64 b, {%2, %5};\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::i8 [%0], a, b, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"((256 >> 4) | (1 << 14)), "r"(elected)
       : "memory");
 }
 
@@ -683,7 +702,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS, 1)
   volatile int* abort = &abort_s;
 
   uint8_t* smem = oz_smem_raw + ((1024 - (smem_u32(oz_smem_raw) & 1023)) & 1023);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1;
@@ -718,94 +737,116 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS, 1)
   const uint32_t tmem = tmem_base_s;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------------------------------------------------- producer
-      uint32_t it = 0;
-      bool ok = true;
-      const long a_row = (long)tm * 256 + rank * OZ_BM;
-      const long b_row = (long)tn * BN + rank * (BN / 2);
-      for (int pass = 0; pass < npass && ok; ++pass) {
-        const int dhi = min(S - 1, pass * ACC + ACC - 1);
-        const int ns = min(S, dhi + 1);
-        const uint32_t bytes = (uint32_t)ns * (OZ_A_PLANE + B_HALF);
-        for (int kb = 0; kb < args.kblocks; ++kb) {
-          const int st = it % stages;
-          if (it >= (uint32_t)stages &&
-              !mbar_wait(&empty_bar[st], ((it / stages) - 1) & 1, abort, args.flag)) {
-            ok = false;
-            break;
-          }
-          uint8_t* a_dst = smem + st * stage_bytes;
-          uint8_t* b_dst = a_dst + S * OZ_A_PLANE;
-          mbar_expect_tx(&full_bar[st], bytes);
-          const long slab = (long)(args.kb0 + kb) * S;
-          for (int j = 0; j < ns; ++j) {
-            bulk_load(a_dst + j * OZ_A_PLANE, digits_a + ((slab + j) * args.rows_pa + a_row) * OZ_BK,
-                      (uint32_t)OZ_A_PLANE, &full_bar[st]);
-            bulk_load(b_dst + j * B_HALF, digits_b + ((slab + j) * args.rows_pb + b_row) * OZ_BK,
-                      (uint32_t)B_HALF, &full_bar[st]);
-          }
-          ++it;
+    // ------------------------------------------------------------ producer
+    const bool elected = elect_one();
+    uint32_t it = 0;
+    bool ok = true;
+    const long a_row = (long)tm * 256 + rank * OZ_BM;
+    const long b_row = (long)tn * BN + rank * (BN / 2);
+    for (int pass = 0; pass < npass && ok; ++pass) {
+      const int dhi = min(S - 1, pass * ACC + ACC - 1);
+      const int ns = min(S, dhi + 1);
+      const int kbs = S / ns;  // k-blocks packed into a stage, as in the single-CTA kernel
+      for (int kb = 0; kb < args.kblocks; kb += kbs) {
+        const int nk = min(kbs, args.kblocks - kb);
+        const int st = it % stages;
+        if (it >= (uint32_t)stages &&
+            !warp_wait(&empty_bar[st], ((it / stages) - 1) & 1, abort, args.flag)) {
+          ok = false;
+          break;
         }
+        uint8_t* a_dst = smem + st * stage_bytes;
+        uint8_t* b_dst = a_dst + S * OZ_A_PLANE;
+        if (elected) mbar_expect_tx(&full_bar[st], (uint32_t)(nk * ns) * (OZ_A_PLANE + B_HALF));
+        for (int q = 0; q < nk; ++q) {
+          const long slab = (long)(args.kb0 + kb + q) * S;
+          const int8_t* a_src = digits_a + (slab * args.rows_pa + a_row) * OZ_BK;
+          const int8_t* b_src = digits_b + (slab * args.rows_pb + b_row) * OZ_BK;
+          for (int j = 0; j < ns; ++j) {
+            if (elected) {
+              bulk_load(a_dst, a_src, (uint32_t)OZ_A_PLANE, &full_bar[st]);
+              bulk_load(b_dst, b_src, (uint32_t)B_HALF, &full_bar[st]);
+            }
+            a_dst += OZ_A_PLANE;
+            b_dst += B_HALF;
+            a_src += (long)args.rows_pa * OZ_BK;
+            b_src += (long)args.rows_pb * OZ_BK;
+          }
+        }
+        ++it;
       }
-      for (uint32_t j = it > (uint32_t)stages ? it - stages : 0; j < it; ++j)
-        mbar_wait(&full_bar[j % stages], (j / stages) & 1, abort, args.flag, true);
     }
+    for (uint32_t j = it > (uint32_t)stages ? it - stages : 0; j < it; ++j)
+      mbar_wait(&full_bar[j % stages], (j / stages) & 1, abort, args.flag, true);
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    const uint32_t elected = elect_one();
+    uint32_t it = 0;
+    bool ok = true;
+    if (leader) {
       // -------------------------------------------------- MMA issuer (leader)
-      uint32_t it = 0;
-      bool ok = true;
       for (int pass = 0; pass < npass && ok; ++pass) {
         const int dlo = pass * ACC, dhi = min(S - 1, dlo + ACC - 1);
         if (pass > 0) {
-          if (!mbar_wait_cluster(&acc_empty, (pass - 1) & 1, abort, args.flag)) break;
+          if (!__all_sync(0xffffffffu,
+                          mbar_wait_cluster(&acc_empty, (pass - 1) & 1, abort, args.flag)))
+            break;
           tc_fence_after();
         }
-        for (int kb = 0; kb < args.kblocks; ++kb) {
+        const int ns = min(S, dhi + 1);
+        const int kbs = S / ns;
+        for (int kb = 0; kb < args.kblocks; kb += kbs) {
+          const int nk = min(kbs, args.kblocks - kb);
           const int st = it % stages;
           const uint32_t ph = (it / stages) & 1;
-          if (!mbar_wait(&full_bar[st], ph, abort, args.flag) ||
-              !mbar_wait_cluster(&peer_full[st], ph, abort, args.flag)) {
+          if (!__all_sync(0xffffffffu,
+                          mbar_wait(&full_bar[st], ph, abort, args.flag) &&
+                              mbar_wait_cluster(&peer_full[st], ph, abort, args.flag))) {
             ok = false;
             break;
           }
           tc_fence_after();
+          constexpr uint32_t A_STEP = OZ_A_PLANE >> 4, B_STEP = B_HALF >> 4;
           const uint32_t a0 = smem_u32(smem + st * stage_bytes);
-          const uint32_t b0 = a0 + S * OZ_A_PLANE;
-          for (int d = dlo; d <= dhi; ++d)
-            for (int s = 0; s <= d; ++s) {
-              const uint64_t ad = core_desc(a0 + s * OZ_A_PLANE);
-              const uint64_t bd = core_desc(b0 + (d - s) * B_HALF);
-              const uint32_t acc = (kb > 0 || s > 0) ? 1u : 0u;
-              tc_mma_i8_pair(tmem + (uint32_t)((d - dlo) * BN), ad, bd, IDESC, acc);
+          const uint32_t a_lo = (a0 >> 4) | kCoreDescLo;
+          const uint32_t b_lo = ((a0 + S * OZ_A_PLANE) >> 4) | kCoreDescLo;
+          for (int d = dlo; d <= dhi; ++d) {
+            const uint32_t acc = tmem + (uint32_t)((d - dlo) * BN);
+            for (int q = 0; q < nk; ++q) {
+              uint32_t ad = a_lo + q * ns * A_STEP, bd = b_lo + (q * ns + d) * B_STEP;
+#pragma unroll 1
+              for (int s = 0; s <= d; ++s) {
+                tc_mma_i8_pair(acc, ad, bd, IDESC, kb + q > 0 || s > 0, elected);
+                ad += A_STEP;
+                bd -= B_STEP;
+              }
             }
-          tc_commit_pair(&empty_bar[st]);
+          }
+          if (elected) tc_commit_pair(&empty_bar[st]);
           ++it;
         }
-        if (ok) tc_commit_pair(&acc_full);
+        if (ok && elected) tc_commit_pair(&acc_full);
       }
-      tc_commit_pair(&drain_bar);
-      mbar_wait(&drain_bar, 0, abort, args.flag, true);
-    } else if (lane == 0) {
+      if (elected) tc_commit_pair(&drain_bar);
+    } else {
       // ------------------------------------------ relay (second CTA of the pair)
       const uint32_t leader_peer_full = cluster_addr(&peer_full[0], 0);
-      uint32_t it = 0;
-      bool ok = true;
-      for (int pass = 0; pass < npass && ok; ++pass)
-        for (int kb = 0; kb < args.kblocks; ++kb) {
+      for (int pass = 0; pass < npass && ok; ++pass) {
+        const int kbs = S / min(S, pass * ACC + ACC);
+        for (int kb = 0; kb < args.kblocks; kb += kbs) {
           const int st = it % stages;
-          if (!mbar_wait(&full_bar[st], (it / stages) & 1, abort, args.flag)) {
+          if (!warp_wait(&full_bar[st], (it / stages) & 1, abort, args.flag)) {
             ok = false;
             break;
           }
-          mbar_arrive_remote(leader_peer_full + (uint32_t)(st * sizeof(uint64_t)));
+          if (elected) mbar_arrive_remote(leader_peer_full + (uint32_t)(st * sizeof(uint64_t)));
           ++it;
         }
-      // the leader's MMAs write this CTA's TMEM: wait for them before it is freed
-      mbar_wait(&drain_bar, 0, abort, args.flag, true);
+      }
     }
+    // the leader's MMAs write both CTAs' TMEM: they have completed before it is freed
+    __syncwarp();
+    mbar_wait(&drain_bar, 0, abort, args.flag, true);
     __syncwarp();
   } else {
     // ------------------------------------------------------------ epilogue
@@ -813,8 +854,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS, 1)
     const int quarter = warp & 3;
     const int half = (warp - 2) >> 2;
     const int row = tm * 256 + (int)rank * OZ_BM + quarter * 32 + lane;
-    const bool row_ok = row < args.M;
-    const double sa = row_ok ? args.scale_a[row] : 0.0;
+    const double sa = row < args.M ? args.scale_a[row] : 0.0;
     const uint32_t mine = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * HALF);
     const int col0 = tn * BN + half * HALF;
     const uint32_t leader_acc_empty = cluster_addr(&acc_empty, 0);
@@ -823,30 +863,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OZ_THREADS, 1)
       const int nd = dhi - dlo + 1;
       const bool last = pass + 1 == npass;
       int ready = 0;
-      if (lane == 0) ready = mbar_wait_cluster(&acc_full, pass & 1, abort, args.flag) ? 1 : 0;
+      if (lane == 0) {
+        for (int t = 0; t < 65536 && !*abort && !mbar_test_cluster(&acc_full, pass & 1); ++t)
+          __nanosleep(256);
+        ready = mbar_wait_cluster(&acc_full, pass & 1, abort, args.flag) ? 1 : 0;
+      }
       ready = __shfl_sync(0xffffffffu, ready, 0);
       if (!ready) break;
       tc_fence_after();
       double w[ACC];
 #pragma unroll
       for (int a = 0; a < ACC; ++a) w[a] = a < nd ? kOzWeight[dlo + a] : 0.0;
-#pragma unroll 2
-      for (int c = 0; c < HALF / 4; ++c) {
-        double v[4];
-        pass_sum4<ACC, BN>(mine + (uint32_t)(c * 4), nd, w, v);
-        if (row_ok) {
-          const bool add = pass > 0 || args.accumulate;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int col = col0 + c * 4 + j;
-            if (col < args.N) {
-              double* dst = args.C + row + (long)col * args.ldc;
-              const double val = __dmul_rn(__dmul_rn(v[j], sa), args.scale_b[col]);
-              *dst = add ? __dadd_rn(*dst, val) : val;
-            }
-          }
-        }
-      }
+      store_pass<ACC, BN>(args, mine, nd, w, row, col0, sa, pass > 0 || args.accumulate);
       if (!last) {
         tc_fence_before();
         mbar_arrive_remote(leader_acc_empty);
@@ -1053,7 +1081,7 @@ TileChoice pick_tile(int M, int N, int tile_n, int pair) {
     double step_clk;
   };
   const Cand cands[] = {{128, false, 106.0}, {192, false, 137.0}, {256, false, 159.0},
-                        {192, true, 327.0},  {256, true, 342.0}};
+                        {192, true, 172.0},  {256, true, 192.0}};
   TileChoice best{128, false};
   double best_cost = -1.0;
   const int sms = num_sms();

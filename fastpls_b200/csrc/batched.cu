@@ -406,6 +406,10 @@ __global__ void scores_batched(InstanceView v, const double* Y1, double* Tm,
   }
 }
 
+inline int deflate_threads(int n) {
+  return std::min(kDeflateMaxThreads, (int)ceil_div(ceil_div(n, kDeflateRows), 32) * 32);
+}
+
 // A, E (q^2 each), row (q), h (kmax) and the partial dots, later the scratch of
 // dominant_z.
 inline size_t deflate_shared_bytes(int q, int kmax, int threads) {
@@ -1265,13 +1269,9 @@ void BatchedCv<T>::gram_product(const double* rhs, int cols, double* out,
 template <class T>
 void BatchedCv<T>::enqueue_group(int I, int nlanes, int tile_n, cudaStream_t s) {
   const size_t smem_dir = (3 * (size_t)q * q + q + 2) * sizeof(double);
-  const int defl_bt = std::min(kDeflateMaxThreads, (int)ceil_div(ceil_div(n, kDeflateRows), 32) * 32);
+  const int defl_bt = deflate_threads(n);
   const bool one = defl_bt * kDeflateRows >= n;
   const size_t smem_defl = deflate_shared_bytes(q, kmax, defl_bt);
-  if (smem_defl > 40 * 1024) {
-    FPLS_CHECK(cudaFuncSetAttribute(deflate_batched<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_defl));
-    FPLS_CHECK(cudaFuncSetAttribute(deflate_batched<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_defl));
-  }
   const size_t nq = (size_t)n * q;
   const int rpt = rows_per_thread(n);
   FPLS_CHECK(cudaEventRecord(ws->fork, s));
@@ -1673,7 +1673,13 @@ void BatchedCv<T>::run(const T* X_, int n_, int p_, const T* Y_, int q_,
     ws = own.get();
   }
   last_batched_stats() = BatchedStats{};
-  if (digits > 0) ozaki_configure_kernels();  // attributes are not set inside a capture
+  // attributes are not set inside a capture
+  if (digits > 0) ozaki_configure_kernels();
+  const size_t smem_defl = deflate_shared_bytes(q, kmax, deflate_threads(n));
+  if (smem_defl > 40 * 1024) {
+    FPLS_CHECK(cudaFuncSetAttribute(deflate_batched<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_defl));
+    FPLS_CHECK(cudaFuncSetAttribute(deflate_batched<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_defl));
+  }
   const cudaStream_t s = ws->main;
   // the caller's earlier work (input copies) before ours; ours before its later work
   FPLS_CHECK(cudaEventRecord(ws->fork, caller));

@@ -22,7 +22,7 @@
 // the tcgen05 and bulk-copy instructions under the elected lane: behind
 // `if (lane == 0)` an MMA took about 100 clocks to issue, a commit and its
 // wait 180 more and a copy about 100. 5000 x 2010 x 5000, six digits, BN 192
-// and 256: 1297 and 1370 us, 798 and 930 us with this and an epilogue that
+// and 256: 1297 and 1370 us, 766 and 913 us with this and an epilogue that
 // reads C ahead and TMEM 16 columns at a time (1068 and 1125 us with the reads
 // of C alone).
 // TMEM holds four 128-column accumulators, so the S diagonals run in passes
@@ -272,6 +272,13 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[COLS]
   }
 }
 
+// An int32 as FP64, exactly: its bits, offset by 2^31, as the low word of 2^52 + ..
+// (conversions run at a fraction of the rate of this subtraction: 5000 x 2010 x
+// 5000 at width 192, 798 us with them, 766 so).
+__device__ __forceinline__ double int_f64(uint32_t r) {
+  return __dsub_rn(__hiloint2double(0x43300000, (int)(r ^ 0x80000000u)), 4503601774854144.0);
+}
+
 // Weighted sum over the nd accumulators of a pass for COLS columns of this
 // thread's TMEM lane, smallest weight first (exact int32 -> FP64).
 template <int ACC, int BN, int COLS>
@@ -288,7 +295,7 @@ __device__ __forceinline__ void pass_sum(uint32_t addr, int nd, const double (&w
   for (int a = ACC - 1; a >= 0; --a)
     if (a < nd) {
 #pragma unroll
-      for (int j = 0; j < COLS; ++j) v[j] = __dadd_rn(v[j], __dmul_rn(w[a], (double)(int)r[a][j]));
+      for (int j = 0; j < COLS; ++j) v[j] = __dadd_rn(v[j], __dmul_rn(w[a], int_f64(r[a][j])));
     }
 }
 
@@ -900,15 +907,16 @@ __device__ __forceinline__ size_t digit_offset(int row, int k, int s, int slices
          (size_t)(((k & 31) >> 4) * 128 + (row & 7) * 16 + (k & 15));
 }
 // x = 2^e (d0 + d1/254 + ...)/127: scaled by 2^-e (exact) and 127, then
-// rounded to nearest digit by digit.
+// rounded to nearest digit by digit. |v| <= 127, so adding 1.5 2^52 rounds v to
+// the nearest integer (ties to even, as rint) and leaves it in the low word.
 __device__ __forceinline__ void split_value(double x, double inv, int slices, int (&d)[kOzakiMaxSlices]) {
   double v = __dmul_rn(__dmul_rn(x, inv), 127.0);
 #pragma unroll
   for (int s = 0; s < kOzakiMaxSlices; ++s) {
     if (s < slices) {
-      const double r = rint(v);
-      d[s] = (int)r;
-      v = __dmul_rn(__dsub_rn(v, r), 254.0);
+      const double shifted = __dadd_rn(v, 6755399441055744.0);
+      d[s] = __double2loint(shifted);
+      v = __dmul_rn(__dsub_rn(v, __dsub_rn(shifted, 6755399441055744.0)), 254.0);
     } else {
       d[s] = 0;
     }
@@ -928,8 +936,9 @@ __device__ __forceinline__ void row_exponent(double mx, double* inv, double* sca
 }
 
 // Block per row; rows stored contiguously (row r at src + r * ld). Each
-// thread digitises 16 consecutive values per step and stores one 16-byte
-// core-matrix row per digit plane.
+// thread digitises 4 consecutive values per step and stores 4 bytes per digit
+// plane. Bound by L1: with 16 values per thread every load of a warp touched 32
+// lines (2010 rows of 5000: 79 us, 61 so).
 constexpr int OZ_SPLIT_THREADS = 128;
 
 __global__ void __launch_bounds__(OZ_SPLIT_THREADS)
@@ -960,25 +969,24 @@ __global__ void __launch_bounds__(OZ_SPLIT_THREADS)
   row_exponent(mx, &inv, &sc);
   if (threadIdx.x == 0) scale[row] = sc;
   const int rows_p = gridDim.x;
-  for (int c16 = threadIdx.x * 16; c16 < k_p; c16 += OZ_SPLIT_THREADS * 16) {
-    uint32_t pk[kOzakiMaxSlices][4];
+  for (int c4 = threadIdx.x * 4; c4 < k_p; c4 += OZ_SPLIT_THREADS * 4) {
+    uint32_t pk[kOzakiMaxSlices];
 #pragma unroll
-    for (int s = 0; s < kOzakiMaxSlices; ++s) pk[s][0] = pk[s][1] = pk[s][2] = pk[s][3] = 0u;
+    for (int s = 0; s < kOzakiMaxSlices; ++s) pk[s] = 0u;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int c = c16 + j;
+    for (int j = 0; j < 4; ++j) {
+      const int c = c4 + j;
       const double v = (live && c < k) ? x[c] : 0.0;
       int d[kOzakiMaxSlices];
       split_value(isfinite(v) ? v : 0.0, inv, slices, d);
 #pragma unroll
       for (int s = 0; s < kOzakiMaxSlices; ++s)
-        pk[s][j >> 2] |= (uint32_t)(uint8_t)(int8_t)d[s] << (8 * (j & 3));
+        pk[s] |= (uint32_t)(uint8_t)(int8_t)d[s] << (8 * j);
     }
 #pragma unroll
     for (int s = 0; s < kOzakiMaxSlices; ++s)
       if (s < slices)
-        *reinterpret_cast<int4*>(digits + digit_offset(row, c16, s, slices, rows_p)) =
-            make_int4((int)pk[s][0], (int)pk[s][1], (int)pk[s][2], (int)pk[s][3]);
+        *reinterpret_cast<uint32_t*>(digits + digit_offset(row, c4, s, slices, rows_p)) = pk[s];
   }
 }
 
@@ -1080,8 +1088,8 @@ TileChoice pick_tile(int M, int N, int tile_n, int pair) {
     bool pair;
     double step_clk;
   };
-  const Cand cands[] = {{128, false, 106.0}, {192, false, 137.0}, {256, false, 159.0},
-                        {192, true, 172.0},  {256, true, 192.0}};
+  const Cand cands[] = {{128, false, 100.0}, {192, false, 130.0}, {256, false, 155.0},
+                        {192, true, 166.0},  {256, true, 188.0}};
   TileChoice best{128, false};
   double best_cost = -1.0;
   const int sms = num_sms();
@@ -1196,7 +1204,7 @@ int ozaki_wide_tile(int a_rows, int b_rows) {
     const long tiles = (long)ceil_div(a_rows, OZ_BM) * ceil_div(b_rows, bn);
     return (double)((tiles + sms - 1) / sms) * step_clk;
   };
-  return cost(256, 159.0) <= cost(192, 137.0) ? 256 : 192;
+  return cost(256, 155.0) <= cost(192, 130.0) ? 256 : 192;
 }
 
 void ozaki_profile_read(double* ms, double* int8_ops, unsigned long long* launches) {

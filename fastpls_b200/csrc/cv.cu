@@ -103,12 +103,29 @@ struct Fold {
   std::unique_ptr<PersistentPlan> plan;
   DeviceArray<T> Xtr, Xte, Ytr;
   DeviceArray<double> Yte, Yc, ycsum, scores, pred, sums;
-  DeviceArray<int> top;
   const int *pos = nullptr, *lab = nullptr;  // into the batch's arrays
   std::unique_ptr<LdaState> lda;
-  std::vector<int> active, host_labels;
-  std::vector<double> host_pred, host_sums;
-  int bad = 0;
+  std::vector<int> active;
+  std::vector<double> host_pred;
+  size_t at_sums = 0, at_pred = 0, at_labels = 0, at_flag = 0;  // into the batch's Results
+};
+
+// What the host reads of a batch, in one device buffer and one copy: a copy to
+// pageable memory waits for its stream, 15 us each, and three per fold were 460
+// of the 3500 us of a 10-fold call (541 x 1500). Allocated and freed on `main`.
+struct Results {
+  size_t bytes = 0;
+  DeviceArray<unsigned char> dev;
+  std::vector<unsigned char> host;
+  size_t take(size_t b) {
+    const size_t at = bytes;
+    bytes += (b + 255) / 256 * 256;
+    return at;
+  }
+  template <class V>
+  V* on_device(size_t at) { return reinterpret_cast<V*>(dev.get() + at); }
+  template <class V>
+  const V* on_host(size_t at) const { return reinterpret_cast<const V*>(host.data() + at); }
 };
 
 constexpr int kLanes = 4;
@@ -235,6 +252,19 @@ void launch_plans(std::vector<std::unique_ptr<Fold<T>>>& batch, Lanes& lanes) {
   lanes.lanes_after_main();
 }
 
+// The flags of the batch's fits beside its results, then one copy of all of it
+// after every lane.
+template <class T>
+void collect(std::vector<std::unique_ptr<Fold<T>>>& batch, Results& out, Lanes& lanes) {
+  if (batch.empty()) return;
+  for (auto& d : batch)
+    FPLS_CHECK(cudaMemcpyAsync(out.on_device<int>(d->at_flag), d->ws.flag.get(), sizeof(int),
+                               cudaMemcpyDeviceToDevice, d->st));
+  out.host.resize(out.bytes);
+  lanes.main_after_lanes();
+  FPLS_CHECK(cudaMemcpyAsync(out.host.data(), out.dev.get(), out.bytes, cudaMemcpyDeviceToHost, lanes.main));
+}
+
 // Position of every row in the training (k) or held-out (~k) matrix of the
 // fold that holds out `held`, into pos (n).
 void fold_positions(const std::vector<int>& held, int n, int* pos) {
@@ -325,6 +355,7 @@ void cv_regression(int method, const T* predictors, const T* responses,
                                  cudaMemcpyHostToDevice, lanes.main));
       lanes.lanes_after_main();
       std::vector<std::unique_ptr<Fold<T>>> batch;
+      Results out;
       Settle settle{lanes};
       try {
         for (int f = f0; f < f1; ++f) {
@@ -357,50 +388,52 @@ void cv_regression(int method, const T* predictors, const T* responses,
       } catch (...) {
         failed = std::current_exception();  // after the folds before it
       }
+      const bool copy_pred = store_predictions && step == prefix_count;
+      for (auto& fold : batch) {
+        Fold<T>& d = *fold;
+        d.at_sums = out.take(sizeof(double) * 2 * q * prefix_count);
+        if (copy_pred) d.at_pred = out.take(sizeof(double) * d.nte * q * prefix_count);
+        d.at_flag = out.take(sizeof(int));
+      }
+      out.dev.allocate(out.bytes, lanes.main);
       launch_plans(batch, lanes);
+      lanes.lanes_after_main();
       for (auto& fold : batch) {
         Fold<T>& d = *fold;
         d.scores.allocate((size_t)d.nte * maximum_prefix, d.st);
-        d.pred.allocate((size_t)d.nte * q * step, d.st);
-        d.sums.allocate((size_t)2 * q * prefix_count, d.st);
-        d.host_sums.resize((size_t)2 * q * prefix_count);
-        if (store_predictions) d.host_pred.resize((size_t)d.nte * q * prefix_count);
+        if (!copy_pred) d.pred.allocate((size_t)d.nte * q * step, d.st);
+        double* pred = copy_pred ? out.on_device<double>(d.at_pred) : d.pred.get();
+        double* sums = out.on_device<double>(d.at_sums);
+        if (store_predictions && !copy_pred) d.host_pred.resize((size_t)d.nte * q * prefix_count);
         project_rows<T>(d.model, d.Xte.get(), d.nte, d.nte, maximum_prefix, d.scores.get(), d.nte, d.ws, d.st);
         for (int j = 0; j < prefix_count; j += step) {
           const int w = std::min(step, prefix_count - j);
-          predict_prefixes<double>(d.model, d.scores.get(), d.nte, d.nte, prefixes + j, w, d.pred.get(), d.st);
-          fold_sums_kernel<<<dim3(q, w), 256, 0, d.st>>>(d.pred.get(), d.Yte.get(), d.model.ymean.get(), d.nte,
-                                                         q, d.sums.get() + (size_t)2 * q * j);
+          predict_prefixes<double>(d.model, d.scores.get(), d.nte, d.nte, prefixes + j, w, pred, d.st);
+          fold_sums_kernel<<<dim3(q, w), 256, 0, d.st>>>(pred, d.Yte.get(), d.model.ymean.get(), d.nte,
+                                                         q, sums + (size_t)2 * q * j);
           count_launch();
           FPLS_LAUNCH("fold_sums");
           if (store_predictions && step < prefix_count)
-            FPLS_CHECK(cudaMemcpyAsync(d.host_pred.data() + (size_t)j * d.nte * q, d.pred.get(),
+            FPLS_CHECK(cudaMemcpyAsync(d.host_pred.data() + (size_t)j * d.nte * q, pred,
                                        sizeof(double) * d.nte * q * w, cudaMemcpyDeviceToHost, d.st));
         }
       }
-      // copies to pageable memory wait for their stream: after every fold is enqueued
-      for (auto& fold : batch) {
-        Fold<T>& d = *fold;
-        if (store_predictions && step == prefix_count)
-          FPLS_CHECK(cudaMemcpyAsync(d.host_pred.data(), d.pred.get(), sizeof(double) * d.host_pred.size(),
-                                     cudaMemcpyDeviceToHost, d.st));
-        FPLS_CHECK(cudaMemcpyAsync(d.host_sums.data(), d.sums.get(), sizeof(double) * d.host_sums.size(),
-                                   cudaMemcpyDeviceToHost, d.st));
-        FPLS_CHECK(cudaMemcpyAsync(&d.bad, d.ws.flag.get(), sizeof(int), cudaMemcpyDeviceToHost, d.st));
-      }
+      collect(batch, out, lanes);
       lanes.sync();
       for (auto& fold : batch) {
         Fold<T>& d = *fold;
-        if (d.bad)
+        if (*out.on_host<int>(d.at_flag))
           throw std::runtime_error(method == kPlssvd
               ? "resident PLS-SVD failed: invalid labels, decomposition or score Gram"
               : "resident SIMPLS failed: invalid labels, decomposition or component norm");
         const auto& held = fp.test[d.f];
+        const double* sums = out.on_host<double>(d.at_sums);
+        const double* pred = copy_pred ? out.on_host<double>(d.at_pred) : d.host_pred.data();
         for (int j = 0; j < prefix_count; ++j) {
           long double sse = 0.0L, tss = 0.0L;
           for (int c = 0; c < q; ++c) {
-            sse += d.host_sums[(size_t)2 * q * j + 2 * c];
-            tss += d.host_sums[(size_t)2 * q * j + 2 * c + 1];
+            sse += sums[(size_t)2 * q * j + 2 * c];
+            tss += sums[(size_t)2 * q * j + 2 * c + 1];
           }
           metrics[j] += (double)sse;
           fold_ss[j] += (double)tss;
@@ -409,7 +442,7 @@ void cv_regression(int method, const T* predictors, const T* responses,
             for (int c = 0; c < q; ++c)
               for (int i = 0; i < d.nte; ++i)
                 prediction_output[(size_t)j * n * q + (size_t)c * n + held[i]] =
-                    d.host_pred[((size_t)j * q + c) * d.nte + i];
+                    pred[((size_t)j * q + c) * d.nte + i];
         }
         status[d.f] = 1;
       }
@@ -499,6 +532,7 @@ void cv_classification(int method, const T* predictors, const int* labels,
                                  cudaMemcpyHostToDevice, lanes.main));
       lanes.lanes_after_main();
       std::vector<std::unique_ptr<Fold<T>>> batch;
+      Results out;
       Settle settle{lanes};
       try {
         for (int f = f0; f < f1; ++f) {
@@ -551,7 +585,13 @@ void cv_classification(int method, const T* predictors, const int* labels,
       } catch (...) {
         failed = std::current_exception();  // after the folds before it
       }
+      for (auto& fold : batch) {
+        fold->at_labels = out.take(sizeof(int) * (size_t)fold->nte * prefix_count);
+        fold->at_flag = out.take(sizeof(int));
+      }
+      out.dev.allocate(out.bytes, lanes.main);
       launch_plans(batch, lanes);
+      lanes.lanes_after_main();
       std::vector<std::vector<double>> host_scores(batch.size());
       for (size_t b = 0; b < batch.size(); ++b) {
         Fold<T>& d = *batch[b];
@@ -559,14 +599,13 @@ void cv_classification(int method, const T* predictors, const int* labels,
         d.scores.allocate((size_t)d.nte * maximum_prefix, d.st);
         d.pred.allocate((size_t)d.nte * c * step, d.st);
         if (use_lda && store_scores) d.sums.allocate((size_t)d.nte * c * step, d.st);
-        d.top.allocate((size_t)d.nte * step, d.st);
+        int* top = out.on_device<int>(d.at_labels);
         project_rows<T>(d.model, d.Xte.get(), d.nte, d.nte, maximum_prefix, d.scores.get(), d.nte, d.ws, d.st);
         if (use_lda) {
           d.lda.reset(new LdaState());
           d.lda->train(d.model.T.get(), d.ntr, d.ntr, maximum_prefix, d.lab, c, d.model.class_counts,
                        d.ws.flag.get(), d.st);
         }
-        d.host_labels.assign((size_t)d.nte * prefix_count, 0);
         if (store_scores) host_scores[b].resize((size_t)d.nte * c * prefix_count);
         for (int j = 0; j < prefix_count; j += step) {
           const int w = std::min(step, prefix_count - j);
@@ -576,40 +615,33 @@ void cv_classification(int method, const T* predictors, const int* labels,
           if (store_scores || !use_lda)
             predict_prefixes<double>(d.model, d.scores.get(), d.nte, d.nte, prefixes + j, w, resp, d.st);
           if (use_lda) d.lda->discriminants(d.scores.get(), d.nte, d.nte, prefixes + j, w, d.pred.get(), d.st);
-          topk_rows(d.pred.get(), d.nte, c, 1, w, d.top.get(), d.nte, d.st);
-          if (step < prefix_count) {
-            if (store_scores)
-              FPLS_CHECK(cudaMemcpyAsync(host_scores[b].data() + (size_t)j * d.nte * c, resp,
-                                         sizeof(double) * d.nte * c * w, cudaMemcpyDeviceToHost, d.st));
-            FPLS_CHECK(cudaMemcpyAsync(d.host_labels.data() + (size_t)j * d.nte, d.top.get(),
-                                       sizeof(int) * d.nte * w, cudaMemcpyDeviceToHost, d.st));
-          }
+          topk_rows(d.pred.get(), d.nte, c, 1, w, top + (size_t)j * d.nte, d.nte, d.st);
+          if (store_scores && step < prefix_count)
+            FPLS_CHECK(cudaMemcpyAsync(host_scores[b].data() + (size_t)j * d.nte * c, resp,
+                                       sizeof(double) * d.nte * c * w, cudaMemcpyDeviceToHost, d.st));
         }
       }
       // copies to pageable memory wait for their stream: after every fold is enqueued
-      for (size_t b = 0; b < batch.size(); ++b) {
-        Fold<T>& d = *batch[b];
-        if (step == prefix_count) {
-          if (store_scores)
-            FPLS_CHECK(cudaMemcpyAsync(host_scores[b].data(), use_lda ? d.sums.get() : d.pred.get(),
-                                       sizeof(double) * host_scores[b].size(), cudaMemcpyDeviceToHost, d.st));
-          FPLS_CHECK(cudaMemcpyAsync(d.host_labels.data(), d.top.get(), sizeof(int) * d.host_labels.size(),
-                                     cudaMemcpyDeviceToHost, d.st));
+      if (store_scores && step == prefix_count)
+        for (size_t b = 0; b < batch.size(); ++b) {
+          Fold<T>& d = *batch[b];
+          FPLS_CHECK(cudaMemcpyAsync(host_scores[b].data(), use_lda ? d.sums.get() : d.pred.get(),
+                                     sizeof(double) * host_scores[b].size(), cudaMemcpyDeviceToHost, d.st));
         }
-        FPLS_CHECK(cudaMemcpyAsync(&d.bad, d.ws.flag.get(), sizeof(int), cudaMemcpyDeviceToHost, d.st));
-      }
+      collect(batch, out, lanes);
       lanes.sync();
       for (size_t b = 0; b < batch.size(); ++b) {
         Fold<T>& d = *batch[b];
         const int c = d.m;
         const auto& held = fp.test[d.f];
-        if (d.bad)
+        const int* labels_of = out.on_host<int>(d.at_labels);
+        if (*out.on_host<int>(d.at_flag))
           throw std::runtime_error(method == kPlssvd
               ? "resident PLS-SVD failed: invalid labels, decomposition or score Gram"
               : "resident SIMPLS failed: invalid labels, decomposition or component norm");
         for (int j = 0; j < prefix_count; ++j) {
           for (int i = 0; i < d.nte; ++i) {
-            const int predicted = d.active[d.host_labels[(size_t)j * d.nte + i] - 1];
+            const int predicted = d.active[labels_of[(size_t)j * d.nte + i] - 1];
             const int row = held[i];
             if (store_predictions) prediction_output[(size_t)j * n + row] = predicted;
             metrics[j] += predicted == labels[row] ? 1.0 : 0.0;

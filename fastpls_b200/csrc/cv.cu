@@ -112,7 +112,7 @@ struct Fold {
 
 // What the host reads of a batch, in one device buffer and one copy: a copy to
 // pageable memory waits for its stream, 15 us each, and three per fold were 460
-// of the 3500 us of a 10-fold call (541 x 1500). Allocated and freed on `main`.
+// of the 3500 us of a 10-fold call (601 x 1500). Allocated and freed on `main`.
 struct Results {
   size_t bytes = 0;
   DeviceArray<unsigned char> dev;

@@ -228,14 +228,22 @@ __global__ void xtv_finish(const double* __restrict__ partial, int chunks,
   }
 }
 
+// The staged V block: 64 KB, and past it what a chunk of rows rounded up to a
+// multiple of 128 (from one of 64) adds for up to 32 columns. One limit for
+// every call: callers on several threads launch the kernel with different
+// widths.
+constexpr int kXtvMaxColumns = 32;
+constexpr int kXtvStagedBytes = 64 * 1024;
+constexpr int kXtvSharedBytes = kXtvStagedBytes + 64 * kXtvMaxColumns * (int)sizeof(double);
+
 template <class T, int MB, bool MOMENTS, bool FINITE>
 void xtv_launch(const T* X, int n, int p, long ld, const double* V, long ldv,
                 int nb, double* out, long ldo, double* sum, double* sumsq,
                 DeviceArray<double>& scratch, cudaStream_t stream) {
-  // rows per chunk: keep the staged V block <= 64 KB and give the grid
+  // rows per chunk: keep the staged V block near 64 KB and give the grid
   // enough blocks to cover every SM several times.
   int rc = 2048;
-  if (nb > 0) rc = std::min(rc, std::max(128, (64 * 1024 / 8) / nb / 64 * 64));
+  if (nb > 0) rc = std::min(rc, std::max(128, kXtvStagedBytes / (int)sizeof(double) / nb / 64 * 64));
   const int col_tiles = (int)ceil_div(p, 32);
   int chunks = (int)ceil_div(n, rc);
   const int want = 6 * num_sms();
@@ -250,9 +258,10 @@ void xtv_launch(const T* X, int n, int p, long ld, const double* V, long ldv,
   const int slots = nb + (MOMENTS ? 2 : 0);
   scratch.reserve((size_t)chunks * p * slots, stream);
   const size_t smem = (size_t)rc * std::max(nb, 1) * sizeof(double);
+  require(nb <= kXtvMaxColumns && smem <= (size_t)kXtvSharedBytes, "X^T V takes up to 32 columns");
   auto run = [&](auto kernel) {
     if (smem > 48 * 1024)
-      FPLS_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+      FPLS_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kXtvSharedBytes));
     kernel<<<dim3(col_tiles, chunks), kThreads, smem, stream>>>(X, n, p, ld, V, ldv, nb, rc, scratch.get());
   };
   if (pair_aligned(X, ld)) run(xtv_kernel<T, MB, MOMENTS, true, FINITE>);

@@ -136,32 +136,39 @@ void LdaState::train(const double* scores, int n_, long lds, int a_,
 }
 
 void LdaState::finalize(const int* ks, int count, cudaStream_t stream) {
-  LdaJobs jobs;
-  int pending = 0, kmax = 0;
+  // terms on their way: they join `prefixes` once the launch that computes them
+  // is enqueued, so that a call that fails leaves none behind uncomputed
+  std::vector<Prefix> pending;
   auto flush = [&] {
-    if (pending == 0) return;
+    if (pending.empty()) return;
+    LdaJobs jobs;
+    int kmax = 0;
+    for (size_t j = 0; j < pending.size(); ++j) {
+      jobs.k[j] = pending[j].k;
+      jobs.linear[j] = pending[j].linear.get();
+      jobs.constants[j] = pending[j].constants.get();
+      kmax = std::max(kmax, pending[j].k);
+    }
     const size_t smem = (2 * (size_t)kmax * kmax + (size_t)c * kmax) * sizeof(double);
     if (smem > 48 * 1024)
       FPLS_CHECK(cudaFuncSetAttribute(lda_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    lda_finalize<<<pending, 256, smem, stream>>>(gram.get(), a, sums.get(), c, counts_dev.get(), n, jobs, flag);
+    lda_finalize<<<(unsigned)pending.size(), 256, smem, stream>>>(gram.get(), a, sums.get(), c, counts_dev.get(), n,
+                                                                  jobs, flag);
     count_launch();
     FPLS_LAUNCH("lda_finalize");
-    pending = kmax = 0;
+    for (Prefix& pr : pending) prefixes.push_back(std::move(pr));
+    pending.clear();
   };
   for (int j = 0; j < count; ++j) {
     const int k = ks[j];
     require(k >= 1 && k <= a, "invalid LDA prefix");
     if (find(k)) continue;
-    prefixes.emplace_back();
-    Prefix& pr = prefixes.back();
+    Prefix pr;
     pr.k = k;
     pr.linear.allocate((size_t)c * k, stream);
     pr.constants.allocate(c + 1, stream);
-    jobs.k[pending] = k;
-    jobs.linear[pending] = pr.linear.get();
-    jobs.constants[pending] = pr.constants.get();
-    kmax = std::max(kmax, k);
-    if (++pending == kLdaBatch) flush();
+    pending.push_back(std::move(pr));
+    if (pending.size() == kLdaBatch) flush();
   }
   flush();
 }

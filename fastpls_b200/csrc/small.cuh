@@ -98,8 +98,19 @@ __device__ inline int jacobi_eigen(double* A, double* E, int m, int max_sweeps =
             // + e^2) the half-angle forms c^2 = (1 + |d| / h) / 2 and
             // s = sgn(d) e / (2 c h): two reciprocal square roots on the
             // dependent path
-            const double d = A[b + b * m] - A[a + a * m], e = 2.0 * apq;
-            const double rh = rsqrt(fma(d, d, e * e));
+            double d = A[b + b * m] - A[a + a * m], e = 2.0 * apq;
+            double h2 = fma(d, d, e * e);
+            // h^2 outside [2^-900, 2^901): the squares lose bits, vanish or
+            // pass the range. The angle does not depend on a common factor,
+            // so both legs are brought near 1 by a power of two (the test
+            // costs 7 of 314 us at m = 41).
+            if ((unsigned)(__double2hiint(h2) - (123 << 20)) >= (1801u << 20)) {
+              const double f = h2 < 1.0 ? 0x1p600 : 0x1p-600;
+              d *= f;
+              e *= f;
+              h2 = fma(d, d, e * e);
+            }
+            const double rh = rsqrt(h2);
             const double c2 = fma(0.5 * fabs(d), rh, 0.5);
             const double rc = rsqrt(c2);
             c = c2 * rc;

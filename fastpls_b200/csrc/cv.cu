@@ -186,18 +186,18 @@ struct Settle {
   }
 };
 
-// Folds per batch and the persistent CTAs each may take: as many as device
-// memory (a quarter of what is free, at most 8 GB, at least one fold) and the
-// co-resident CTAs hold, in batches of equal size.
+// Folds per batch and the persistent CTAs each may take. The CTA share decides
+// how a fold's sums are split, so it follows from the shape, the number of
+// folds and the device alone: as many folds as 8 GB and the co-resident CTAs
+// hold, in batches of equal size. Free memory (a quarter of it, at least one
+// fold) only lowers how many of them are resident at a time.
 template <class T>
 void batch_shape(int method, const Folds& fp, int n, int p, int m, int a, int folds, size_t pred_bytes,
                  int* per_batch, int* max_ctas) {
-  size_t free_b = 0, total_b = 0;
-  FPLS_CHECK(cudaMemGetInfo(&free_b, &total_b));
   const double one = (double)n * p * sizeof(T) + 8.0 * ((double)p * (2.0 * a + 4.0 * m + 16.0) +
                                                       (double)n * (2.0 * a + 3.0 * m + 8.0)) +
                      (double)pred_bytes + 64.0 * 1024 * 1024;
-  int most = (int)std::max(1.0, std::min((double)folds, std::min(8e9, 0.25 * (double)free_b) / one));
+  int most = (int)std::max(1.0, std::min((double)folds, 8e9 / one));
   *max_ctas = 0;
   if (method != kPlssvd) {
     const int cap = persistent_capacity((int)sizeof(T));
@@ -206,7 +206,10 @@ void batch_shape(int method, const Folds& fp, int n, int p, int m, int a, int fo
     if (cap > 0) *max_ctas = cap / most;
   }
   const int batches = (folds + most - 1) / most;
-  *per_batch = (folds + batches - 1) / batches;
+  size_t free_b = 0, total_b = 0;
+  FPLS_CHECK(cudaMemGetInfo(&free_b, &total_b));
+  const int resident = (int)std::max(1.0, std::min((double)folds, 0.25 * (double)free_b / one));
+  *per_batch = std::min((folds + batches - 1) / batches, resident);
 }
 
 // The fit of a prepared fold on its stream; a SIMPLS fold that takes the

@@ -23,9 +23,10 @@
 //
 // At each barrier every CTA sums the per-CTA partials itself, in one order
 // (deterministic); B2 has nothing to sum and joins only the CTAs of a row
-// block. Chunk sizes depend only on (n, p), so the result does not depend
-// on the storage type of X: BF16 storage gives the same bits as FP32
-// storage of the same values. All arithmetic is FP64.
+// block. Chunk sizes depend only on (n, p) and, where the caller runs
+// several fits in one launch, on the CTA share it gives each, so the result
+// does not depend on the storage type of X: BF16 storage gives the same bits
+// as FP32 storage of the same values. All arithmetic is FP64.
 //
 // Every barrier wait is bounded (about 2 s): on expiry the CTA sets the
 // error flag (5) and returns, so a fit never hangs. Blocks of one fit wait on
@@ -191,7 +192,8 @@ __device__ __forceinline__ void col_range(int p, int C, int c, int& j0, int& j1)
 // slot. The scores pass walks the region's columns forward, the loading
 // pass backward, so the stages read last by one pass are read first by the
 // next while they are still in L2. The partition and the order of every sum
-// depend on (n, p) only: every storage type sums in the same order.
+// depend on (n, p) and the caller's CTA share only: every storage type sums in
+// the same order.
 
 constexpr int kBlockRows = 512;   // largest row block (rows of a segment)
 constexpr int kAuxDoubles = 1024; // rt of the region's columns / t of its rows

@@ -25,6 +25,8 @@ namespace fpls {
 // Returns the number of sweeps used (<= max_sweeps). Matrices of order
 // m <= warp_limit run in the first warp alone.
 constexpr int kJacobiMaxRotations = 64;
+// its static arrays: rotations and the block sum's scratch
+constexpr int kJacobiStaticBytes = kJacobiMaxRotations * 2 * (int)(sizeof(int) + sizeof(double)) + 32 * 8;
 
 // threads for a block that runs jacobi_eigen on an m x m matrix
 inline unsigned jacobi_threads(int m) { return m > 32 ? 512u : m > 16 ? 256u : 64u; }

@@ -165,7 +165,13 @@ __global__ void gaussian_fill(double* out, long count, unsigned long long seed) 
   }
 }
 
-constexpr int kSketchMaxWidth = 120;  // 2 l^2 doubles + l ints <= 227 KB
+// Widest sketch: the small eigenproblem's 2 l^2 doubles and l ints beside the
+// static arrays of its sweeps in one block's shared memory (227 KB).
+constexpr int kSketchMaxWidth = 119;
+constexpr size_t sketch_shared_bytes(int l) { return 2 * (size_t)l * l * sizeof(double) + l * sizeof(int) + 16; }
+static_assert(sketch_shared_bytes(kSketchMaxWidth) + kJacobiStaticBytes <= 227 * 1024 &&
+                  sketch_shared_bytes(kSketchMaxWidth + 1) + kJacobiStaticBytes > 227 * 1024,
+              "the widest sketch that fits one block");
 
 // out = L^-T (upper, l x l) of the Cholesky factor G = L L^T (Q = Y L^-T), one
 // block. Latency-bound: l dependent pivots, one block barrier each. The lower
@@ -403,8 +409,8 @@ class SvdOperator {
   Triplets rsvd(int r, int oversample, int power, unsigned long long seed) {
     const int n = n_, p = p_;
     const int l = std::min(std::min(n, p), r + std::max(oversample, 0));
-    const size_t smem = 2 * (size_t)l * l * sizeof(double) + l * sizeof(int) + 16;
-    require(l <= 256 && smem <= 227 * 1024, "fastsvd sketch too wide for one block");
+    const size_t smem = sketch_shared_bytes(l);
+    require(l <= kSketchMaxWidth, "fastsvd sketch too wide for one block");
     DeviceArray<double> Om((size_t)p * l, s_), Y((size_t)n * l, s_), Z((size_t)p * l, s_);
     gaussian_fill<<<grid_for((long)p * l), TB, 0, s_>>>(Om.get(), (long)p * l, seed);
     count_launch();
@@ -696,8 +702,7 @@ void fastsvd_impl(const T* x, int n, int p, int k, int oversample, int power,
       previous = std::move(accepted);
     }
     // widest sketch whose small l x l eigenproblem fits one block's shared
-    // memory (2 l^2 doubles + l ints): recoveries widen up to it, then add
-    // only power steps
+    // memory: recoveries widen up to it, then add only power steps
     const int widest = std::max(audit_rank, std::min(maximum, kSketchMaxWidth));
     for (int recovery = 0; !certified && recovery < 4; ++recovery) {
       const int current = std::min(widest, audit_rank + std::max(os, 0));

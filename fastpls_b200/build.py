@@ -28,7 +28,7 @@ def build(verbose: bool = False, jobs: int | None = None) -> str:
     objdir = os.path.join(HERE, "_build")
     os.makedirs(objdir, exist_ok=True)
     srcs = sources()
-    deps = srcs + glob.glob(os.path.join(SRC, "*.cuh")) + \
+    deps = srcs + glob.glob(os.path.join(SRC, "*.cuh")) + glob.glob(os.path.join(SRC, "*.hpp")) + \
         [os.path.join(HERE, os.pardir, "include", "fastpls_b200.h")]
     newest = max(os.path.getmtime(p) for p in deps)
     if os.path.exists(LIB) and os.path.getmtime(LIB) >= newest:

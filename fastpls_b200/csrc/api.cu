@@ -12,6 +12,7 @@
 #include "ozaki.cuh"
 #include "cv.cuh"
 #include "handle.cuh"
+#include "once_per_device.hpp"
 #include "persistent.cuh"
 
 #include <atomic>
@@ -41,6 +42,20 @@ void keep_pool_memory() {
   }
   cudaGetLastError();
   configured_device = dev;
+}
+
+void allow_shared_memory(const void* kernel) {
+  static OncePerDevice* once = new OncePerDevice();  // never destroyed: threads may outlive main
+  int dev = 0;
+  FPLS_CHECK(cudaGetDevice(&dev));
+  once->run(kernel, dev, [&] {
+    cudaFuncAttributes attr{};
+    int block = 0;
+    FPLS_CHECK(cudaFuncGetAttributes(&attr, kernel));
+    FPLS_CHECK(cudaDeviceGetAttribute(&block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    FPLS_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    block - (int)attr.sharedSizeBytes));
+  });
 }
 
 cudaStream_t& caller_stream() {

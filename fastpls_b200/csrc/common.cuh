@@ -36,6 +36,12 @@ inline void require(bool ok, const char* message) {
 // repeated fits then reuse mapped pages rather than remapping gigabytes.
 void keep_pool_memory();
 
+// Lets a kernel be launched with as much dynamic shared memory as the current
+// device has for it, set once per kernel and device. A limit set to each
+// call's own size is shared by all threads: a call with a smaller size could
+// lower it between another call's setting and its launch.
+void allow_shared_memory(const void* kernel);
+
 // Device buffer owned by the host object that allocated it (stream-ordered).
 template <class T>
 class DeviceArray {

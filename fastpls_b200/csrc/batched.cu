@@ -1676,10 +1676,8 @@ void BatchedCv<T>::run(const T* X_, int n_, int p_, const T* Y_, int q_,
   // attributes are not set inside a capture
   if (digits > 0) ozaki_configure_kernels();
   const size_t smem_defl = deflate_shared_bytes(q, kmax, deflate_threads(n));
-  if (deflate_shared_bytes(q, kmax, deflate_threads(n)) > 40 * 1024) {
-    allow_shared_memory((const void*)deflate_batched<true>);
-    allow_shared_memory((const void*)deflate_batched<false>);
-  }
+  allow_shared_memory((const void*)deflate_batched<true>);
+  allow_shared_memory((const void*)deflate_batched<false>);
   const cudaStream_t s = ws->main;
   // the caller's earlier work (input copies) before ours; ours before its later work
   FPLS_CHECK(cudaEventRecord(ws->fork, caller));

@@ -39,7 +39,8 @@ void keep_pool_memory();
 // Lets a kernel be launched with as much dynamic shared memory as the current
 // device has for it, set once per kernel and device. A limit set to each
 // call's own size is shared by all threads: a call with a smaller size could
-// lower it between another call's setting and its launch.
+// lower it between another call's setting and its launch. Called whatever the
+// size: the 48 KB a kernel may take without it include its static arrays.
 void allow_shared_memory(const void* kernel);
 
 // Device buffer owned by the host object that allocated it (stream-ordered).

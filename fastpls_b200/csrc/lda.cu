@@ -150,7 +150,7 @@ void LdaState::finalize(const int* ks, int count, cudaStream_t stream) {
       kmax = std::max(kmax, pending[j].k);
     }
     const size_t smem = (2 * (size_t)kmax * kmax + (size_t)c * kmax) * sizeof(double);
-    if (smem > 48 * 1024) allow_shared_memory((const void*)lda_finalize);
+    allow_shared_memory((const void*)lda_finalize);
     lda_finalize<<<(unsigned)pending.size(), 256, smem, stream>>>(gram.get(), a, sums.get(), c, counts_dev.get(), n,
                                                                   jobs, flag);
     count_launch();

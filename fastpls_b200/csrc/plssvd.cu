@@ -115,7 +115,7 @@ void fit_plssvd(const T* X, int n, int p, long ld, const double* Yc,
   model.Q.allocate((size_t)m * k, stream);
   DeviceArray<double> Z((size_t)m * k, stream);
   const size_t smem = 2 * (size_t)m * m * sizeof(double) + m * sizeof(int) + 16;
-  if (smem > 48 * 1024) allow_shared_memory((const void*)small_svd_kernel);
+  allow_shared_memory((const void*)small_svd_kernel);
   small_svd_kernel<<<1, jacobi_threads(m), smem, stream>>>(gpk, m, k, model.sigma.get(),
                                             model.Q.get(), Z.get(), ws.flag.get());
   count_launch();
@@ -153,7 +153,7 @@ void fit_plssvd(const T* X, int n, int p, long ld, const double* Yc,
   gemm_f64(h, stream);
   model.W.allocate((size_t)k * k * m, stream);
   const size_t smem_w = (size_t)k * k * sizeof(double);
-  if (smem_w > 48 * 1024) allow_shared_memory((const void*)plssvd_weights_kernel);
+  allow_shared_memory((const void*)plssvd_weights_kernel);
   plssvd_weights_kernel<<<k, kWeightThreads, smem_w, stream>>>(gram.get(), k, model.sigma.get(), model.Q.get(),
                                                                m, model.W.get(), ws.flag.get());
   count_launch();

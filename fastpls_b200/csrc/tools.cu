@@ -441,7 +441,7 @@ class SvdOperator {
     g.C = G.get();
     g.ldc = l;
     gemm_f64(g, s_);
-    if (smem > 48 * 1024) allow_shared_memory((const void*)small_svd_from_gram);
+    allow_shared_memory((const void*)small_svd_from_gram);
     small_svd_from_gram<<<1, jacobi_threads(l), smem, s_>>>(G.get(), l, r, t.d.get(), Ub.get(), Ud.get());
     count_launch();
     FPLS_LAUNCH("small_svd_from_gram");

@@ -445,15 +445,9 @@ __global__ void gram_tstats(const double* __restrict__ r, const double* __restri
   last_block_reduce(vals, 2, partial, counter, scal + 1);
 }
 
-// The dynamic shared memory any response count needs (one setting: callers on
-// several threads launch these with different counts).
 void configure_small_kernels() {
-  static const bool configured = [] {
-    FPLS_CHECK(cudaFuncSetAttribute(tail3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    FPLS_CHECK(cudaFuncSetAttribute(direction_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    return true;
-  }();
-  (void)configured;
+  allow_shared_memory((const void*)tail3_kernel);
+  allow_shared_memory((const void*)direction_kernel);
 }
 
 }  // namespace

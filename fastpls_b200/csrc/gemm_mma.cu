@@ -257,12 +257,7 @@ template <class TA, class TB, bool A_T, bool B_T, int TM, int TN>
 void launch(const GemmArgs& g, const GemmPlan& plan, const Target& t, cudaStream_t stream) {
   constexpr size_t smem = (size_t)STAGES * (slab_elems<TA>(A_T, TM) * sizeof(TA) +
                                             slab_elems<TB>(!B_T, TN) * sizeof(TB));
-  static const bool configured = [] {
-    FPLS_CHECK(cudaFuncSetAttribute(dgemm_mma<TA, TB, A_T, B_T, TM, TN>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return true;
-  }();
-  (void)configured;
+  allow_shared_memory((const void*)dgemm_mma<TA, TB, A_T, B_T, TM, TN>);
   const int kps = ((g.K + plan.splits - 1) / plan.splits + TK - 1) / TK * TK;
   const unsigned tm = ceil_div(g.M, TM), tn = ceil_div(g.N, TN);
   const dim3 grid = g.lower ? dim3(tm * (tm + 1) / 2, 1, plan.splits) : dim3(tn, tm, plan.splits);

@@ -1108,13 +1108,8 @@ TileChoice pick_tile(int M, int N, int tile_n, int pair) {
 }
 
 template <int BN>
-bool configure_gemm() {
-  static const bool configured = [] {
-    FPLS_CHECK(cudaFuncSetAttribute(ozaki_gemm_kernel<BN>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_DATA + 1024));
-    return true;
-  }();
-  return configured;
+void configure_gemm() {
+  allow_shared_memory((const void*)ozaki_gemm_kernel<BN>);
 }
 
 template <int BN>
@@ -1160,12 +1155,7 @@ void launch_gemm_pair(const OzakiOperand& a, const OzakiOperand& b, OzArgs args,
   args.stages = std::min(OZ_MAX_STAGES, OZ_DATA / stage_bytes);
   require(args.stages >= 2, "int8 split product: stages do not fit shared memory");
   const size_t smem = (size_t)args.stages * stage_bytes + 1024;
-  static const bool configured = [] {
-    FPLS_CHECK(cudaFuncSetAttribute(ozaki_gemm_pair_kernel<BN>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_DATA + 1024));
-    return true;
-  }();
-  (void)configured;
+  allow_shared_memory((const void*)ozaki_gemm_pair_kernel<BN>);
   const int kb_total = a.k_p / OZ_BK;
   const int seg_bytes = std::max(OZ_KPAD, (int)((2147483647LL / (16129LL * S)) / OZ_KPAD * OZ_KPAD));
   const int kb_seg = seg_bytes / OZ_BK;

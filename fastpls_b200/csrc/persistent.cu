@@ -38,7 +38,9 @@
 #include "small.cuh"
 
 #include <algorithm>
+#include <map>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 namespace fpls {
@@ -1131,21 +1133,36 @@ int persistent_ctas(int n, int p, int max_ctas) {
 namespace {
 
 template <class T>
+int measure_capacity(int dev) {
+  int v = 0, coop = 0;
+  try {
+    allow_shared_memory((const void*)persistent_simpls<T>);
+  } catch (const std::runtime_error&) {
+    return 0;
+  }
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, persistent_simpls<T>, PT, Ring<T>::kDynBytes) !=
+          cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return v >= 2 ? v * num_sms() : 0;
+}
+
+// Co-resident CTAs of the current device, measured once for each.
+template <class T>
 int capacity_of() {
-  static const int cap = [] {
-    int v = 0, coop = 0, dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-        cudaFuncSetAttribute(persistent_simpls<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             Ring<T>::kDynBytes) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, persistent_simpls<T>, PT,
-                                                      Ring<T>::kDynBytes) != cudaSuccess) {
-      cudaGetLastError();
-      return 0;
-    }
-    return v >= 2 ? v * num_sms() : 0;
-  }();
-  return cap;
+  static std::mutex mu;
+  static std::map<int, int> caps;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  std::lock_guard<std::mutex> lock(mu);
+  const auto at = caps.find(dev);
+  if (at != caps.end()) return at->second;
+  return caps[dev] = measure_capacity<T>(dev);
 }
 
 }  // namespace
@@ -1272,11 +1289,7 @@ __global__ void ring_finish(const double* __restrict__ part, int ranges, int n, 
 template <class T, int NB>
 void launch_xr_ring(const Fit& f, const double* Rt, int nb, double* part, cudaStream_t s) {
   const int dyn = Ring<T, kRSlice>::kBytes;
-  static const bool configured = [dyn] {
-    FPLS_CHECK(cudaFuncSetAttribute(xr_ring_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-    return true;
-  }();
-  (void)configured;
+  allow_shared_memory((const void*)xr_ring_kernel<T, NB>);
   xr_ring_kernel<T, NB><<<f.C, PT, dyn, s>>>(f, Rt, nb, part);
   count_launch();
   FPLS_LAUNCH("xr_ring_kernel");

@@ -228,13 +228,9 @@ __global__ void xtv_finish(const double* __restrict__ partial, int chunks,
   }
 }
 
-// The staged V block: 64 KB, and past it what a chunk of rows rounded up to a
-// multiple of 128 (from one of 64) adds for up to 32 columns. One limit for
-// every call: callers on several threads launch the kernel with different
-// widths.
 constexpr int kXtvMaxColumns = 32;
+// V rows of a chunk, before the chunk is rounded up to 128 rows (up to 76.8 KB then)
 constexpr int kXtvStagedBytes = 64 * 1024;
-constexpr int kXtvSharedBytes = kXtvStagedBytes + 64 * kXtvMaxColumns * (int)sizeof(double);
 
 template <class T, int MB, bool MOMENTS, bool FINITE>
 void xtv_launch(const T* X, int n, int p, long ld, const double* V, long ldv,
@@ -258,10 +254,9 @@ void xtv_launch(const T* X, int n, int p, long ld, const double* V, long ldv,
   const int slots = nb + (MOMENTS ? 2 : 0);
   scratch.reserve((size_t)chunks * p * slots, stream);
   const size_t smem = (size_t)rc * std::max(nb, 1) * sizeof(double);
-  require(nb <= kXtvMaxColumns && smem <= (size_t)kXtvSharedBytes, "X^T V takes up to 32 columns");
+  require(nb <= kXtvMaxColumns, "X^T V takes up to 32 columns");
   auto run = [&](auto kernel) {
-    if (smem > 48 * 1024)
-      FPLS_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kXtvSharedBytes));
+    allow_shared_memory((const void*)kernel);
     kernel<<<dim3(col_tiles, chunks), kThreads, smem, stream>>>(X, n, p, ld, V, ldv, nb, rc, scratch.get());
   };
   if (pair_aligned(X, ld)) run(xtv_kernel<T, MB, MOMENTS, true, FINITE>);
@@ -702,13 +697,7 @@ void class_moments(const T* X, int n, int p, long ld, const int* labels, int m,
   const int slots = m + 2;
   scratch.reserve((size_t)chunks * p * slots, stream);
   const size_t smem = (size_t)(rc + 1) / 2 * sizeof(double) + (size_t)8 * m * 32 * sizeof(double);
-  static const bool configured = [] {
-    FPLS_CHECK(cudaFuncSetAttribute(class_moments_kernel<T>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (2048 / 2 + 8 * kClassMomentsMaxClasses * 32) * 8));
-    return true;
-  }();
-  (void)configured;
+  allow_shared_memory((const void*)class_moments_kernel<T>);
   class_moments_kernel<T><<<dim3(col_tiles, chunks), kThreads, smem, stream>>>(
       X, n, p, ld, labels, m, rc, scratch.get());
   count_launch();

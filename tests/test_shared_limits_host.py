@@ -69,3 +69,16 @@ def test_no_limit_follows_a_call():
             line = text[:m.start()].count("\n") + 1
             # a size that is a constant of the kernel's template
             assert "constexpr size_t smem" in text, f"{os.path.basename(path)}:{line}"
+
+
+def test_every_limit_is_set_per_device():
+    """The limit belongs to one device: only the registry sets it, so a thread
+    on another device of the process gets it too."""
+    sites = []
+    for path in glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")):
+        text = open(path).read()
+        for m in re.finditer(r"cudaFuncSetAttribute\(", text):
+            body = text[:m.start()].rsplit("\n}", 1)[-1]
+            if "void allow_shared_memory(const void* kernel) {" not in body:
+                sites.append(f"{os.path.basename(path)}:{text[:m.start()].count(chr(10)) + 1}")
+    assert not sites, sites

@@ -1110,11 +1110,21 @@ bool persistent_grid(int n, int p, int max_ctas, int& Cr, int& Cc, int& rb, int&
   // 2^14 beyond (fit in us at 2^15 / 2^14 / 2^13 / 2^12 elements: 97 x 311 FP64,
   // 4 components 533 / 351 / 252 / 224; 200 x 300 FP32, 6: 404 / 328 / 292 /
   // 311; 500 x 2000 FP64, 10: 630 / 545 / 587 / 659; 541 x 1500 FP64, 8: 607 /
-  // 466 / 477 / 421). Fewer CTAs per fit also leave room for other fits of a
-  // batch in one launch.
+  // 466 / 477 / 421).
+  // A fit also leaves room for others in one launch (the serving loop's batches;
+  // a served fit has the bits of the same fit alone, so the rule cannot look at
+  // the batch): past a quarter of the CTAs, four fits a launch, it takes 2^15
+  // elements a CTA. At 2^14 / so, 10 components: 1000 x 3000 FP32 375 / 600
+  // fits/s served by one worker, 975 / 1380 by four, 532 / 515 us alone; 1500 x
+  // 2500 FP64 295 / 470, 815 / 1000, 548 / 554 us; 700 x 2500 FP32 (107 / 74
+  // CTAs) 990 / 1000, 1440 / 1580, 522 / 559 us. A caller that
+  // gives each fit its share keeps 2^14.
   const int shift = elems <= (32L << 13) ? 13 : 14;
-  const long most = max_ctas > 0 ? std::min<long>(max_ctas, 2L * num_sms()) : 2L * num_sms();
-  const int c0 = (int)std::max(1L, std::min<long>(most, (elems + (1L << shift) - 1) >> shift));
+  const long all = 2L * num_sms();
+  const long most = max_ctas > 0 ? std::min<long>(max_ctas, all) : all;
+  long want = (elems + (1L << shift) - 1) >> shift;
+  if (max_ctas <= 0 && want > all / 4) want = std::max(all / 4, (elems + (1L << 15) - 1) >> 15);
+  const int c0 = (int)std::max(1L, std::min<long>(most, want));
   Cr = (n + kBlockRows - 1) / kBlockRows;
   rb = round_up((n + Cr - 1) / Cr, 8);
   Cr = (n + rb - 1) / rb;

@@ -44,6 +44,20 @@ void keep_pool_memory() {
   configured_device = dev;
 }
 
+double device_memory() {
+  static OncePerDevice* once = new OncePerDevice();
+  static std::atomic<double> bytes[64];
+  int dev = 0;
+  FPLS_CHECK(cudaGetDevice(&dev));
+  require(dev >= 0 && dev < 64, "device index beyond the memory table");
+  once->run(bytes, dev, [&] {
+    size_t free_b = 0, total_b = 0;
+    FPLS_CHECK(cudaMemGetInfo(&free_b, &total_b));
+    bytes[dev] = (double)total_b;
+  });
+  return bytes[dev];
+}
+
 void allow_shared_memory(const void* kernel) {
   static OncePerDevice* once = new OncePerDevice();  // never destroyed: threads may outlive main
   int dev = 0;

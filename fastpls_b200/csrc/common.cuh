@@ -17,11 +17,15 @@ namespace fpls {
 // ---------------------------------------------------------------------------
 // host-side error handling
 // ---------------------------------------------------------------------------
+struct OutOfMemory : std::runtime_error {  // device memory, for callers that can do with less
+  using std::runtime_error::runtime_error;
+};
 inline void check(cudaError_t status, const char* what) {
   if (status != cudaSuccess) {
     cudaGetLastError();  // clear a sticky launch error so the context stays usable
-    throw std::runtime_error(std::string(what) + ": " +
-                             cudaGetErrorString(status));
+    const std::string message = std::string(what) + ": " + cudaGetErrorString(status);
+    if (status == cudaErrorMemoryAllocation) throw OutOfMemory(message);
+    throw std::runtime_error(message);
   }
 }
 #define FPLS_CHECK(expr) ::fpls::check((expr), #expr)
@@ -35,6 +39,9 @@ inline void require(bool ok, const char* message) {
 // device) instead of returning it to the driver at every synchronisation:
 // repeated fits then reuse mapped pages rather than remapping gigabytes.
 void keep_pool_memory();
+
+// Bytes of the current device, asked once for each.
+double device_memory();
 
 // Lets a kernel be launched with as much dynamic shared memory as the current
 // device has for it, set once per kernel and device. A limit set to each

@@ -14,6 +14,7 @@
 // batch. The many-fold / many-permutation batched engine lives in batched.cu.
 #include "upload.cuh"
 #include "cv.cuh"
+#include "cv_batches.hpp"
 #include "handle.cuh"
 #include "lda.cuh"
 #include "persistent.cuh"
@@ -186,30 +187,40 @@ struct Settle {
   }
 };
 
-// Folds per batch and the persistent CTAs each may take. The CTA share decides
-// how a fold's sums are split, so it follows from the shape, the number of
-// folds and the device alone: as many folds as 8 GB and the co-resident CTAs
-// hold, in batches of equal size. Free memory (a quarter of it, at least one
-// fold) only lowers how many of them are resident at a time.
+// The grouping of the call's folds (cv_batches.hpp).
 template <class T>
-void batch_shape(int method, const Folds& fp, int n, int p, int m, int a, int folds, size_t pred_bytes,
-                 int* per_batch, int* max_ctas) {
+CvBatches batch_shape(int method, const Folds& fp, int n, int p, int m, int a, size_t pred_bytes) {
   const double one = (double)n * p * sizeof(T) + 8.0 * ((double)p * (2.0 * a + 4.0 * m + 16.0) +
                                                       (double)n * (2.0 * a + 3.0 * m + 8.0)) +
                      (double)pred_bytes + 64.0 * 1024 * 1024;
-  int most = (int)std::max(1.0, std::min((double)folds, 8e9 / one));
-  *max_ctas = 0;
-  if (method != kPlssvd) {
-    const int cap = persistent_capacity((int)sizeof(T));
-    while (most > 1 && most * persistent_ctas(fp.max_train, p, cap / most) > cap) --most;
-    if ((long)fp.max_train * p > kPersistMaxElements) most = 1;
-    if (cap > 0) *max_ctas = cap / most;
+  const bool simpls = method != kPlssvd;
+  return cv_batches(
+      fp.count, one, device_memory(), simpls ? persistent_capacity((int)sizeof(T)) : -1,
+      simpls && (long)fp.max_train * p > kPersistMaxElements,
+      [&](int share) { return persistent_ctas(fp.max_train, p, share); },
+      [] {
+        size_t free_b = 0, total_b = 0;
+        FPLS_CHECK(cudaMemGetInfo(&free_b, &total_b));
+        return (double)free_b;
+      });
+}
+
+// run(f0, f1) for all folds in batches. A batch that does not find its memory
+// leaves no result behind (run writes them last) and is taken again in halves,
+// down to one fold. run returns the error of a fold, if any, after the results
+// of the folds before it.
+template <class F>
+void in_batches(int folds, int per_batch, F&& run) {
+  for (int f0 = 0; f0 < folds;) {
+    const int f1 = std::min(folds, f0 + per_batch);
+    try {
+      if (std::exception_ptr failed = run(f0, f1)) std::rethrow_exception(failed);
+      f0 = f1;
+    } catch (const OutOfMemory&) {
+      if (f1 - f0 <= 1) throw;
+      per_batch = (f1 - f0) / 2;
+    }
   }
-  const int batches = (folds + most - 1) / most;
-  size_t free_b = 0, total_b = 0;
-  FPLS_CHECK(cudaMemGetInfo(&free_b, &total_b));
-  const int resident = (int)std::max(1.0, std::min((double)folds, 0.25 * (double)free_b / one));
-  *per_batch = std::min((folds + batches - 1) / batches, resident);
 }
 
 // The fit of a prepared fold on its stream; a SIMPLS fold that takes the
@@ -341,14 +352,11 @@ void cv_regression(int method, const T* predictors, const T* responses,
     lanes.lanes_after_main();
     const size_t block = (size_t)fp.max_test * q;
     const int step = prefixes_at_once(block * sizeof(double), prefix_count);
-    int per_batch = 1, max_ctas = 0;
-    batch_shape<T>(method, fp, n, p, q, maximum_prefix, fp.count, block * step * sizeof(double), &per_batch,
-                   &max_ctas);
+    const CvBatches shape = batch_shape<T>(method, fp, n, p, q, maximum_prefix, block * step * sizeof(double));
     std::fill(metrics, metrics + prefix_count, 0.0);
     std::vector<double> counts(prefix_count, 0.0), fold_ss(prefix_count, 0.0);
-    std::exception_ptr failed;
-    for (int f0 = 0; f0 < fp.count && !failed; f0 += per_batch) {
-      const int f1 = std::min(fp.count, f0 + per_batch);
+    in_batches(fp.count, shape.per_batch, [&](int f0, int f1) {
+      std::exception_ptr failed;
       // row positions of the batch's folds: one copy (a copy from pageable
       // memory waits for its stream)
       std::vector<int> host_pos((size_t)(f1 - f0) * n);
@@ -385,9 +393,11 @@ void cv_regression(int method, const T* predictors, const T* responses,
           d.model.ymean.allocate(q, d.st);
           prepare_responses<T>(d.Ytr.get(), nullptr, d.ntr, q, d.Yc.get(), d.model.ymean.get(), d.ycsum.get(),
                                d.ws.flag.get(), d.st);
-          fit_fold<T>(method, d, p, maximum_prefix, scaling, max_ctas);
+          fit_fold<T>(method, d, p, maximum_prefix, scaling, shape.max_ctas);
           batch.push_back(std::move(fold));
         }
+      } catch (const OutOfMemory&) {
+        throw;
       } catch (...) {
         failed = std::current_exception();  // after the folds before it
       }
@@ -449,8 +459,8 @@ void cv_regression(int method, const T* predictors, const T* responses,
         }
         status[d.f] = 1;
       }
-    }
-    if (failed) std::rethrow_exception(failed);
+      return failed;
+    });
     const double nan = std::numeric_limits<double>::quiet_NaN();
     for (int j = 0; j < prefix_count; ++j) {
       const double sse = metrics[j];
@@ -501,15 +511,12 @@ void cv_classification(int method, const T* predictors, const int* labels,
     lanes.lanes_after_main();
     const size_t block = (size_t)fp.max_test * classes;
     const int step = prefixes_at_once(block * sizeof(double), prefix_count);
-    int per_batch = 1, max_ctas = 0;
-    batch_shape<T>(method, fp, n, p, classes, maximum_prefix, fp.count, 2 * block * step * sizeof(double),
-                   &per_batch, &max_ctas);
+    const CvBatches shape = batch_shape<T>(method, fp, n, p, classes, maximum_prefix, 2 * block * step * sizeof(double));
     std::fill(metrics, metrics + prefix_count, 0.0);
     std::vector<double> counts(prefix_count, 0.0);
     if (store_scores) std::fill(score_output, score_output + (size_t)n * classes * prefix_count, T(0));
-    std::exception_ptr failed;
-    for (int f0 = 0; f0 < fp.count && !failed; f0 += per_batch) {
-      const int f1 = std::min(fp.count, f0 + per_batch);
+    in_batches(fp.count, shape.per_batch, [&](int f0, int f1) {
+      std::exception_ptr failed;
       // row positions and compacted training labels of the batch's folds: one
       // copy each (a copy from pageable memory waits for its stream)
       std::vector<int> host_pos((size_t)(f1 - f0) * n), host_lab(host_pos.size(), 1);
@@ -534,6 +541,7 @@ void cv_classification(int method, const T* predictors, const int* labels,
       FPLS_CHECK(cudaMemcpyAsync(lab.get(), host_lab.data(), sizeof(int) * host_lab.size(),
                                  cudaMemcpyHostToDevice, lanes.main));
       lanes.lanes_after_main();
+      std::vector<std::pair<int, int>> single;  // folds left with one class to learn, and that class
       std::vector<std::unique_ptr<Fold<T>>> batch;
       Results out;
       Settle settle{lanes};
@@ -549,14 +557,7 @@ void cv_classification(int method, const T* predictors, const int* labels,
           for (int c = 0; c < classes; ++c)
             if (cnt[c] > 0) active.push_back(c + 1);
           if (active.size() <= 1) {
-            const int fallback = active.empty() ? 1 : active.front();
-            for (int j = 0; j < prefix_count; ++j)
-              for (int r : held) {
-                if (store_predictions) prediction_output[(size_t)j * n + r] = fallback;
-                metrics[j] += labels[r] == fallback ? 1.0 : 0.0;
-                counts[j] += 1.0;
-              }
-            status[f] = 4;
+            single.push_back({f, active.empty() ? 1 : active.front()});
             continue;
           }
           if (maximum_prefix > std::min(n - (int)held.size() - 1, p))
@@ -582,9 +583,11 @@ void cv_classification(int method, const T* predictors, const int* labels,
           d.model.ymean.allocate(d.m, d.st);
           prepare_responses<T>(nullptr, d.lab, d.ntr, d.m, d.Yc.get(), d.model.ymean.get(),
                                d.ycsum.get(), d.ws.flag.get(), d.st);
-          fit_fold<T>(method, d, p, maximum_prefix, scaling, max_ctas);
+          fit_fold<T>(method, d, p, maximum_prefix, scaling, shape.max_ctas);
           batch.push_back(std::move(fold));
         }
+      } catch (const OutOfMemory&) {
+        throw;
       } catch (...) {
         failed = std::current_exception();  // after the folds before it
       }
@@ -633,6 +636,15 @@ void cv_classification(int method, const T* predictors, const int* labels,
         }
       collect(batch, out, lanes);
       lanes.sync();
+      for (const auto& [f, fallback] : single) {
+        for (int j = 0; j < prefix_count; ++j)
+          for (int r : fp.test[f]) {
+            if (store_predictions) prediction_output[(size_t)j * n + r] = fallback;
+            metrics[j] += labels[r] == fallback ? 1.0 : 0.0;
+            counts[j] += 1.0;
+          }
+        status[f] = 4;
+      }
       for (size_t b = 0; b < batch.size(); ++b) {
         Fold<T>& d = *batch[b];
         const int c = d.m;
@@ -660,8 +672,8 @@ void cv_classification(int method, const T* predictors, const int* labels,
         }
         status[d.f] = 1;
       }
-    }
-    if (failed) std::rethrow_exception(failed);
+      return failed;
+    });
     for (int j = 0; j < prefix_count; ++j)
       metrics[j] = counts[j] > 0.0 ? metrics[j] / counts[j]
                                    : std::numeric_limits<double>::quiet_NaN();

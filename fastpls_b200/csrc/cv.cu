@@ -6,12 +6,12 @@
 // double, prediction and score output layouts). X and Y are uploaded once;
 // each fold's training and held-out rows are split on the device and the
 // fold model is fitted by the resident engine (fit.cu / plssvd.cu). Folds run
-// in batches: every fold of a batch is prepared on one of a few streams, the
-// SIMPLS folds that take the persistent form run their component loops in one
-// launch with the co-resident CTAs shared between them (a fold alone leaves
-// most SMs idle: ten folds of 541 x 1500 FP64 were ten launches of 24 CTAs, 527
-// us each), and the held-out predictions follow on the streams; one wait per
-// batch. The many-fold / many-permutation batched engine lives in batched.cu.
+// in batches: the SIMPLS folds of a batch that take the persistent form run
+// their component loops in one launch with the co-resident CTAs shared between
+// them (a fold alone leaves most SMs idle: ten folds of 541 x 1500 FP64 were ten
+// launches of 24 CTAs, 527 us each), the others' loops overlap on a few
+// streams, the held-out predictions follow, and the call waits once per batch.
+// The many-fold / many-permutation batched engine lives in batched.cu.
 #include "upload.cuh"
 #include "cv.cuh"
 #include "cv_batches.hpp"
@@ -129,19 +129,28 @@ struct Results {
   const V* on_host(size_t at) const { return reinterpret_cast<const V*>(host.data() + at); }
 };
 
-constexpr int kLanes = 4;
+// Lanes of the call's folds (cv_batches.hpp).
+int call_lanes(int method, int folds, int n, int p, int m, int a, bool classification, int elem) {
+  if (method == kPlssvd || (long)n * p > kPersistMaxElements) return 0;
+  const bool persistent = persistent_enabled() && persistent_supported(m, a) && persistent_ctas(n, p) > 0 &&
+                          persistent_capacity(elem) > 0 && !simpls_gram_route(n, p, a, classification) &&
+                          simpls_block_size(n, p, m, a, classification, elem == 4) <= 1;
+  return fold_lanes(folds, !persistent);
+}
 
 // The streams of one call: `main` (uploads, shared launches) and the lanes
-// that prepare and finish the folds.
+// that prepare and finish the folds, if any.
 struct Lanes {
   cudaStream_t main = nullptr, lane[kLanes] = {};
   cudaEvent_t ev = nullptr;
-  explicit Lanes(int lanes) {
+  const int count;
+  explicit Lanes(int lanes) : count(lanes) {
     FPLS_CHECK(cudaStreamCreateWithFlags(&main, cudaStreamNonBlocking));
     FPLS_CHECK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    for (int k = 0; k < std::min(lanes, kLanes); ++k)
-      FPLS_CHECK(cudaStreamCreateWithFlags(&lane[k], cudaStreamNonBlocking));
+    for (int k = 0; k < count; ++k) FPLS_CHECK(cudaStreamCreateWithFlags(&lane[k], cudaStreamNonBlocking));
   }
+  // the stream of the k-th fold of a batch
+  cudaStream_t of(size_t k) const { return count > 0 ? lane[k % count] : main; }
   ~Lanes() {
     for (cudaStream_t s : lane)
       if (s) {
@@ -344,7 +353,7 @@ void cv_regression(int method, const T* predictors, const T* responses,
     total_ss += ss - s * s / n;
   }
 
-  Lanes lanes(fp.count);
+  Lanes lanes(call_lanes(method, fp.count, fp.max_train, p, q, maximum_prefix, false, (int)sizeof(T)));
   {
     DeviceArray<T> X((size_t)n * p, lanes.main), Y((size_t)n * q, lanes.main);
     upload_h2d(X.get(), predictors, sizeof(T) * n * p, lanes.main);
@@ -381,7 +390,7 @@ void cv_regression(int method, const T* predictors, const T* responses,
           Fold<T>& d = *fold;
           d.f = f;
           d.m = q;
-          d.st = lanes.lane[batch.size() % std::min(fp.count, kLanes)];
+          d.st = lanes.of(batch.size());
           d.nte = (int)held.size();
           d.ntr = n - d.nte;
           d.pos = pos.get() + (size_t)(f - f0) * n;
@@ -504,7 +513,7 @@ void cv_classification(int method, const T* predictors, const int* labels,
   if (fp.max_test < 1 || fp.max_train < 2)
     throw std::invalid_argument("CUDA CV contains an empty train or test fold");
 
-  Lanes lanes(fp.count);
+  Lanes lanes(call_lanes(method, fp.count, fp.max_train, p, classes, maximum_prefix, true, (int)sizeof(T)));
   {
     DeviceArray<T> X((size_t)n * p, lanes.main);
     upload_h2d(X.get(), predictors, sizeof(T) * n * p, lanes.main);
@@ -567,7 +576,7 @@ void cv_classification(int method, const T* predictors, const int* labels,
           d.f = f;
           d.m = (int)active.size();
           d.active = active;
-          d.st = lanes.lane[batch.size() % std::min(fp.count, kLanes)];
+          d.st = lanes.of(batch.size());
           d.nte = (int)held.size();
           d.ntr = n - d.nte;
           d.pos = pos.get() + (size_t)(f - f0) * n;

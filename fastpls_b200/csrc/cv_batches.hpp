@@ -6,6 +6,20 @@
 
 namespace fpls {
 
+constexpr int kLanes = 4;
+
+// Streams beside the main one that the folds of a batch are spread over (0:
+// everything on the main one). Folds whose component loop is a chain of small
+// kernels overlap on lanes; the others have no chain to hide, and lanes cost
+// them: an allocation that takes a block last used on another stream is about
+// 10 us instead of 0.6, some 30 a fold, and a stream about 0.14 ms to make and
+// destroy. us a call with no lane / four lanes (one fold after another before
+// the batches): 246 x 62, 5 folds 640 / 1620 (1090); PLS-SVD 288 x 7, 60 folds
+// 7000 / 26300 (12800); 601 x 1500, 10 folds 2080 / 3120 (9380). With the loop as
+// kernels: 60 x 40, 40 responses, 6 components, 10 folds 9950 / 4580 (22900);
+// 3000 x 200 in 12 classes, 10 components, 10 folds 9900 / 6980 (30200).
+inline int fold_lanes(int folds, bool kernel_loops) { return kernel_loops ? std::min(folds, kLanes) : 0; }
+
 struct CvBatches {
   int per_batch = 1;  // folds resident at a time
   int max_ctas = 0;   // persistent CTAs of each (0: no shared launch)

@@ -35,6 +35,9 @@ int main() {
             if (asked && b.per_batch > 1 && b.per_batch * fold > 0.25 * free * device) return 6;
           }
         }
+  // lanes only where the component loops are chains of kernels
+  if (fpls::fold_lanes(60, false) != 0 || fpls::fold_lanes(2, true) != 2 || fpls::fold_lanes(60, true) != fpls::kLanes)
+    return 9;
   // a method without persistent fits, and a device without cooperative launches
   const auto none = [] { return 1e12; };
   const auto all = [](int) { return 296; };

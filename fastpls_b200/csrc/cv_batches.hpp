@@ -48,7 +48,7 @@ CvBatches cv_batches(int folds, double fold_bytes, double device_bytes, int capa
   }
   const int batches = (folds + most - 1) / most;
   out.per_batch = (folds + batches - 1) / batches;
-  if (out.per_batch * fold_bytes > device_bytes / 64)
+  if (out.per_batch * fold_bytes > device_bytes / 32)
     out.per_batch = std::min(out.per_batch, (int)std::max(1.0, std::min((double)folds, 0.25 * free_bytes() / fold_bytes)));
   return out;
 }

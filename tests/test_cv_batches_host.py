@@ -31,7 +31,7 @@ int main() {
             if (b.per_batch < 1 || b.per_batch > roomy.per_batch) return 2;
             if (b.per_batch > 1 && b.per_batch * ctas(b.max_ctas) > cap) return 3;
             if (alone && b.per_batch != 1) return 4;
-            if (roomy.per_batch * fold <= device / 64 ? asked : !asked) return 5;
+            if (roomy.per_batch * fold <= device / 32 ? asked : !asked) return 5;
             if (asked && b.per_batch > 1 && b.per_batch * fold > 0.25 * free * device) return 6;
           }
         }

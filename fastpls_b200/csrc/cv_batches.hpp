@@ -28,7 +28,7 @@ struct CvBatches {
 // folds: their number; fold_bytes: device memory of one; device_bytes: of the
 // device; capacity: co-resident persistent CTAs; alone: a fold takes a launch of
 // its own; ctas(share): CTAs a fold takes out of a share; free_bytes(): asked
-// only when the folds take more than a 64th of the device, since the query is
+// only when the folds take more than a 32nd of the device, since the query is
 // a call into the driver that other processes' calls hold up (66 to 220 us at
 // the median, 2 ms at the 90th percentile and 30 to 60 at the 99th on a shared
 // host, where a small cross-validation takes 0.5 ms).

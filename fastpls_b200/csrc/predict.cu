@@ -102,7 +102,8 @@ void project_rows(const DeviceModel& model, const T* X, int rows, long ld,
   // bulk-copy stages (both HBM-bound or near it). Otherwise a DMMA product
   // with X in its storage type and K in slices of 256 predictors, so that few
   // rows still fill the SMs and every sum has the same order at any number of
-  // rows and columns (a prefix alone equals the same prefix in a path). 451
+  // rows and columns (a prefix alone equals the same prefix in a path; the forms
+  // for a large X depend on the number of columns). 451
   // new rows x 10000, 20 columns: 93 us in passes of 8, 8 and 4 columns
   // before, 37 us now; 4001 x 4000, 12 columns: 78 us, 46 us.
   const bool large = (long)rows * p >= (1L << 24);

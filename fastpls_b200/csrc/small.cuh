@@ -67,8 +67,9 @@ __device__ inline int jacobi_eigen(double* A, double* E, int m, int max_sweeps =
   const int ek0 = et / m, ei0 = et % m, edk = nt / m, edi = nt % m;
   int sweep = 0;
   double prev = 0.0;
-  for (; sweep < max_sweeps && m > 1; ++sweep) {
-    double off = 0.0, diag = 0.0;
+  int shift = 0;  // A is held times 2^-shift
+  auto masses = [&](double& off, double& diag) {
+    off = diag = 0.0;
     for (int k = tid; k < m * m; k += nt) {
       const int i = k % m, j = k / m;
       if (i != j) off += A[k] * A[k];
@@ -76,6 +77,23 @@ __device__ inline int jacobi_eigen(double* A, double* E, int m, int max_sweeps =
     }
     off = total(off);
     diag = total(diag);
+  };
+  for (; sweep < max_sweeps && m > 1; ++sweep) {
+    double off, diag;
+    masses(off, diag);
+    if (sweep == 0 && !(diag > 0x1p-800 && diag < 0x1p800)) {
+      // entries whose squares vanish or pass the range (data of about 1e-60 or
+      // 1e60 and beyond): the stopping rule would see nothing to do
+      double top = 0.0;
+      for (int k = 0; k < m * m; ++k) top = fmax(top, fabs(A[k]));
+      sync();
+      if (top > 0.0 && isfinite(top)) {
+        shift = ilogb(top);
+        for (int k = tid; k < m * m; k += nt) A[k] = scalbn(A[k], -shift);
+        sync();
+        masses(off, diag);
+      }
+    }
     if (off <= 1e-30 * diag || off == 0.0) break;
     // at the rounding floor (large m) the off-diagonal mass stops shrinking
     if (sweep > 0 && off <= 1e-24 * diag && off > 0.25 * prev) break;
@@ -191,6 +209,10 @@ __device__ inline int jacobi_eigen(double* A, double* E, int m, int max_sweeps =
       }
       sync();
     }
+  }
+  if (shift != 0) {
+    sync();
+    for (int i = tid; i < m; i += nt) A[i + i * m] = scalbn(A[i + i * m], shift);
   }
   __syncthreads();
   return sweep;

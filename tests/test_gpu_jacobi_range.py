@@ -36,3 +36,31 @@ def test_small_responses_beside_ordinary_ones(q, small, exponent):
     sign = np.sign((u[:, :k] * R).sum(0))
     assert np.max(np.abs(R * sign - u[:, :k])) <= tol * s[0] / s[k - 1]
     assert np.max(np.abs(Q * sign - vt[:k].T)) <= tol
+
+
+@pytest.mark.parametrize("exponent", [-450, -300, -210, 210, 300])
+@pytest.mark.parametrize("q", [3, 12, 40])
+def test_plssvd_of_scaled_responses(q, exponent):
+    """A power of two on the responses leaves the directions alone: the squares
+    of the Gram's entries vanish or pass the range, the entries do not."""
+    n, p, k = 120, 60, min(q, 5)
+    x, y = W.latent_regression(n, p, q, q + 2, 0.5, q, dtype=np.float64)
+    got = []
+    for z in (y, np.ldexp(y, exponent)):
+        m = api.fit_resident(x, np.asfortranarray(z), ncomp=k, method="plssvd", precision=64)
+        got.append((m.weights(), m.loadings(), m.predict_path(x[:9], [1, k])))
+        m.close()
+    (R0, Q0, y0), (R1, Q1, y1) = got
+    # exact scaling up to the rounding of values that leave the normal range
+    assert np.max(np.abs(R1 - R0)) <= 1e-12
+    assert np.max(np.abs(Q1 - Q0)) <= 1e-12
+    assert np.max(np.abs(np.ldexp(y1, -exponent) - y0)) <= 1e-12 * np.max(np.abs(y0))
+
+
+@pytest.mark.parametrize("exponent", [-300, -210, 210])
+def test_svd_of_scaled_matrices(exponent):
+    x = np.random.default_rng(2).standard_normal((90, 50)) * 0.7 ** np.arange(50)
+    u0, d0, v0 = api.fastsvd(x, 4)
+    u, d, v = api.fastsvd(np.ldexp(x, exponent), 4)
+    assert np.max(np.abs(np.ldexp(d, -exponent) - d0)) <= 1e-12 * d0[0]
+    assert np.max(np.abs(u - u0)) <= 1e-9 and np.max(np.abs(v - v0)) <= 1e-9

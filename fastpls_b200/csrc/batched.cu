@@ -1675,7 +1675,6 @@ void BatchedCv<T>::run(const T* X_, int n_, int p_, const T* Y_, int q_,
   last_batched_stats() = BatchedStats{};
   // attributes are not set inside a capture
   if (digits > 0) ozaki_configure_kernels();
-  const size_t smem_defl = deflate_shared_bytes(q, kmax, deflate_threads(n));
   allow_shared_memory((const void*)deflate_batched<true>);
   allow_shared_memory((const void*)deflate_batched<false>);
   const cudaStream_t s = ws->main;
